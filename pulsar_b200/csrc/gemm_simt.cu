@@ -2,19 +2,292 @@
 //
 // This is the matrix product of the true 32-bit path: no tensor cores and no
 // reduced-precision mode.  Each output element is a plain float32 sum over k in
-// ascending order, so its value does not depend on M, on the position of its row in
-// the batch, or on which other rows are present.  A and W may be float32 or
-// bfloat16 (read exactly, accumulated in float32); the output is float32 or the
-// activation type.  Any M, N, K is accepted.
+// ascending order (one chain of multiply-adds, in every kernel of this file), so its value
+// does not depend on M, on the position of its row in the batch, on which other rows are
+// present or on which of the kernels ran.  A and W may be float32 or bfloat16 (read exactly,
+// accumulated in float32); the output is float32 or the activation type.  Any M, N, K is accepted.
+//
+// Three kernels:
+//   * simt_rows_kernel (up to 16 rows of A, float32 operands): streams the weights, bound by HBM;
+//   * simt_tile_kernel (more rows, float32 operands): bound by the FMA pipes;
+//   * gemm_simt_kernel: everything else (bfloat16 operands, rows of K that are no multiple of 16 bytes).
 //
 // The reference uses at::linear here (cuBLAS SGEMM in float32,
 // pulsar-core/src/model/qwen3.cpp:82-84, 114, 117-119, 128).
-#include "common.cuh"
+#include "mma_common.cuh"
 
 namespace {
 
 using namespace pb;
 
+// ---------------------------------------------------------------- up to 16 rows
+// Bound by reading W once, and with more rows of A by shared memory.  The sums stay chains in ascending k: a chain takes 4 cycles
+// a step, so 128 blocks of 32 weight rows ask for 8 TB/s, above what HBM gives, and a split of K (which would change the sums)
+// is not needed.  W and A come through shared memory in stages of 64 k by 16-byte asynchronous copies of four warps that do
+// nothing else; CW further warps compute, a thread R rows of W times T rows of A.  W depends on no earlier kernel: its first
+// stages are asked for before griddepcontrol.wait.  A 16-byte read of shared memory costs a warp 4 cycles, 2 where neighbouring
+// lanes read the same place (measured), so lanes that share a row of W stand side by side; W's rows stand 68 floats apart, which
+// keeps the others off each other's banks.
+// us on the sizes of an 8B layer, 64 x 64 tiles of the general kernel before: 6144 x 4096 1 row 21.7 (was 277), 4 rows 27.2, 8 rows
+// 36.7, 16 rows 63; 4096 x 4096 19.3 / 21.6 / 27.4 / 47 (282); 24576 x 4096 66.8 / 74.8 / 103 / 188 (480); 4096 x 12288
+// 43.7 / 50.8 / 69 / 120 (851); 151936 x 4096 376 (6.6 TB/s) / 406 / 562 / 1055.
+constexpr int RN = 32, RK = 64, RSTRIDE = RK + 4, RLOAD = 128;
+
+template <int R, int T, int CW, int RST, typename TO>
+__global__ void __launch_bounds__(RLOAD + 32 * CW)
+simt_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out, int M, int N, int K) {
+    extern __shared__ __align__(16) float rows_smem[];
+    constexpr int LR = RN / R, LT = 32 / LR, MR = LT * T * CW;      // lanes along the rows of W, along those of A; rows of A held
+    float* ws = rows_smem;                                  // [RST][RN][RSTRIDE]
+    float* as = ws + RST * RN * RSTRIDE;                    // [RST][MR][RK]
+    const int tid = threadIdx.x;
+    const int row0 = blockIdx.x * RN;
+    const int n_kt = (K + RK - 1) / RK;
+
+    if (tid < RLOAD) {                                      // the copying warps
+        const uint64_t policy = l2_policy_evict_first();
+        const int q = tid % (RK / 4) * 4, r0 = tid / (RK / 4);     // this thread's column of 4 floats and its first row
+        auto load_w = [&](int kt) {
+            float* dst = ws + (kt % RST) * RN * RSTRIDE;
+#pragma unroll
+            for (int e = 0; e < RN * RK / 4 / RLOAD; ++e) {
+                const int r = r0 + e * (RLOAD / (RK / 4));
+                const bool ok = row0 + r < N && kt * RK + q < K;
+                cp_async16_policy(smem_u32(dst + r * RSTRIDE + q), ok ? W + (size_t)(row0 + r) * K + kt * RK + q : W, ok, policy);
+            }
+        };
+        auto load_a = [&](int kt) {
+            float* dst = as + (kt % RST) * MR * RK;
+#pragma unroll
+            for (int r = r0; r < MR; r += RLOAD / (RK / 4)) {
+                const bool ok = r < M && kt * RK + q < K;
+                cp_async16(smem_u32(dst + r * RK + q), ok ? A + (size_t)r * K + kt * RK + q : A, ok);
+            }
+        };
+#pragma unroll
+        for (int s = 0; s < RST - 1; ++s) {
+            if (s < n_kt) load_w(s);
+            if (s < RST - 2) cp_async_commit();
+        }
+        pdl_wait();
+        // A's first stages through registers, beside W's copies (a group of their own would have to wait for all of those)
+        for (int s = 0; s < RST - 1 && s < n_kt; ++s)
+            for (int r = r0; r < MR; r += RLOAD / (RK / 4)) {
+                const bool ok = r < M && s * RK + q < K;
+                *reinterpret_cast<float4*>(as + (s * MR + r) * RK + q) =
+                    ok ? *reinterpret_cast<const float4*>(A + (size_t)r * K + s * RK + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        cp_async_commit();
+        for (int kt = 0; kt < n_kt; ++kt) {
+            cp_async_wait<RST - 2>();
+            __syncthreads();                                // stage kt has landed; the one before it is done with
+            if (kt + RST - 1 < n_kt) {
+                load_w(kt + RST - 1);
+                load_a(kt + RST - 1);
+            }
+            cp_async_commit();
+        }
+        pdl_trigger();
+        return;
+    }
+
+    const int lane = tid & 31, warp = (tid - RLOAD) >> 5;
+    constexpr int RU = R + T <= 2 ? 4 : R + T <= 4 ? 2 : 1;
+    const int lr = LT == 1 ? lane : LT == 2 ? lane >> 1 : (lane & 1) | lane >> 3 << 1;
+    const int m0 = warp * LT * T + (LT == 1 ? 0 : LT == 2 ? lane & 1 : lane >> 1 & 3) * T;
+    float acc[R][T];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int t = 0; t < T; ++t) acc[r][t] = 0.0f;
+    pdl_wait();
+    for (int kt = 0; kt < n_kt; ++kt) {
+        __syncthreads();
+        const float* wr = ws + (kt % RST) * RN * RSTRIDE + lr * RSTRIDE;
+        const float* ar = as + ((kt % RST) * MR + m0) * RK;
+        float4 w[2][RU][R], a[2][RU][T];                    // the operands of a batch of 4 RU k, and of the next one
+        auto fetch = [&](int b, int kk) {
+#pragma unroll
+            for (int u = 0; u < RU; ++u) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) w[b][u][r] = *reinterpret_cast<const float4*>(wr + r * LR * RSTRIDE + kk + 4 * u);
+#pragma unroll
+                for (int t = 0; t < T; ++t) a[b][u][t] = *reinterpret_cast<const float4*>(ar + t * RK + kk + 4 * u);
+            }
+        };
+        auto step = [&](float (&c)[R][T], const float4 (&x)[T], const float4 (&y)[R]) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int t = 0; t < T; ++t) c[r][t] = fmaf(x[t].x, y[r].x, c[r][t]);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int t = 0; t < T; ++t) c[r][t] = fmaf(x[t].y, y[r].y, c[r][t]);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int t = 0; t < T; ++t) c[r][t] = fmaf(x[t].z, y[r].z, c[r][t]);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int t = 0; t < T; ++t) c[r][t] = fmaf(x[t].w, y[r].w, c[r][t]);
+        };
+        fetch(0, 0);
+#pragma unroll
+        for (int kk = 0; kk < RK; kk += 4 * RU) {
+            const int b = kk / (4 * RU) & 1;
+            if (kk + 4 * RU < RK) fetch(b ^ 1, kk + 4 * RU);
+#pragma unroll
+            for (int u = 0; u < RU; ++u) step(acc, a[b][u], w[b][u]);
+        }
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int n = row0 + lr + r * LR;
+            if (m0 + t < M && n < N) out[(size_t)(m0 + t) * N + n] = from_float<TO>(acc[r][t]);
+        }
+}
+
+template <int R, int T, int CW, int RST, typename TO>
+int launch_rows_st(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
+    constexpr int MR = 32 / (RN / R) * T * CW;
+    constexpr size_t smem = sizeof(float) * RST * (RN * RSTRIDE + MR * RK);
+    static const cudaError_t allowed =
+        cudaFuncSetAttribute(simt_rows_kernel<R, T, CW, RST, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (allowed != cudaSuccess) return (int)allowed;
+    return launch_pdl(simt_rows_kernel<R, T, CW, RST, TO>, dim3((N + RN - 1) / RN), dim3(RLOAD + 32 * CW), smem, stream, A, W, out, M, N, K);
+}
+
+// With one block an SM or fewer a block's ring has to keep HBM busy by itself: 16 stages instead of 8 (4096 x 4096, one row of A:
+// 19.3 against 19.5 us; 4096 x 12288: 43.9 against 50.3).
+template <int R, int T, int CW, typename TO>
+int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
+    if ((N + RN - 1) / RN <= 148) return launch_rows_st<R, T, CW, 16>(A, W, out, M, N, K, stream);
+    return launch_rows_st<R, T, CW, 8>(A, W, out, M, N, K, stream);
+}
+
+// ---------------------------------------------------------------- more rows
+// Bound by the FMA pipes (59 % of their cycles with 24576 x 1024 weights and 384 rows; the issue slots 71 %).  A block of 128
+// threads owns 8 TM x 128 outputs, a warp 8 TM x 32, a thread TM x 8 of them (rows ty + 8 i, columns tx + 4 j).  Both operands
+// stand in shared memory as they do in memory, k fastest, so that asynchronous 16-byte copies bring them and a thread reads four
+// k of a row at once: 16 reads per 256 multiply-adds with TM 8.  Rows stand 20 floats apart (an odd number of 16-byte units: no
+// bank conflicts), and of the 8 x 4 lanes of a warp neighbours share a row or a column (see above).  Three stages of 16 k.  A block
+// whose last rows lie behind M computes 8 or 16 rows instead.  k slowest in shared memory (copies of 4 bytes) was slower (35 against 39
+// TFLOP/s at 24576 x 4096, 387 rows), packed pairs of multiply-adds are not faster than single ones on this chip (61 against 65).
+constexpr int GN = 128, GK = 16, GST = 3, GSTRIDE = GK + 4;
+
+template <int GM, int NI, typename TO>
+__device__ __forceinline__ void tile_block(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out,
+                                           int M, int N, int K, float* smem) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = lane >> 1 & 3, ty = (lane & 1) | lane >> 3 << 1;
+    const int row0 = blockIdx.x * GM, col0 = blockIdx.y * GN;
+    constexpr int kStage = (GM + GN) * GSTRIDE;
+    const int n_kt = (K + GK - 1) / GK;
+    const int lq = tid % 4 * 4, lr = tid / 4;               // this thread's four k and its row within a copy of 32 rows
+    auto load = [&](int kt) {
+        float* dst = smem + (kt % GST) * kStage + lq;
+        const int k = kt * GK + lq;
+#pragma unroll
+        for (int r = lr; r < 8 * NI; r += 32) {
+            const bool ok = k < K && row0 + r < M;
+            cp_async16(smem_u32(dst + r * GSTRIDE), ok ? A + (size_t)(row0 + r) * K + k : A, ok);
+        }
+#pragma unroll
+        for (int r = lr; r < GN; r += 32) {
+            const bool ok = k < K && col0 + r < N;
+            cp_async16(smem_u32(dst + (GM + r) * GSTRIDE), ok ? W + (size_t)(col0 + r) * K + k : W, ok);
+        }
+    };
+    float acc[NI][8];
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+#pragma unroll
+    for (int s = 0; s < GST - 1; ++s) {
+        if (s < n_kt) load(s);
+        cp_async_commit();
+    }
+    for (int kt = 0; kt < n_kt; ++kt) {
+        cp_async_wait<GST - 2>();
+        __syncthreads();
+        if (kt + GST - 1 < n_kt) load(kt + GST - 1);
+        cp_async_commit();
+        const float* a_s = smem + (kt % GST) * kStage + ty * GSTRIDE;
+        const float* w_s = smem + (kt % GST) * kStage + (GM + warp * 32 + tx) * GSTRIDE;
+#pragma unroll
+        for (int kk = 0; kk < GK; kk += 4) {
+            float4 a[NI];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) a[i] = *reinterpret_cast<const float4*>(a_s + 8 * i * GSTRIDE + kk);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 w = *reinterpret_cast<const float4*>(w_s + 4 * j * GSTRIDE + kk);
+#pragma unroll
+                for (int i = 0; i < NI; ++i) acc[i][j] = fmaf(a[i].x, w.x, acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < NI; ++i) acc[i][j] = fmaf(a[i].y, w.y, acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < NI; ++i) acc[i][j] = fmaf(a[i].z, w.z, acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < NI; ++i) acc[i][j] = fmaf(a[i].w, w.w, acc[i][j]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int r = row0 + ty + 8 * i;
+        if (r >= M) continue;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = col0 + warp * 32 + tx + 4 * j;
+            if (c < N) out[(size_t)r * N + c] = from_float<TO>(acc[i][j]);
+        }
+    }
+}
+
+template <int TM, typename TO>
+__global__ void __launch_bounds__(128, TM == 8 ? 3 : 4)
+simt_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out, int M, int N, int K) {
+    constexpr int GM = 8 * TM;
+    __shared__ __align__(16) float tile_smem[GST * (GM + GN) * GSTRIDE];
+    const int left = M - (int)blockIdx.x * GM;
+    if (TM == 8 && left > 32) tile_block<GM, TM, TO>(A, W, out, M, N, K, tile_smem);
+    else if (left > 16) tile_block<GM, 4, TO>(A, W, out, M, N, K, tile_smem);
+    else if (left > 8) tile_block<GM, 2, TO>(A, W, out, M, N, K, tile_smem);
+    else tile_block<GM, 1, TO>(A, W, out, M, N, K, tile_smem);
+}
+
+template <int TM, typename TO>
+int launch_tile(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
+    dim3 grid((M + 8 * TM - 1) / (8 * TM), (N + GN - 1) / GN);
+    if (grid.y > 65535) return PB_ERR_TOO_LARGE;
+    simt_tile_kernel<TM, TO><<<grid, 128, 0, stream>>>(A, W, out, M, N, K);
+    return launch_status();
+}
+
+// float32 operands whose rows are multiples of 16 bytes on 16-byte addresses
+template <typename TO>
+int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
+    if (M == 1) return launch_rows<1, 1, 1>(A, W, out, M, N, K, stream);
+    if (M == 2) return launch_rows<2, 1, 1>(A, W, out, M, N, K, stream);
+    if (M <= 4) return launch_rows<2, 1, 2>(A, W, out, M, N, K, stream);
+    const bool few = (N + RN - 1) / RN <= 148;
+    if (M <= 8) return few ? launch_rows<2, 1, 4>(A, W, out, M, N, K, stream) : launch_rows<2, 2, 2>(A, W, out, M, N, K, stream);
+    if (M <= 16) return few ? launch_rows<2, 1, 8>(A, W, out, M, N, K, stream) : launch_rows<4, 2, 2>(A, W, out, M, N, K, stream);
+    // 64 rows a block where there are blocks for 16 rounds of the SMs (151936 x 4096, 387 rows: 11.3 against 11.9 ms), else 32, whose last
+    // rounds are less empty (4096 x 4096: 33 rows 161 against 269 us, 387 rows 389 against 500, the general kernel 656;
+    // 24576 x 4096, 387 rows: 2.03 against 2.00 ms, 2.96 before)
+    if ((long)((M + 63) / 64) * ((N + GN - 1) / GN) >= 16 * 148) return launch_tile<8>(A, W, out, M, N, K, stream);
+    return launch_tile<4>(A, W, out, M, N, K, stream);
+}
+
+// ---------------------------------------------------------------- any operands
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;   // 256 threads, 4x4 outputs each
 
 template <typename TA, typename TW, typename TO>
@@ -86,6 +359,11 @@ PB_EXPORT int pb_gemm_simt(int a_dtype, int w_dtype, int out_dtype, const void* 
     if (K <= 0) return PB_ERR_BAD_SIZE;
     if ((a_dtype | w_dtype | out_dtype) & ~1) return PB_ERR_BAD_DTYPE;
     typedef __nv_bfloat16 bf;
+    if (a_dtype == PB_F32 && w_dtype == PB_F32 && K % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0) {
+        const int status = out_dtype == PB_F32 ? launch_f32((const float*)A, (const float*)W, (float*)out, M, N, K, stream)
+                                               : launch_f32((const float*)A, (const float*)W, (bf*)out, M, N, K, stream);
+        if (status != PB_ERR_TOO_LARGE) return status;
+    }
     const int key = a_dtype * 4 + w_dtype * 2 + out_dtype;
     switch (key) {
         case 0: return launch<float, float, float>(A, W, out, M, N, K, stream);
