@@ -92,22 +92,32 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
             float sc[kGP];
 #pragma unroll
             for (int g = 0; g < kGP; ++g) sc[g] = 0.0f;
+            size_t at = 0;                                  // where the key's row begins in the pools
             if (valid) {
                 int page = table[j / page_size];
                 if (!page_ok(page, bounds)) page = 0;
-                const T* kr = k_pool + (((size_t)page * Hkv + kvh) * page_size + j % page_size) * D;
-                for (int d = 0; d < D; d += 8) {
-                    float kf[8];
-                    load_row16(kr + d, kf);
+                at = (((size_t)page * Hkv + kvh) * page_size + j % page_size) * D;
+                const T* kr = k_pool + at;
+                // 32 elements of the row asked for before the first is used (a trip to L2 per 32 elements instead of one per 8)
+                for (int d0 = 0; d0 < D; d0 += 32) {
+                    float kf[4][8];
 #pragma unroll
-                    for (int g = 0; g < kGP; ++g) {
-                        if (g < gn) {
-                            const float4 qa = *reinterpret_cast<const float4*>(q_s + g * D + d);
-                            const float4 qb = *reinterpret_cast<const float4*>(q_s + g * D + d + 4);
-                            sc[g] = fmaf(qa.x, kf[0], sc[g]); sc[g] = fmaf(qa.y, kf[1], sc[g]);
-                            sc[g] = fmaf(qa.z, kf[2], sc[g]); sc[g] = fmaf(qa.w, kf[3], sc[g]);
-                            sc[g] = fmaf(qb.x, kf[4], sc[g]); sc[g] = fmaf(qb.y, kf[5], sc[g]);
-                            sc[g] = fmaf(qb.z, kf[6], sc[g]); sc[g] = fmaf(qb.w, kf[7], sc[g]);
+                    for (int u = 0; u < 4; ++u)
+                        if (d0 + 8 * u < D) load_row16(kr + d0 + 8 * u, kf[u]);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int d = d0 + 8 * u;
+                        if (d >= D) break;
+#pragma unroll
+                        for (int g = 0; g < kGP; ++g) {
+                            if (g < gn) {
+                                const float4 qa = *reinterpret_cast<const float4*>(q_s + g * D + d);
+                                const float4 qb = *reinterpret_cast<const float4*>(q_s + g * D + d + 4);
+                                sc[g] = fmaf(qa.x, kf[u][0], sc[g]); sc[g] = fmaf(qa.y, kf[u][1], sc[g]);
+                                sc[g] = fmaf(qa.z, kf[u][2], sc[g]); sc[g] = fmaf(qa.w, kf[u][3], sc[g]);
+                                sc[g] = fmaf(qb.x, kf[u][4], sc[g]); sc[g] = fmaf(qb.y, kf[u][5], sc[g]);
+                                sc[g] = fmaf(qb.z, kf[u][6], sc[g]); sc[g] = fmaf(qb.w, kf[u][7], sc[g]);
+                            }
                         }
                     }
                 }
@@ -128,23 +138,28 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
             }
             __syncwarp();
             const int n_here = min(32, end - j0);
-            for (int kk = 0; kk < n_here; ++kk) {
-                const int jj = j0 + kk;
-                int page = table[jj / page_size];
-                if (!page_ok(page, bounds)) page = 0;
-                const T* vr = v_pool + (((size_t)page * Hkv + kvh) * page_size + jj % page_size) * D;
-                float vf[kAcc];
+            // four keys' values asked for at once, their rows' places from the lanes that own the keys
+            for (int k0 = 0; k0 < n_here; k0 += 4) {
+                float vf[4][kAcc];
 #pragma unroll
-                for (int i = 0; i < kAcc; ++i) {
-                    const int d = lane + 32 * i;
-                    vf[i] = d < D ? to_float(vr[d]) : 0.0f;
+                for (int u = 0; u < 4; ++u) {
+                    const T* vr = v_pool + __shfl_sync(0xffffffffu, at, min(k0 + u, n_here - 1));
+#pragma unroll
+                    for (int i = 0; i < kAcc; ++i) {
+                        const int d = lane + 32 * i;
+                        vf[u][i] = d < D ? to_float(vr[d]) : 0.0f;
+                    }
                 }
 #pragma unroll
-                for (int g = 0; g < kGP; ++g) {
-                    if (g < gn) {
-                        const float pk = p_s[(warp * kGP + g) * 32 + kk];
+                for (int u = 0; u < 4; ++u) {
+                    if (k0 + u >= n_here) break;
 #pragma unroll
-                        for (int i = 0; i < kAcc; ++i) acc[g][i] = fmaf(pk, vf[i], acc[g][i]);
+                    for (int g = 0; g < kGP; ++g) {
+                        if (g < gn) {
+                            const float pk = p_s[(warp * kGP + g) * 32 + k0 + u];
+#pragma unroll
+                            for (int i = 0; i < kAcc; ++i) acc[g][i] = fmaf(pk, vf[u][i], acc[g][i]);
+                        }
                     }
                 }
             }

@@ -34,3 +34,43 @@ def test_products_of_rows_and_tiles(m, n, k):
         half = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
         ops.gemm_simt(a, w, half)
         assert torch.equal(half, out.bfloat16())
+
+
+# 16 rows a block (many rows; head sizes up to 64 and 128), 8 (wider heads), 4 (few rows); groups of one to more heads than a block
+# has rows, blocks whose tokens belong to several sequences, windows that begin inside a tile
+@pytest.mark.parametrize("q_lens,kv_lens,hq,hkv,d,page,window", [
+    ([387], [420], 16, 4, 128, 16, None), ([300, 1, 41, 3], [300, 70, 500, 3], 20, 4, 64, 16, 150), ([700], [700], 8, 2, 208, 8, 40),
+    ([5, 1, 70], [5, 90, 200], 6, 2, 32, 4, None), ([33], [164], 40, 2, 80, 16, 50), ([260], [261], 36, 1, 48, 4, 33)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_of_rows_that_share_keys(q_lens, kv_lens, hq, hkv, d, page, window, dtype):
+    from pulsar_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(hq * 100 + d)
+    need = [-(-k // page) for k in kv_lens]
+    ids = torch.randperm(sum(need) + 3, generator=torch.Generator().manual_seed(d)).to(torch.int32)
+    table = torch.full((len(need), max(need)), -1, dtype=torch.int32)
+    for s, n in enumerate(need):
+        table[s, :n] = ids[sum(need[:s]):sum(need[:s]) + n]
+        if window:
+            table[s, :max(0, kv_lens[s] - q_lens[s] - window + 1) // page] = -1        # released pages are never looked at
+    pools = [torch.randn(len(ids), hkv, page, d, generator=g, device="cuda").to(dtype) for _ in range(2)]
+    q = torch.randn(sum(q_lens), hq, d, generator=g, device="cuda").to(dtype)
+    out = torch.full_like(q, float("nan"))
+    as_i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")                       # noqa: E731
+    cu = as_i32([sum(q_lens[:i]) for i in range(len(q_lens) + 1)])
+    seq = torch.repeat_interleave(torch.arange(len(q_lens), device="cuda"), as_i32(q_lens)).to(torch.int32)
+    ops.paged_attention_generic(q, pools[0], pools[1], out, table.cuda(), cu, as_i32(kv_lens), seq, d ** -0.5, window)
+    at = 0
+    for s, (n, kl) in enumerate(zip(q_lens, kv_lens)):
+        key = torch.arange(kl)
+        k, v = (p[table[s, key // page].clamp_min(0).long().cuda(), :, (key % page).cuda()].double() for p in pools)
+        k, v = (t.repeat_interleave(hq // hkv, dim=1) for t in (k, v))
+        pos = torch.arange(kl - n, kl, device="cuda")[:, None]
+        hidden = key.cuda()[None] > pos
+        if window:
+            hidden |= key.cuda()[None] <= pos - window
+        scores = torch.einsum("ihd,jhd->hij", q[at:at + n].double(), k) * d ** -0.5
+        want = torch.einsum("hij,jhd->ihd", torch.softmax(scores.masked_fill(hidden, -float("inf")), dim=-1), v)
+        # float32: scores a few units off in the last place and a few hundred rounded additions; bfloat16: the one rounding
+        tol = 2e-5 if dtype == torch.float32 else 2.0 ** -8
+        assert float((out[at:at + n].double() - want).abs().max() / want.abs().max()) < tol
+        at += n
