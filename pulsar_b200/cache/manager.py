@@ -193,6 +193,7 @@ class CacheManager:
             if device is not None:
                 grp.pools = {t.name: torch.zeros((len(grp.entries), c, t.heads, self.page_size, t.width),
                                                  dtype=t.dtype or dtype, device=device) for t in grp.need.tensors}
+        self._entry_pools: Dict[int, Dict[str, torch.Tensor]] = {}      # an entry's part of its group's pools, made at its first use
         self.state: Dict[int, torch.Tensor] = {}
         for e, need in enumerate(self.needs):
             if need.kind == "state" and device is not None:
@@ -365,8 +366,11 @@ class CacheManager:
 
     def pools(self, entry: int) -> Dict[str, torch.Tensor]:
         """The entry's pools by tensor name, each ``[pages, heads, page_size, width]``."""
-        g, i = self.group_of_entry[entry], self.index_in_group[entry]
-        return {name: pool[i] for name, pool in self.groups[g].pools.items()}
+        pools = self._entry_pools.get(entry)
+        if pools is None:
+            g, i = self.group_of_entry[entry], self.index_in_group[entry]
+            pools = self._entry_pools[entry] = {name: pool[i] for name, pool in self.groups[g].pools.items()}
+        return dict(pools)
 
     def kv_pools(self, entry: int) -> Tuple[torch.Tensor, torch.Tensor]:
         pools = self.pools(entry)

@@ -62,7 +62,8 @@ class ModelRunner:
         self.dtype = model.dtype
         self.vocab = model.spec.vocab_size
         self.position_axes = int(getattr(model.spec, "position_axes", 1))
-        self._scratch: Dict[str, torch.Tensor] = {}
+        self._scratch: Dict[tuple, torch.Tensor] = {}
+        self._scratch_views: Dict[tuple, Dict[tuple, torch.Tensor]] = {}      # of each buffer, by shape
         self.scratch_epoch = 0
         self._staging: List[Optional[torch.Tensor]] = [None] * self.N_STAGING
         self._staging_events: List[Optional[torch.cuda.Event]] = [None] * self.N_STAGING
@@ -90,10 +91,16 @@ class ModelRunner:
 
     # ------------------------------------------------------------------ memory
     def scratch(self, tag: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        # Every layer of a step asks for the same few shapes: their views are kept until the buffer is replaced.
+        key = (tag, dtype)
+        views = self._scratch_views.get(key)
+        if views is not None:
+            view = views.get(shape)
+            if view is not None:
+                return view
         numel = 1
         for s in shape:
             numel *= s
-        key = f"{tag}|{dtype}"
         buf = self._scratch.get(key)
         if buf is None or buf.numel() < numel:
             if self._capturing:
@@ -102,7 +109,11 @@ class ModelRunner:
             buf = torch.empty(grow, dtype=dtype, device=self.device)
             self._scratch[key] = buf
             self.scratch_epoch += 1
-        return buf[:numel].view(shape)
+            views = None
+        if views is None or len(views) >= 16:
+            views = self._scratch_views[key] = {}
+        view = views[shape] = buf[:numel].view(shape)
+        return view
 
     def cache_view(self, ctx: StepContext, entry: int) -> CacheView:
         need = self.cache.needs[entry]

@@ -11,6 +11,7 @@ The reference exposes its kernels as ``torch.ops.pulsar.*`` through TorchBind
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional, Tuple
 
@@ -187,8 +188,12 @@ def code(dtype: torch.dtype) -> int:
         raise KernelError(f"dtype {dtype} is not float32 or bfloat16") from None
 
 
+# The current device's current stream as a number, without the Stream object that torch.cuda.current_stream() makes.
+_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device())
 
 
 def _cuda(*tensors) -> None:
@@ -381,6 +386,8 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: boo
     ``squared_relu``: ``out`` [M, N] receives max(a @ w.T, 0)^2.
     Returns False, having done nothing, when the sizes are not the kernel's."""
     m, k = a.shape
+    if m > 16:
+        return False
     n = w.shape[0]
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or w.shape[1] != k:
         return False
@@ -686,11 +693,18 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         return
     if GEMM_BACKEND == "tcgen05" and gemm_tcgen05(a, w, out):
         return
-    with profiling.kernel("library product (torch.mm)"):
-        if out.dtype == torch.bfloat16:
-            torch.mm(a, w.t(), out=out)
-        else:
-            torch.mm(a, w.t(), out_dtype=torch.float32, out=out)
+    if profiling.ENABLED:
+        with profiling.kernel("library product (torch.mm)"):
+            _library_product(a, w, out)
+    else:
+        _library_product(a, w, out)
+
+
+def _library_product(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    if out.dtype == torch.bfloat16:
+        torch.mm(a, w.t(), out=out)
+    else:
+        torch.mm(a, w.t(), out_dtype=torch.float32, out=out)
 
 
 def gated_linear(ctx, a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, gating=None) -> None:
@@ -753,6 +767,7 @@ _TICKETS = 1 << 16
 _decode_tickets = {}
 
 
+@functools.lru_cache(maxsize=256)
 def decode_tc_supported(dtype: torch.dtype, n_heads: int, n_kv_heads: int, head_dim: int, page_size: int) -> bool:
     """Whether the tensor-core decode kernel takes these sizes (bfloat16, head size 64 or 128,
     groups up to 16, pages that divide 64)."""
@@ -846,6 +861,7 @@ def paged_attention_decode_qkv(qkv: torch.Tensor, q_weight: Optional[torch.Tenso
           "paged_attention_decode_tc_qkv", kernels=1 if tickets is not None else 2)
 
 
+@functools.lru_cache(maxsize=256)
 def prefill_tc_supported(dtype: torch.dtype, n_heads: int, n_kv_heads: int, head_dim: int, page_size: int) -> bool:
     if dtype != torch.bfloat16:
         return False
@@ -877,6 +893,7 @@ def paged_attention_prefill_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: to
           "paged_attention_prefill_tc")
 
 
+@functools.lru_cache(maxsize=256)
 def prefill_tcgen05_supported(dtype: torch.dtype, n_heads: int, n_kv_heads: int, head_dim: int, page_size: int) -> bool:
     if dtype != torch.bfloat16:
         return False
