@@ -488,55 +488,374 @@ general_tiled_kernel(const float* __restrict__ q, const T* __restrict__ k_pool, 
 // out[row] = sum over the splits, in their order, of their partial outputs weighted by exp(m_split - m_all), over the
 // weighted sum of their sums.  One block per (token, head).
 // (With `sigmoid` the partial outputs are added as they are; a row's columns turn back where the launch says so.)
+// Every warp takes the weights of 32 splits side by side, a lane one; a thread's columns of those splits are asked for before the
+// weights are known, so that one trip to L2 brings all of it.
 template <typename T>
 __global__ void general_combine_kernel(const float* __restrict__ partial, T* __restrict__ out, const float* __restrict__ sinks,
                                        int n_splits, const GeneralShape sh) {
+    pdl_trigger();
     pdl_wait();
     const size_t row = blockIdx.x;
-    const int Hq = sh.Hq, Dv = sh.Dv, out_f32 = sh.out_f32;
+    const int Hq = sh.Hq, Dv = sh.Dv, lane = threadIdx.x & 31;
     const float* pp = partial + row * n_splits * (Dv + 2);
-    if (sh.sigmoid) {                                        // uniform over the grid
-        auto column = [&](int c) {
-            float o = 0.0f;
-            for (int z = 0; z < n_splits; ++z) o += pp[(size_t)z * (Dv + 2) + 2 + c];
-            return o;
-        };
-        if (sh.out_cos) {                                    // a thread takes both columns of a pair
+    float m_all = -INFINITY, l_all = 0.0f;
+    if (!sh.sigmoid && n_splits > 32) {
+        for (int z = lane; z < n_splits; z += 32) m_all = fmaxf(m_all, pp[(size_t)z * (Dv + 2)]);
+        m_all = warp_max(m_all);
+    }
+    float o[2] = {0.0f, 0.0f};                               // this thread's columns (at most 512 in blocks of 256)
+    for (int z0 = 0; z0 < n_splits; z0 += 32) {
+        const int nz = min(32, n_splits - z0);
+        float v[2][32];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int c = threadIdx.x + i * blockDim.x;
+#pragma unroll
+            for (int z = 0; z < 32; ++z) v[i][z] = (z < nz && c < Dv) ? pp[(size_t)(z0 + z) * (Dv + 2) + 2 + c] : 0.0f;
+        }
+        float w = lane < nz ? 1.0f : 0.0f;
+        if (!sh.sigmoid) {                                   // uniform over the grid
+            const float* mine = pp + (size_t)(z0 + min(lane, nz - 1)) * (Dv + 2);
+            const float m = lane < nz ? mine[0] : -INFINITY, l = mine[1];
+            if (n_splits <= 32) m_all = warp_max(m);
+            w = m != -INFINITY ? expf(m - m_all) : 0.0f;
+            l_all += warp_sum(w != 0.0f ? l * w : 0.0f);
+        }
+#pragma unroll
+        for (int z = 0; z < 32; ++z) {
+            const float wz = __shfl_sync(0xffffffffu, w, z);
+            if (wz != 0.0f) {                                // uniform over the warp
+                o[0] = fmaf(v[0][z], wz, o[0]);
+                o[1] = fmaf(v[1][z], wz, o[1]);
+            }
+        }
+    }
+    if (sh.sigmoid) l_all = 1.0f;
+    else if (sinks) l_all += expf(sinks[row % Hq] - m_all);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        float v = o[i] / l_all;
+        if (sh.out_cos) {                                    // uniform over the grid; the pair's other column is the neighbouring lane's
+            const float other = __shfl_xor_sync(0xffffffffu, v, 1);
             const size_t at = row / Hq * (Dv >> 1);
-            for (int m = threadIdx.x; m < (Dv >> 1); m += blockDim.x) {
-                const float u = column(2 * m), v = column(2 * m + 1);
-                store_out(out, row * Dv + 2 * m, turned_back(u, v, m, 1, sh.out_cos + at, sh.out_sin + at), out_f32);
-                store_out(out, row * Dv + 2 * m + 1, turned_back(v, u, m, 0, sh.out_cos + at, sh.out_sin + at), out_f32);
+            if (c < Dv) v = turned_back(v, other, c >> 1, !(c & 1), sh.out_cos + at, sh.out_sin + at);
+        }
+        if (c < Dv) store_out(out, row * Dv + c, v, sh.out_f32);
+    }
+}
+
+// ---------------------------------------------------------------- the tiled form on the tensor cores
+// The same blocks, tiles, splits and partial results as above for bfloat16 pools, with both products on mma.sync (m16n8k16: a
+// block's 16 rows are one fragment).  Queries and softmax weights keep their 24 bits: each is the sum of three bfloat16 numbers
+// (x = hi + mid + lo, exact to float32's last bit or one below) and every product is three MMAs into one float32 accumulator;
+// keys and values are bfloat16 in the cache and exact as they are.  Where the time went before: shared memory, which a
+// multiply-add on the CUDA cores reads half a word for; the matrix instruction reads a staged row once per 16 rows.
+// The four warps share the key's width for the scores (a warp holds its share of the 16 queries in registers from the start, KS
+// steps of 16 elements, and adds its part to the others' through shared memory, in warp order) and the value's width for the
+// outputs (VT tiles of 8 columns).  Every warp takes the same softmax.  Tiles are fetched one ahead.
+constexpr int kSRow = kTile + 4;        // floats of a row of partial scores
+
+// x as a sum of three bfloat16 pairs: element pairs packed as mma wants them.  An infinite number is its own first part and
+// has nothing left.
+__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    hi = pack_bf16(x, y);
+    x = fabsf(x) == INFINITY ? 0.0f : x - __uint_as_float(hi << 16);
+    y = fabsf(y) == INFINITY ? 0.0f : y - __uint_as_float(hi & 0xffff0000u);
+    mid = pack_bf16(x, y);
+    x -= __uint_as_float(mid << 16);
+    y -= __uint_as_float(mid & 0xffff0000u);
+    lo = pack_bf16(x, y);
+}
+
+template <int KS, int VT>
+__global__ void __launch_bounds__(128)
+general_rows_tc_kernel(const float* __restrict__ q, const bf16* __restrict__ k_pool, const bf16* __restrict__ v_pool, bf16* __restrict__ out,
+                       float* __restrict__ partial, const int* __restrict__ block_table, const int* __restrict__ cu_q,
+                       const int* __restrict__ kv_len, const float* __restrict__ slopes, const float* __restrict__ sinks,
+                       const TiledShape ts, const PoolBounds bounds) {
+    pdl_wait();
+    const GeneralShape& sh = ts.g;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int Dk = sh.Dk, Dv = sh.Dv, GH = sh.Hq / sh.Hkv;
+    float* s_s = reinterpret_cast<float*>(smem_raw);                          // [4 warps][kRows][kSRow] partial scores
+    bf16* kv_s = reinterpret_cast<bf16*>(s_s + 4 * kRows * kSRow);            // two stages of [kTile][k_row] (and [kTile][v_row])
+    const size_t stage = (size_t)kTile * (ts.k_row + (ts.v_in_k ? 0 : ts.v_row));
+
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = blockIdx.y, split = blockIdx.z;
+    int tile = blockIdx.x, s = 0, q0 = 0, q_len = 0;
+    for (; s < ts.n_seqs; ++s) {
+        q0 = cu_q[s];
+        q_len = cu_q[s + 1] - q0;
+        const int nt = (q_len * GH + kRows - 1) / kRows;
+        if (tile < nt) break;
+        tile -= nt;
+    }
+    if (s >= ts.n_seqs) return;
+    const int ctx0 = kv_len[s] - q_len;
+    const int idx0 = tile * kRows;
+    const int n_rows = min(kRows, q_len * GH - idx0);
+    const int* table = block_table + (size_t)s * sh.table_stride;
+
+    // the block's span of keys: lowest keys ascend with the rows' positions, so the first row sees the lowest key, the last the highest
+    auto lowest = [&](int p) {
+        int lo = 0;
+        if (sh.window > 0 && p - sh.window + 1 > lo) lo = p - sh.window + 1;
+        if (sh.chunk > 0 && (p / sh.chunk) * sh.chunk > lo) lo = (p / sh.chunk) * sh.chunk;
+        return lo;
+    };
+    const int lo_blk = lowest(ctx0 + idx0 / GH), hi_blk = ctx0 + (idx0 + n_rows - 1) / GH;
+    const int kt0 = lo_blk / kTile, n_kept = kept_tiles(lo_blk, sh.keep_first);
+    const int n_tiles = n_kept + hi_blk / kTile - kt0 + 1;
+    const int per = (n_tiles + ts.n_splits - 1) / ts.n_splits;
+    const int t_begin = split * per, t_end = min(n_tiles, t_begin + per);
+
+    auto load = [&](int ti) {
+        const int j0 = (ti < n_kept ? ti : kt0 + ti - n_kept) * kTile;
+        bf16* k_s = kv_s + (ti & 1) * stage;
+        bf16* v_s = k_s + (size_t)kTile * ts.k_row;
+        const int key = threadIdx.x >> 2, sub = threadIdx.x & 3, j = j0 + key;
+        const bool ok = j <= hi_blk && (j >= lo_blk || j < sh.keep_first);   // rows outside the block's span are filled with zeros
+        const bf16* k_src = k_pool;
+        const bf16* v_src = v_pool;
+        if (ok) {
+            int page = table[j / sh.page_size];
+            if (!page_ok(page, bounds)) page = 0;
+            k_src += (((size_t)page * sh.Hkv + g) * sh.page_size + j % sh.page_size) * sh.k_stride;
+            v_src += (((size_t)page * (sh.Hkv / sh.v_share) + g / sh.v_share) * sh.page_size + j % sh.page_size) * sh.v_stride;
+        }
+        for (int part = sub; part < Dk / 8; part += 4) cp_async16(smem_u32(k_s + (size_t)key * ts.k_row + part * 8), k_src + part * 8, ok);
+        if (!ts.v_in_k)
+            for (int part = sub; part < Dv / 8; part += 4) cp_async16(smem_u32(v_s + (size_t)key * ts.v_row + part * 8), v_src + part * 8, ok);
+    };
+    if (t_begin < t_end) load(t_begin);
+    cp_async_commit();
+
+    // this thread's two rows of the fragments
+    int pos[2], lo_r[2], tok[2], head[2];
+    float slope[2], bias[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int row = (lane >> 2) + 8 * r;
+        const bool on = row < n_rows;
+        const int idx = idx0 + (on ? row : 0);
+        tok[r] = q0 + idx / GH;
+        head[r] = g * GH + idx % GH;
+        pos[r] = on ? ctx0 + idx / GH : -1;                  // -1: sees no key
+        lo_r[r] = on ? lowest(pos[r]) : 0;
+        slope[r] = slopes ? slopes[head[r]] : 0.0f;
+        bias[r] = (sh.sigmoid && sh.score_bias) ? sh.score_bias[head[r]] : 0.0f;
+    }
+    // this warp's share of the queries, split: [step][a register of the fragment: (row, row + 8) x (8 columns, the next 8)]
+    const int steps = Dk / 16;
+    uint32_t qf[3][KS][4];
+#pragma unroll
+    for (int i = 0; i < KS; ++i) {
+        const int ks = warp * KS + i;
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            const int r = f & 1, col = ks * 16 + (f >> 1) * 8 + (lane & 3) * 2;
+            float2 v = make_float2(0.0f, 0.0f);
+            if (ks < steps && pos[r] >= 0) v = *reinterpret_cast<const float2*>(q + ((size_t)tok[r] * sh.Hq + head[r]) * Dk + col);
+            split3(v.x, v.y, qf[0][i][f], qf[1][i][f], qf[2][i][f]);
+        }
+    }
+
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f}, acc[VT][4];
+#pragma unroll
+    for (int i = 0; i < VT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
+
+    for (int ti = t_begin; ti < t_end; ++ti) {
+        cp_async_wait<0>();
+        __syncthreads();                                   // the tile has landed; the one before it, and its scores, are done with
+        if (ti + 1 < t_end) load(ti + 1);
+        cp_async_commit();
+        const int j0 = (ti < n_kept ? ti : kt0 + ti - n_kept) * kTile;
+        const bf16* k_s = kv_s + (ti & 1) * stage;
+        const bf16* v_s = ts.v_in_k ? k_s : k_s + (size_t)kTile * ts.k_row;
+
+        // this warp's part of the scores of 32 keys; the queries' first parts and the small rest in accumulators of their own
+        // (an MMA cuts off what falls below its accumulator's last bits)
+        float sc[4][4], sr[4][4];
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sc[n][e] = sr[n][e] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < KS; ++i) {
+            const int ks = warp * KS + i;
+            if (ks < steps) {                               // uniform over the warp
+#pragma unroll
+                for (int n2 = 0; n2 < 2; ++n2) {
+                    uint32_t b[4];                          // keys 16 n2 .. + 7: two registers, the next 8 keys: two more
+                    const int key = n2 * 16 + (lane & 7) + (lane >> 4) * 8, col = ks * 16 + (lane >> 3 & 1) * 8;
+                    ldmatrix_x4(b, smem_u32(k_s + (size_t)key * ts.k_row + col));
+#pragma unroll
+                    for (int p = 2; p >= 0; --p) {
+                        mma_bf16(p ? sr[2 * n2] : sc[2 * n2], qf[p][i], b[0], b[1]);
+                        mma_bf16(p ? sr[2 * n2 + 1] : sc[2 * n2 + 1], qf[p][i], b[2], b[3]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                *reinterpret_cast<float2*>(s_s + (warp * kRows + (lane >> 2) + 8 * r) * kSRow + n * 8 + (lane & 3) * 2) =
+                    make_float2(sc[n][2 * r] + sr[n][2 * r], sc[n][2 * r + 1] + sr[n][2 * r + 1]);
+        __syncthreads();
+
+        // the softmax weights of this thread's two rows: keys 8 n + 2 (lane mod 4) + {0, 1}, the columns of the scores' fragments
+        float pw[4][4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float m_tile = -INFINITY;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                float2 x = make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const float2 y = *reinterpret_cast<const float2*>(s_s + (w * kRows + (lane >> 2) + 8 * r) * kSRow + n * 8 + (lane & 3) * 2);
+                    x.x += y.x;
+                    x.y += y.y;
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int j = j0 + n * 8 + (lane & 3) * 2 + e;
+                    const float raw = e ? x.y : x.x;
+                    const bool vis = j <= pos[r] && (j >= lo_r[r] || j < sh.keep_first);
+                    const float v = vis ? (sh.softcap > 0.0f ? cap_score(raw * sh.scale, sh.softcap) - slope[r] * (float)(pos[r] - j)
+                                                             : fmaf(raw, sh.scale, -slope[r] * (float)(pos[r] - j)))
+                                        : -INFINITY;
+                    pw[n][2 * r + e] = v;
+                    m_tile = fmaxf(m_tile, v);
+                }
+            }
+            if (sh.sigmoid) {                               // uniform over the grid
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float v = pw[n][2 * r + e];
+                        pw[n][2 * r + e] = v == -INFINITY ? 0.0f : sigmoid_weight(v + bias[r]);
+                    }
+                continue;
+            }
+            m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 1));
+            m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 2));
+            const float m_new = fmaxf(m_run[r], m_tile);
+            float corr = 1.0f, sum = 0.0f;
+            if (m_new != -INFINITY) corr = expf(m_run[r] - m_new);      // 0 while the row had seen nothing
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float v = pw[n][2 * r + e];
+                    const float p = v == -INFINITY ? 0.0f : expf(v - m_new);
+                    pw[n][2 * r + e] = p;
+                    sum += p;
+                }
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            l_run[r] = l_run[r] * corr + sum;
+            m_run[r] = m_new;
+            if (corr != 1.0f) {
+#pragma unroll
+                for (int i = 0; i < VT; ++i) {
+                    acc[i][2 * r] *= corr;
+                    acc[i][2 * r + 1] *= corr;
+                }
+            }
+        }
+        // outputs: this warp's columns.  A tile's sums begin at zero and join the others in an addition of their own, rounded to
+        // nearest: the MMAs' cut-off would add up over a long row of keys.
+        uint32_t pf[2][3][4];                               // [16 keys][part][register: (row, row + 8) of the first 8 keys, of the next 8]
+#pragma unroll
+        for (int k2 = 0; k2 < 2; ++k2)
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                const int n = 2 * k2 + (f >> 1), r = f & 1;
+                split3(pw[n][2 * r], pw[n][2 * r + 1], pf[k2][0][f], pf[k2][1][f], pf[k2][2][f]);
+            }
+#pragma unroll
+        for (int i = 0; i < VT; i += 2) {
+            const int col = (warp * VT + i) * 8;
+            if (col >= Dv) break;                           // uniform over the warp; Dv is a multiple of 16
+            float o[2][4], rest[2][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[0][e] = o[1][e] = rest[0][e] = rest[1][e] = 0.0f;
+#pragma unroll
+            for (int k2 = 0; k2 < 2; ++k2) {
+                uint32_t b[4];                              // columns col .. + 7: two registers (8 keys each), the next 8 columns: two more
+                const int key = k2 * 16 + (lane & 7) + (lane >> 3 & 1) * 8;
+                ldmatrix_x4_trans(b, smem_u32(v_s + (size_t)key * ts.v_row + col + (lane >> 4) * 8));
+#pragma unroll
+                for (int p = 2; p >= 0; --p) {
+                    mma_bf16(p ? rest[0] : o[0], pf[k2][p], b[0], b[1]);
+                    mma_bf16(p ? rest[1] : o[1], pf[k2][p], b[2], b[3]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc[i][e] += o[0][e] + rest[0][e];
+                acc[i + 1][e] += o[1][e] + rest[1][e];
+            }
+        }
+    }
+    cp_async_wait<0>();
+    pdl_trigger();
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        if (pos[r] < 0) continue;
+        const size_t row = (size_t)tok[r] * sh.Hq + head[r];
+        if (ts.n_splits == 1) {
+            const float inv = sh.sigmoid ? 1.0f : 1.0f / (sinks ? l_run[r] + expf(sinks[head[r]] - m_run[r]) : l_run[r]);
+            const size_t at = (size_t)tok[r] * (Dv >> 1);
+#pragma unroll
+            for (int i = 0; i < VT; ++i) {
+                const int c = (warp * VT + i) * 8 + (lane & 3) * 2;
+                if (c >= Dv) break;
+                float u = acc[i][2 * r] * inv, v = acc[i][2 * r + 1] * inv;
+                if (sh.out_cos) {                           // uniform over the grid; both columns of a pair are this thread's
+                    const float a = turned_back(u, v, c >> 1, 1, sh.out_cos + at, sh.out_sin + at);
+                    v = turned_back(v, u, c >> 1, 0, sh.out_cos + at, sh.out_sin + at);
+                    u = a;
+                }
+                store_out(out, row * Dv + c, u, sh.out_f32);
+                store_out(out, row * Dv + c + 1, v, sh.out_f32);
             }
         } else {
-            for (int c = threadIdx.x; c < Dv; c += blockDim.x) store_out(out, row * Dv + c, column(c), out_f32);
+            float* pp = partial + (row * ts.n_splits + split) * (Dv + 2);
+            if (warp == 0 && (lane & 3) == 0) { pp[0] = m_run[r]; pp[1] = l_run[r]; }
+#pragma unroll
+            for (int i = 0; i < VT; ++i) {
+                const int c = (warp * VT + i) * 8 + (lane & 3) * 2;
+                if (c >= Dv) break;
+                *reinterpret_cast<float2*>(pp + 2 + c) = make_float2(acc[i][2 * r], acc[i][2 * r + 1]);
+            }
         }
-        return;
     }
-    float m_all = -INFINITY;
-    for (int z = 0; z < n_splits; ++z) m_all = fmaxf(m_all, pp[(size_t)z * (Dv + 2)]);
-    float l_all = 0.0f;
-    for (int z = 0; z < n_splits; ++z) {
-        const float m = pp[(size_t)z * (Dv + 2)];
-        if (m != -INFINITY) l_all += pp[(size_t)z * (Dv + 2) + 1] * expf(m - m_all);
-    }
-    if (sinks) l_all += expf(sinks[row % Hq] - m_all);
-    auto column = [&](int c) {
-        float o = 0.0f;
-        for (int z = 0; z < n_splits; ++z) {
-            const float m = pp[(size_t)z * (Dv + 2)];
-            if (m != -INFINITY) o += pp[(size_t)z * (Dv + 2) + 2 + c] * expf(m - m_all);
-        }
-        return o / l_all;
-    };
-    for (int c = threadIdx.x; c < Dv; c += blockDim.x) {
-        float o = column(c);
-        if (sh.out_cos) {
-            const size_t at = row / Hq * (Dv >> 1);
-            o = turned_back(o, column(c ^ 1), c >> 1, !(c & 1), sh.out_cos + at, sh.out_sin + at);
-        }
-        store_out(out, row * Dv + c, o, out_f32);
-    }
+}
+
+// Shared memory of the kernel above; 0 where it does not take the sizes (key and value widths in steps of 16 up to 576 and 512).
+size_t rows_tc_smem(const TiledShape& ts) {
+    const GeneralShape& sh = ts.g;
+    if (sh.Dk % 16 || sh.Dv % 16 || sh.Dk > 576 || sh.Dv > 512) return 0;
+    return sizeof(float) * 4 * kRows * kSRow + 2 * sizeof(bf16) * kTile * ((size_t)ts.k_row + (ts.v_in_k ? 0 : ts.v_row));
+}
+
+template <int KS, int VT>
+int launch_rows_tc(const float* q, const void* k_pool, const void* v_pool, void* out, float* partial, const int* block_table,
+                   const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int row_tiles, const TiledShape& ts,
+                   size_t smem, cudaStream_t stream) {
+    static const cudaError_t allowed = cudaFuncSetAttribute(general_rows_tc_kernel<KS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (allowed != cudaSuccess) return (int)allowed;
+    return launch_pdl(general_rows_tc_kernel<KS, VT>, dim3(row_tiles, ts.g.Hkv, ts.n_splits), dim3(128), smem, stream, q, (const bf16*)k_pool,
+                      (const bf16*)v_pool, (bf16*)out, partial, block_table, cu_q, kv_len, slopes, sinks, ts, pb::pool_bounds_now());
 }
 
 template <typename T>
@@ -546,8 +865,8 @@ size_t tiled_smem(const TiledShape& ts) {
 
 template <typename T, int ACC>
 int launch_tiled(const float* q, const void* k_pool, const void* v_pool, void* out, float* partial, const int* block_table,
-                 const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int n_tokens, int row_tiles,
-                 const TiledShape& ts, cudaStream_t stream) {
+                 const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int row_tiles, const TiledShape& ts,
+                 cudaStream_t stream) {
     const size_t smem = tiled_smem<T>(ts);
     static size_t allowed = 48 * 1024;                     // per instantiation
     if (smem > allowed) {
@@ -556,15 +875,8 @@ int launch_tiled(const float* q, const void* k_pool, const void* v_pool, void* o
         allowed = smem;
     }
     dim3 grid(row_tiles, ts.g.Hkv, ts.n_splits);
-    int status = launch_pdl(general_tiled_kernel<T, ACC>, grid, dim3(128), smem, stream, q, (const T*)k_pool, (const T*)v_pool, (T*)out, partial,
-                            block_table, cu_q, kv_len, slopes, sinks, ts, pb::pool_bounds_now());
-    if (status == 0 && ts.n_splits > 1) {
-        int b = 32;
-        while (b < ts.g.Dv && b < 256) b <<= 1;
-        status = launch_pdl(general_combine_kernel<T>, dim3(n_tokens * ts.g.Hq), dim3(b), 0, stream, (const float*)partial, (T*)out, sinks,
-                            ts.n_splits, ts.g);
-    }
-    return status;
+    return launch_pdl(general_tiled_kernel<T, ACC>, grid, dim3(128), smem, stream, q, (const T*)k_pool, (const T*)v_pool, (T*)out, partial,
+                      block_table, cu_q, kv_len, slopes, sinks, ts, pb::pool_bounds_now());
 }
 
 template <typename T>
@@ -584,14 +896,43 @@ bool tiled_shape(TiledShape& ts, const void* k_pool, const void* v_pool) {
 
 template <typename T>
 int dispatch_tiled(const float* q, const void* k_pool, const void* v_pool, void* out, float* partial, const int* block_table,
-                   const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int n_tokens, int row_tiles,
-                   const TiledShape& ts, cudaStream_t stream) {
-#define PB_TILED(A) return launch_tiled<T, A>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, n_tokens, row_tiles, ts, stream)
+                   const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int row_tiles, const TiledShape& ts,
+                   cudaStream_t stream) {
+#define PB_TILED(A) return launch_tiled<T, A>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, row_tiles, ts, stream)
     if (ts.g.Dv <= 64) PB_TILED(2);
     if (ts.g.Dv <= 128) PB_TILED(4);
     if (ts.g.Dv <= 256) PB_TILED(8);
     PB_TILED(16);
 #undef PB_TILED
+}
+
+// bfloat16 pools take the tensor-core form where it takes the widths, else the CUDA-core form.  us with the merge, CUDA cores -> tensor
+// cores, 8 sequences at 1,900 keys: 16 heads on one row of 576 / 512, 32 splits 60.5 -> 22.7; 16 on 4 heads of 128 / 128, chunks of
+// 1,024, 16 splits 26.7 -> 15.1; the smallest (2 sequences, 8 heads on 4 of 64 / 64, 90 and 333 keys) 7.6 -> 8.2.  Relative error of
+// float32 rows against 64 bits on the first: 5.7e-7 -> 2.0e-7.
+int dispatch_tiled_bf16(const float* q, const void* k_pool, const void* v_pool, void* out, float* partial, const int* block_table,
+                        const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int row_tiles, TiledShape ts,
+                        cudaStream_t stream) {
+    const int v_row = ts.v_row;
+    if (!ts.v_in_k) ts.v_row = (ts.g.Dv / 8 | 1) * 8;       // value rows an odd number of 16-byte units apart as well
+    const size_t smem = rows_tc_smem(ts);
+#define PB_ROWS_TC(K, V) return launch_rows_tc<K, V>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, row_tiles, ts, smem, stream)
+    if (smem > 0 && smem <= 200 * 1024) {
+        if (ts.g.Dk <= 128 && ts.g.Dv <= 128) PB_ROWS_TC(2, 4);
+        if (ts.g.Dk <= 192 && ts.g.Dv <= 128) PB_ROWS_TC(3, 4);
+        if (ts.g.Dk <= 320 && ts.g.Dv <= 256) PB_ROWS_TC(5, 8);
+        PB_ROWS_TC(9, 16);
+    }
+#undef PB_ROWS_TC
+    ts.v_row = v_row;
+    return dispatch_tiled<bf16>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, row_tiles, ts, stream);
+}
+
+template <typename T>
+int launch_combine(const float* partial, void* out, const float* sinks, int n_tokens, const TiledShape& ts, cudaStream_t stream) {
+    int b = 32;
+    while (b < ts.g.Dv && b < 256) b <<= 1;
+    return launch_pdl(general_combine_kernel<T>, dim3(n_tokens * ts.g.Hq), dim3(b), 0, stream, partial, (T*)out, sinks, ts.n_splits, ts.g);
 }
 
 // One warp per (token, head) of the fused projection row [q: Hq*Dk | k: Hk*Dk | v: Hv*Dv]:
@@ -708,12 +1049,15 @@ PB_EXPORT int pb_paged_attention_general_tiled(int dtype, const float* q, const 
                         out_f32 != 0, sigmoid != 0, score_bias, out_cos, out_sin};
     ts.n_seqs = n_seqs;
     ts.n_splits = n_splits;
+    int status;
     if (dtype == PB_F32) {
         tiled_shape<float>(ts, k_pool, v_pool);
-        return dispatch_tiled<float>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, n_tokens, row_tiles, ts,
-                                     stream);
+        status = dispatch_tiled<float>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, row_tiles, ts, stream);
+        if (status == 0 && n_splits > 1) status = launch_combine<float>(partial, out, sinks, n_tokens, ts, stream);
+    } else {
+        tiled_shape<bf16>(ts, k_pool, v_pool);
+        status = dispatch_tiled_bf16(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, row_tiles, ts, stream);
+        if (status == 0 && n_splits > 1) status = launch_combine<bf16>(partial, out, sinks, n_tokens, ts, stream);
     }
-    tiled_shape<__nv_bfloat16>(ts, k_pool, v_pool);
-    return dispatch_tiled<__nv_bfloat16>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, n_tokens, row_tiles,
-                                         ts, stream);
+    return status;
 }

@@ -988,7 +988,8 @@ def squared_relu_linear(ctx, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor
 # ---------------------------------------------------------------- attention in its general form, latent attention
 # The general attention has two kernels: the tiled one (keys and values of a tile staged in shared memory and shared by 16
 # query rows; splits of the keys where the rows alone do not fill the GPU) for rows that are multiples of 16 bytes, and the
-# plain one (a block per token and head) for every other size.  PULSAR_GENERAL_TILED=0 leaves the tiled one out.
+# plain one (a block per token and head) for every other size.  On bfloat16 pools whose widths are steps of 16 (keys up to 576, values
+# up to 512) the tiled one runs on the tensor cores, with queries and weights in three parts.  PULSAR_GENERAL_TILED=0 leaves it out.
 GENERAL_TILED = os.environ.get("PULSAR_GENERAL_TILED", "1") != "0"
 GENERAL_ROWS = 16
 # Steps with portions of GENERAL_TC_MIN tokens or more, on bfloat16 pages with (key, value) widths (64, 64), (64, 128), (128, 128) or

@@ -1,0 +1,100 @@
+"""The general attention's form for a few rows on the tensor cores against float64."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _paged(q_lens, kv_lens, page, pools, dtype, gen):
+    """A shuffled block table and random pools [pages, heads, page, width], one per (heads, width)."""
+    need = [-(-k // page) for k in kv_lens]
+    ids = torch.randperm(sum(need) + 2, generator=gen).to(torch.int32)
+    table = torch.full((len(need), max(need) + 1), -1, dtype=torch.int32)
+    for s, n in enumerate(need):
+        table[s, :n] = ids[sum(need[:s]):sum(need[:s]) + n]
+    made = [torch.randn(len(ids), h, page, w, generator=gen).to(dtype).cuda() for h, w in pools]
+    return table, made
+
+
+def _keys_of(pool, table, s, kl, page):
+    key = torch.arange(kl)
+    return pool[table[s, key // page].long().cuda(), :, (key % page).cuda()].double()
+
+
+class _Ctx:
+    """What the general attention asks of a step."""
+
+    def __init__(self, q_lens, kv_lens):
+        self.host = type("Host", (), {"q_lens": q_lens})()
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")                      # noqa: E731
+        self.cu_q, self.kv_len = i32([sum(q_lens[:i]) for i in range(len(q_lens) + 1)]), i32(kv_lens)
+        self.seq_of_token = torch.repeat_interleave(torch.arange(len(q_lens), device="cuda"), i32(q_lens)).to(torch.int32)
+
+    def scratch(self, tag, shape, dtype):
+        return torch.full(shape, float("nan"), dtype=dtype, device="cuda")
+
+
+# every instance of the kernel at its largest and at an odd size; one long row of keys (what an MMA cuts off must not add up)
+@pytest.mark.parametrize("q_lens,kv_lens,hq,hkv,dk,dv,opts", [
+    ([1, 1], [1900, 70], 16, 1, 576, 512, {}), ([3, 1], [40, 70], 5, 1, 576, 512, dict(sinks=True)),
+    ([1, 2], [1000, 64], 32, 1, 320, 256, {}), ([1, 15], [190, 333], 6, 2, 192, 128, dict(page=5)),
+    ([1] * 3, [100, 1024, 1025], 16, 4, 128, 128, dict(slopes=True, chunk=64)), ([1, 7], [90, 333], 8, 1, 80, 48, dict(sinks=True)),
+    ([1, 5, 2], [64, 37, 300], 12, 4, 64, 64, dict(window=50, keep_first=4, softcap=20.0, sinks=True)),
+    ([2, 1], [90, 33], 8, 2, 64, 128, dict(sigmoid=True, turn=True)), ([1, 1], [90, 2333], 8, 4, 64, 64, dict(sigmoid=True, v_share=2)),
+    ([1], [1], 2, 1, 16, 16, {})])
+def test_few_rows_on_the_tensor_cores(q_lens, kv_lens, hq, hkv, dk, dv, opts):
+    from pulsar_b200 import ops
+    gen = torch.Generator().manual_seed(dk + hq)
+    page, share, n = opts.get("page", 16), opts.get("v_share", 1), sum(q_lens)
+    latent = dk in (576, 320)                                # the value is part of the key's row
+    table, pools = _paged(q_lens, kv_lens, page, [(hkv, dk)] if latent else [(hkv, dk), (hkv // share, dv)], torch.bfloat16, gen)
+    k_pool, v_pool = pools[0], pools[-1]
+    q = torch.randn(n, hq, dk, generator=gen).cuda()
+    vec = lambda on: torch.randn(hq, generator=gen).cuda() if on else None                     # noqa: E731
+    slopes, sinks, bias = vec(opts.get("slopes")), vec(opts.get("sinks")), vec(opts.get("sigmoid"))
+    slopes = slopes.abs() * 0.1 if slopes is not None else None
+    angle = (torch.rand(n, dv // 2, generator=gen) * 6).cuda()
+    turn = (angle.cos(), angle.sin()) if opts.get("turn") else None
+    ctx = _Ctx(q_lens, kv_lens)
+    got = {}
+    for dtype in (torch.float32, torch.bfloat16):
+        got[dtype] = torch.full((n, hq, dv), float("nan"), dtype=dtype, device="cuda")
+        ops.paged_attention_general(ctx, q, k_pool, v_pool, got[dtype], table.cuda(), dk ** -0.5, opts.get("window"), opts.get("chunk"), slopes,
+                                    value_width=dv, tensor_cores=False, keep_first=opts.get("keep_first", 0), softcap=opts.get("softcap"),
+                                    sinks=sinks, v_share=share, sigmoid=bool(opts.get("sigmoid")), score_bias=bias, turn_back=turn)
+    at = 0
+    want = torch.empty(n, hq, dv, dtype=torch.float64, device="cuda")
+    for s, (m, kl) in enumerate(zip(q_lens, kv_lens)):
+        k = _keys_of(k_pool, table, s, kl, page).repeat_interleave(hq // hkv, dim=1)
+        v = _keys_of(v_pool, table, s, kl, page)[..., :dv].repeat_interleave(hq // hkv * share, dim=1)
+        pos, key = torch.arange(kl - m, kl, device="cuda")[:, None], torch.arange(kl, device="cuda")[None]
+        low = torch.zeros_like(pos)
+        if opts.get("window"):
+            low = torch.maximum(low, pos - opts["window"] + 1)
+        if opts.get("chunk"):
+            low = torch.maximum(low, pos // opts["chunk"] * opts["chunk"])
+        seen = (key <= pos) & ((key >= low) | (key < opts.get("keep_first", 0)))
+        sc = torch.einsum("ihd,jhd->hij", q[at:at + m].double(), k) * dk ** -0.5
+        if opts.get("softcap"):
+            sc = opts["softcap"] * torch.tanh(sc / opts["softcap"])
+        if slopes is not None:
+            sc = sc - slopes.double()[:, None, None] * (pos - key)
+        if opts.get("sigmoid"):
+            w = torch.sigmoid(sc + bias.double()[:, None, None]) * seen
+        else:
+            sc = sc.masked_fill(~seen, -math.inf)
+            if sinks is not None:
+                sc = torch.cat([sc, sinks.double()[:, None, None].expand(hq, m, 1)], dim=-1)
+            w = torch.softmax(sc, dim=-1)[..., :kl]
+        out = torch.einsum("hij,jhv->ihv", w, v)
+        if turn is not None:
+            c, sn = turn[0][at:at + m].double()[:, None], turn[1][at:at + m].double()[:, None]
+            u, t = out[..., 0::2], out[..., 1::2]
+            out = torch.stack([u * c + t * sn, t * c - u * sn], dim=-1).flatten(-2)
+        want[at:at + m] = out
+        at += m
+    # float32 rows: scores of up to 576 products and sums over the keys, each a few units in the last place off
+    assert float((got[torch.float32].double() - want).norm() / want.norm()) < 1.5e-6
+    assert float((got[torch.bfloat16].double() - want).abs().max() / want.abs().max()) < 2.0 ** -8
