@@ -5,8 +5,8 @@
 //                    expansion W_uk the query side takes q_abs[h] = W_uk[h]^T q_plain[h]
 //                    (so that q_plain . (W_uk[h] c) = q_abs[h] . c), with the value expansion W_uv
 //                    the output side takes W_uv[h] (sum_j p_j c_j).  float32 accumulation.  A few tokens: a
-//                    block takes 8 tokens x 32 outputs, four slices of K in ascending k each, added in slice
-//                    order (enough blocks to fill the GPU).  Many tokens: 8 tokens x 128 outputs, K whole.
+//                    block takes 8 tokens x 64 outputs, eight slices of K in ascending k each, added in slice
+//                    order.  Many tokens: 8 tokens x 128 outputs, K whole.
 //                    Optionally multiplies by sigmoid(gate[n, h, :]) (an output gate) in float32.
 //   latent_prepare   per token: RMS norm of the latent part of the down projection (float32),
 //                    rotation of the shared key part at the token's position, both written to
@@ -71,60 +71,121 @@ heads_linear_wide_kernel(const T* __restrict__ a, long a_tok, int a_head, const 
     }
 }
 
-constexpr int kSlices = 4;      // a block's 128 threads: 32 outputs x 4 slices of K
-constexpr int kBatch = 16;      // weights a thread asks for before it uses the first
+// A few tokens: bound by the trips to L2, not by bytes (16 heads of 512 x 128 are 2 MB).  A block takes 8 tokens x 64 outputs; its
+// eight warps are slices of K, a lane two neighbouring outputs (one 4-byte load of bfloat16), 16 k asked for at once and the next
+// 16 while these are used.  The weights depend on no earlier kernel: the first batch is asked for before griddepcontrol.wait.
+// 8 tokens, 16 heads, bfloat16: 512 -> 128 with the gate 12.7 -> 5.5 us, 128 -> 512 to float32 4.6 -> 2.8 (four slices of single
+// outputs before).
+constexpr int kSlices = 8;
+constexpr int kBatch = 16;      // k's a thread asks for at once
+constexpr int kOuts = 64;       // outputs of a block
 
-template <typename T, typename TO>
-__global__ void __launch_bounds__(128)
+__host__ __device__ __forceinline__ int heads_slice(int K) {        // k's per slice, a multiple of kBatch
+    return ((K + kSlices - 1) / kSlices + kBatch - 1) / kBatch * kBatch;
+}
+
+// Two neighbouring weights as they lie in memory, made numbers where they are used: a load that is converted at once holds up the
+// loads behind it.
+template <typename T> struct Pair;
+template <> struct Pair<float> {
+    float2 v;
+    __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float2*>(p); }
+    __device__ __forceinline__ void load(const float* p, const float* q) { v = make_float2(*p, *q); }
+    __device__ __forceinline__ float2 get() const { return v; }
+};
+template <> struct Pair<__nv_bfloat16> {
+    uint32_t v;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint32_t*>(p); }
+    __device__ __forceinline__ void load(const __nv_bfloat16* p, const __nv_bfloat16* q) {
+        v = (uint32_t)*reinterpret_cast<const uint16_t*>(p) | (uint32_t)*reinterpret_cast<const uint16_t*>(q) << 16;
+    }
+    __device__ __forceinline__ float2 get() const { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+};
+
+// kPairs: M is even, so that the weights of two neighbouring outputs stand on pair boundaries.
+template <typename T, typename TO, bool kPairs>
+__global__ void __launch_bounds__(32 * kSlices)
 heads_linear_kernel(const T* __restrict__ a, long a_tok, int a_head, const T* __restrict__ w, TO* __restrict__ out, long o_tok,
                     int o_head, const T* __restrict__ gate, long g_tok, int N, int M, int K) {
-    pdl_wait();         // may have come onto the SMs while the product before it was ending: nothing is touched before that one is done
     extern __shared__ __align__(16) float smem[];
-    const int KS = (((K + kSlices - 1) / kSlices) + kBatch - 1) / kBatch * kBatch;      // k's per slice, a multiple of kBatch
-    const int KP = KS * kSlices;
+    const int KS = heads_slice(K), KP = KS * kSlices;
     float* a_s = smem;                             // [kTok][KP], zeros behind K
-    float* r_s = a_s + kTok * KP;                  // [kSlices][kTok][32] partial sums
+    float* r_s = a_s + kTok * KP;                  // [kSlices][kTok][kOuts] partial sums
     const int n0 = blockIdx.x * kTok, h = blockIdx.y;
     const int nt = min(kTok, N - n0);
-    for (int i = threadIdx.x; i < kTok * KP; i += blockDim.x) {
-        const int tt = i / KP, k = i % KP;
-        a_s[i] = (tt < nt && k < K) ? to_float(a[(size_t)(n0 + tt) * a_tok + (size_t)h * a_head + k]) : 0.0f;
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int m = blockIdx.z * kOuts + 2 * lane;   // this thread's outputs m and m + 1
+    const T* wh = w + (size_t)h * K * M;           // [K, M]: neighbouring threads read neighbouring weights
+    const int k0 = slice * KS;
+    // places behind K or M read the last row or column instead; the ones behind K count as zero below, the others are not stored
+    const T* w0 = wh + (kPairs ? min(m, M - 2) : min(m, M - 1));
+    const T* w1 = wh + min(m + 1, M - 1);
+    auto fetch = [&](Pair<T> (&v)[kBatch], int k) {
+#pragma unroll
+        for (int e = 0; e < kBatch; ++e) {
+            const size_t row = (size_t)min(k + e, K - 1) * M;
+            if (kPairs) v[e].load(w0 + row);
+            else v[e].load(w0 + row, w1 + row);
+        }
+    };
+    Pair<T> wv[2][kBatch];
+    fetch(wv[0], k0);
+    pdl_wait();         // may have come onto the SMs while the product before it was ending: nothing else is touched before that one is done
+    if (K % 4 == 0 && a_tok % 4 == 0 && a_head % 4 == 0 && (uintptr_t)a % 16 == 0) {
+        for (int i = threadIdx.x; i < kTok * (KP >> 2); i += blockDim.x) {
+            const int tt = i / (KP >> 2), k = i % (KP >> 2) * 4;
+            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (tt < nt && k < K) load_quad(a + (size_t)(n0 + tt) * a_tok + (size_t)h * a_head + k, v);
+            store_quad(a_s + tt * KP + k, v);
+        }
+    } else {
+        for (int i = threadIdx.x; i < kTok * KP; i += blockDim.x) {
+            const int tt = i / KP, k = i % KP;
+            a_s[i] = (tt < nt && k < K) ? to_float(a[(size_t)(n0 + tt) * a_tok + (size_t)h * a_head + k]) : 0.0f;
+        }
     }
     __syncthreads();
-    const int mx = threadIdx.x & 31, slice = threadIdx.x >> 5;
-    const int m = blockIdx.z * 32 + mx;
-    const bool live = m < M;
-    const T* wh = w + (size_t)h * K * M + (live ? m : 0);       // [K, M]: neighbouring threads read neighbouring weights
-    float acc[kTok];
+    float2 acc[kTok];
 #pragma unroll
-    for (int tt = 0; tt < kTok; ++tt) acc[tt] = 0.0f;
-    const int k0 = slice * KS;
-    for (int k = k0; k < k0 + KS; k += kBatch) {
-        float wv[kBatch];                          // a batch of weights on their way at once
-#pragma unroll
-        for (int e = 0; e < kBatch; ++e) wv[e] = (live && k + e < K) ? to_float(wh[(size_t)(k + e) * M]) : 0.0f;
+    for (int tt = 0; tt < kTok; ++tt) acc[tt] = make_float2(0.0f, 0.0f);
+    auto use = [&](const Pair<T> (&v)[kBatch], int k) {
 #pragma unroll
         for (int e = 0; e < kBatch; e += 4) {
+            float2 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = k + e + u < K ? v[e + u].get() : make_float2(0.0f, 0.0f);
 #pragma unroll
             for (int tt = 0; tt < kTok; ++tt) {
                 const float4 av = *reinterpret_cast<const float4*>(a_s + tt * KP + k + e);
-                acc[tt] = fmaf(av.x, wv[e], acc[tt]);
-                acc[tt] = fmaf(av.y, wv[e + 1], acc[tt]);
-                acc[tt] = fmaf(av.z, wv[e + 2], acc[tt]);
-                acc[tt] = fmaf(av.w, wv[e + 3], acc[tt]);
+                acc[tt].x = fmaf(av.x, x[0].x, acc[tt].x);
+                acc[tt].y = fmaf(av.x, x[0].y, acc[tt].y);
+                acc[tt].x = fmaf(av.y, x[1].x, acc[tt].x);
+                acc[tt].y = fmaf(av.y, x[1].y, acc[tt].y);
+                acc[tt].x = fmaf(av.z, x[2].x, acc[tt].x);
+                acc[tt].y = fmaf(av.z, x[2].y, acc[tt].y);
+                acc[tt].x = fmaf(av.w, x[3].x, acc[tt].x);
+                acc[tt].y = fmaf(av.w, x[3].y, acc[tt].y);
             }
         }
+    };
+    for (int k = k0; k < k0 + KS; k += 2 * kBatch) {
+        if (k + kBatch < k0 + KS) fetch(wv[1], k + kBatch);
+        use(wv[0], k);
+        if (k + kBatch >= k0 + KS) break;
+        if (k + 2 * kBatch < k0 + KS) fetch(wv[0], k + 2 * kBatch);
+        use(wv[1], k + kBatch);
     }
+    pdl_trigger();
 #pragma unroll
-    for (int tt = 0; tt < kTok; ++tt) r_s[(slice * kTok + tt) * 32 + mx] = acc[tt];
+    for (int tt = 0; tt < kTok; ++tt) *reinterpret_cast<float2*>(r_s + (slice * kTok + tt) * kOuts + 2 * lane) = acc[tt];
     __syncthreads();
     // the slices are added in their order by one thread per (token, output)
-    for (int i = threadIdx.x; i < nt * 32; i += blockDim.x) {
-        const int tt = i >> 5, x = i & 31, mm = blockIdx.z * 32 + x;
+    for (int i = threadIdx.x; i < nt * kOuts; i += blockDim.x) {
+        const int tt = i / kOuts, x = i % kOuts, mm = blockIdx.z * kOuts + x;
         if (mm >= M) continue;
         float v = 0.0f;
 #pragma unroll
-        for (int sl = 0; sl < kSlices; ++sl) v += r_s[(sl * kTok + tt) * 32 + x];
+        for (int sl = 0; sl < kSlices; ++sl) v += r_s[(sl * kTok + tt) * kOuts + x];
         if (gate) {
             const float gv = to_float(gate[(size_t)(n0 + tt) * g_tok + (size_t)h * M + mm]);
             v *= 1.0f / (1.0f + expf(-gv));
@@ -297,11 +358,17 @@ int launch_heads(const void* a, long a_tok, int a_head, const void* w, void* out
             (const T*)a, a_tok, a_head, (const T*)w, (TO*)out, o_tok, o_head, (const T*)gate, g_tok, N, M, K);
         return launch_status();
     }
-    const int ks = (((K + kSlices - 1) / kSlices) + kBatch - 1) / kBatch * kBatch;
-    dim3 grid((N + kTok - 1) / kTok, H, (M + 31) / 32);
-    launch_pdl(heads_linear_kernel<T, TO>, grid, 128, sizeof(float) * kTok * (ks * kSlices + kSlices * 32), stream, (const T*)a, a_tok, a_head, (const T*)w, (TO*)out,
-                                                                                 o_tok, o_head, (const T*)gate, g_tok, N, M, K);
-    return launch_status();
+    const int ks = heads_slice(K);
+    const size_t smem = sizeof(float) * kTok * (ks * kSlices + kSlices * kOuts);
+    static const cudaError_t allowed = [] {
+        const cudaError_t e = cudaFuncSetAttribute(heads_linear_kernel<T, TO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(heads_linear_kernel<T, TO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    }();
+    if (allowed != cudaSuccess) return (int)allowed;
+    dim3 grid((N + kTok - 1) / kTok, H, (M + kOuts - 1) / kOuts);
+    const auto kernel = M % 2 == 0 ? heads_linear_kernel<T, TO, true> : heads_linear_kernel<T, TO, false>;
+    return launch_pdl(kernel, grid, dim3(32 * kSlices), smem, stream, (const T*)a, a_tok, a_head, (const T*)w, (TO*)out, o_tok, o_head,
+                      (const T*)gate, g_tok, N, M, K);
 }
 
 }  // namespace

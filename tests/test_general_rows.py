@@ -98,3 +98,23 @@ def test_few_rows_on_the_tensor_cores(q_lens, kv_lens, hq, hkv, dk, dv, opts):
     # float32 rows: scores of up to 576 products and sums over the keys, each a few units in the last place off
     assert float((got[torch.float32].double() - want).norm() / want.norm()) < 1.5e-6
     assert float((got[torch.bfloat16].double() - want).abs().max() / want.abs().max()) < 2.0 ** -8
+
+
+# 16 tokens and fewer: one and two token tiles, outputs around a block's 64, odd counts, k around the slices and behind their end
+@pytest.mark.parametrize("n,heads,k,m", [(1, 2, 1, 1), (8, 3, 16, 64), (9, 2, 17, 65), (16, 5, 100, 66), (3, 2, 512, 128), (5, 2, 1024, 63)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_heads_linear_of_a_few_tokens(n, heads, k, m, dtype):
+    from pulsar_b200 import ops
+    gen = torch.Generator().manual_seed(n * k + m)
+    wide = torch.randn(n, heads * (k + 5), generator=gen).to(dtype).cuda()
+    a = wide.view(n, heads, k + 5)[:, :, :k]                 # strided rows, not all on 16-byte addresses
+    w, gate = (torch.randn(*s, generator=gen).to(dtype).cuda() for s in ((heads, k, m), (n, heads * m)))
+    want = torch.einsum("nhk,hkm->nhm", a.double(), w.double())
+    size = torch.einsum("nhk,hkm->nhm", a.double().abs(), w.double().abs())
+    out = torch.full((n, heads, m), float("nan"), device="cuda")
+    ops.heads_linear(a, w, out)
+    assert bool(((out.double() - want).abs() <= (k + 8) * 2.0 ** -24 * size).all())
+    gated = torch.empty(n, heads, m, dtype=dtype, device="cuda")
+    ops.heads_linear(a, w, gated, gate)
+    want = want * torch.sigmoid(gate.double()).view(n, heads, m)
+    assert bool(((gated.double() - want).abs() <= ((k + 16) * 2.0 ** -24 + (0 if dtype == torch.float32 else 2.0 ** -8)) * size).all())
