@@ -118,3 +118,20 @@ def test_heads_linear_of_a_few_tokens(n, heads, k, m, dtype):
     ops.heads_linear(a, w, gated, gate)
     want = want * torch.sigmoid(gate.double()).view(n, heads, m)
     assert bool(((gated.double() - want).abs() <= ((k + 16) * 2.0 ** -24 + (0 if dtype == torch.float32 else 2.0 ** -8)) * size).all())
+
+
+# rows enough for four vectors a thread, widths below, at and above one round of a block, and the last row alone
+@pytest.mark.parametrize("width", [36, 2048, 4100, 8192])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_add_rmsnorm_of_many_rows(width, dtype):
+    from pulsar_b200 import ops
+    n, gen = 593, torch.Generator().manual_seed(width)
+    residual, delta, weight = (torch.randn(*s, generator=gen).cuda() for s in ((n, width), (n, width), (width,)))
+    delta = delta.to(dtype)
+    out, stream = torch.empty(n, width, dtype=dtype, device="cuda"), residual.clone()
+    ops.add_rmsnorm(stream, delta, weight, 1e-6, out)
+    assert torch.equal(stream, residual + delta.float())
+    x = stream.double()
+    want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6) * weight.double()
+    tol = 2e-6 if dtype == torch.float32 else 2.0 ** -8         # a sum of up to 8,192 squares, a square root and two products; one rounding
+    assert bool(((out.double() - want).abs() <= tol * want.abs() + 1e-30).all())
