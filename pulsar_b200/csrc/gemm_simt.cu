@@ -174,31 +174,35 @@ int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, cu
 // Bound by the FMA pipes (59 % of their cycles with 24576 x 1024 weights and 384 rows; the issue slots 71 %).  A block of 128
 // threads owns 8 TM x 128 outputs, a warp 8 TM x 32, a thread TM x 8 of them (rows ty + 8 i, columns tx + 4 j).  Both operands
 // stand in shared memory as they do in memory, k fastest, so that asynchronous 16-byte copies bring them and a thread reads four
-// k of a row at once: 16 reads per 256 multiply-adds with TM 8.  Rows stand 20 floats apart (an odd number of 16-byte units: no
-// bank conflicts), and of the 8 x 4 lanes of a warp neighbours share a row or a column (see above).  Three stages of 16 k.  A block
+// k of a row at once: 16 reads per 256 multiply-adds with TM 8.  Rows stand an odd number of 16-byte units apart (no
+// bank conflicts), and of the 8 x 4 lanes of a warp neighbours share a row or a column (see above).  Two stages of 32 k with 32 rows
+// (half the barriers of three stages of 16: 24576 x 4096 with 387 rows 2.03 -> 1.90 ms, 4096 x 4096 389 -> 356 us), three of 16 with
+// 64 rows (more would not fit).  A block
 // whose last rows lie behind M computes 8 or 16 rows instead.  k slowest in shared memory (copies of 4 bytes) was slower (35 against 39
 // TFLOP/s at 24576 x 4096, 387 rows), packed pairs of multiply-adds are not faster than single ones on this chip (61 against 65).
-constexpr int GN = 128, GK = 16, GST = 3, GSTRIDE = GK + 4;
+constexpr int GN = 128;
+template <int GM> struct Tile { static constexpr int GK = GM == 64 ? 16 : 32, GST = GM == 64 ? 3 : 2, GSTRIDE = GK + 4; };
 
 template <int GM, int NI, typename TO>
 __device__ __forceinline__ void tile_block(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out,
                                            int M, int N, int K, float* smem) {
+    constexpr int GK = Tile<GM>::GK, GST = Tile<GM>::GST, GSTRIDE = Tile<GM>::GSTRIDE, LR = 128 / (GK / 4);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = lane >> 1 & 3, ty = (lane & 1) | lane >> 3 << 1;
     const int row0 = blockIdx.x * GM, col0 = blockIdx.y * GN;
     constexpr int kStage = (GM + GN) * GSTRIDE;
     const int n_kt = (K + GK - 1) / GK;
-    const int lq = tid % 4 * 4, lr = tid / 4;               // this thread's four k and its row within a copy of 32 rows
+    const int lq = tid % (GK / 4) * 4, lr = tid / (GK / 4);      // this thread's four k and its row within a copy of LR rows
     auto load = [&](int kt) {
         float* dst = smem + (kt % GST) * kStage + lq;
         const int k = kt * GK + lq;
 #pragma unroll
-        for (int r = lr; r < 8 * NI; r += 32) {
+        for (int r = lr; r < 8 * NI; r += LR) {
             const bool ok = k < K && row0 + r < M;
             cp_async16(smem_u32(dst + r * GSTRIDE), ok ? A + (size_t)(row0 + r) * K + k : A, ok);
         }
 #pragma unroll
-        for (int r = lr; r < GN; r += 32) {
+        for (int r = lr; r < GN; r += LR) {
             const bool ok = k < K && col0 + r < N;
             cp_async16(smem_u32(dst + (GM + r) * GSTRIDE), ok ? W + (size_t)(col0 + r) * K + k : W, ok);
         }
@@ -255,7 +259,7 @@ template <int TM, typename TO>
 __global__ void __launch_bounds__(128, TM == 8 ? 3 : 4)
 simt_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out, int M, int N, int K) {
     constexpr int GM = 8 * TM;
-    __shared__ __align__(16) float tile_smem[GST * (GM + GN) * GSTRIDE];
+    __shared__ __align__(16) float tile_smem[Tile<GM>::GST * (GM + GN) * Tile<GM>::GSTRIDE];
     const int left = M - (int)blockIdx.x * GM;
     if (TM == 8 && left > 32) tile_block<GM, TM, TO>(A, W, out, M, N, K, tile_smem);
     else if (left > 16) tile_block<GM, 4, TO>(A, W, out, M, N, K, tile_smem);
@@ -281,8 +285,8 @@ int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, cud
     if (M <= 8) return few ? launch_rows<2, 1, 4>(A, W, out, M, N, K, stream) : launch_rows<2, 2, 2>(A, W, out, M, N, K, stream);
     if (M <= 16) return few ? launch_rows<2, 1, 8>(A, W, out, M, N, K, stream) : launch_rows<4, 2, 2>(A, W, out, M, N, K, stream);
     // 64 rows a block where there are blocks for 16 rounds of the SMs (151936 x 4096, 387 rows: 11.3 against 11.9 ms), else 32, whose last
-    // rounds are less empty (4096 x 4096: 33 rows 161 against 269 us, 387 rows 389 against 500, the general kernel 656;
-    // 24576 x 4096, 387 rows: 2.03 against 2.00 ms, 2.96 before)
+    // rounds are less empty (4096 x 4096: 33 rows 161 against 269 us, 387 rows 356 against 500, the general kernel 656;
+    // 24576 x 4096, 387 rows: 1.90 against 2.00 ms, 2.96 before)
     if ((long)((M + 63) / 64) * ((N + GN - 1) / GN) >= 16 * 148) return launch_tile<8>(A, W, out, M, N, K, stream);
     return launch_tile<4>(A, W, out, M, N, K, stream);
 }
