@@ -763,6 +763,17 @@ def decode_splits(n_seqs: int, n_kv_heads: int, table_tokens: int = 4096) -> int
     return best
 
 
+def decode_shares(n_seqs: int, n_kv_heads: int, table_tokens: int) -> int:
+    """``decode_splits``, or more of them for a sequence or two: one per 64 tokens (a tile of the kernel) while the
+    blocks are no more than 128.  So few blocks are bound by a block's own walk over its keys, not by the bytes of
+    all: one sequence of 1,000 keys, 12 layers of the 8B sizes, 4 splits 1,078 us a step, 8 1,054, 16 1,047; at 4,000
+    keys 16 are ahead of 32 (1,083, 1,104), with four sequences of 1,000 4 ahead of 9 (1,122, 1,125)."""
+    splits = decode_splits(n_seqs, n_kv_heads, table_tokens)
+    if _FORCED_SPLITS > 0:
+        return splits
+    return max(splits, min(table_tokens // 64, 128 // max(1, n_seqs * n_kv_heads)))
+
+
 _TICKETS = 1 << 16
 _decode_tickets = {}
 
@@ -939,7 +950,7 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
     applies (bfloat16, head size 128, pages of 8 or more), else the mma.sync kernel (bfloat16, head
     size 64 or 128), else the generic kernel.  ``PULSAR_ATTENTION=mma`` leaves the tcgen05 kernel out."""
     if ctx.all_decode:
-        n_splits = decode_splits(ctx.n_seqs, cache.k_pool.shape[1], cache.block_table.shape[1] * cache.k_pool.shape[2])
+        n_splits = decode_shares(ctx.n_seqs, cache.k_pool.shape[1], cache.block_table.shape[1] * cache.k_pool.shape[2])
         partial = ctx.scratch("attn.partial", (ctx.n_seqs * q.shape[1] * n_splits * (q.shape[2] + 2),), torch.float32)
         paged_attention_decode(q, cache.k_pool, cache.v_pool, out, partial, cache.block_table, ctx.kv_len, scale,
                                window, n_splits)
@@ -956,7 +967,7 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
             n_dec += 1
         table, cu_q, kv_len = cache.block_table, ctx.cu_q, ctx.kv_len
         if n_dec > 0:
-            n_splits = decode_splits(n_dec, hkv, table.shape[1] * page_size)
+            n_splits = decode_shares(n_dec, hkv, table.shape[1] * page_size)
             partial = ctx.scratch("attn.partial", (n_dec * q.shape[1] * n_splits * (q.shape[2] + 2),), torch.float32)
             paged_attention_decode(q[:n_dec], cache.k_pool, cache.v_pool, out[:n_dec], partial, table[:n_dec], kv_len[:n_dec],
                                    scale, window, n_splits)

@@ -74,3 +74,29 @@ def test_attention_of_rows_that_share_keys(q_lens, kv_lens, hq, hkv, d, page, wi
         tol = 2e-5 if dtype == torch.float32 else 2.0 ** -8
         assert float((out[at:at + n].double() - want).abs().max() / want.abs().max()) < tol
         at += n
+
+
+@pytest.mark.parametrize("kv_lens,hkv,dtype", [([1000], 8, torch.bfloat16), ([130], 2, torch.float32), ([1, 700], 4, torch.bfloat16)])
+def test_decode_attention_of_a_sequence_or_two(kv_lens, hkv, dtype):
+    """As many shares as ``decode_shares`` gives: one per tile of keys, some without a key."""
+    from pulsar_b200 import ops
+    hq, d, page, s = 4 * hkv, 128, 16, len(kv_lens)
+    width = 64 * -(-max(kv_lens) // (64 * page))
+    shares = ops.decode_shares(s, hkv, width * page)
+    assert shares == min(16 if width == 64 else 32, 128 // (s * hkv)) and shares <= 64
+    g = torch.Generator(device="cuda").manual_seed(hkv)
+    table = torch.full((s, width), -1, dtype=torch.int32)
+    for i, n in enumerate(kv_lens):
+        table[i, :-(-n // page)] = torch.arange(-(-n // page)) + i * width
+    pools = [torch.randn(s * width, hkv, page, d, generator=g, device="cuda").to(dtype) for _ in range(2)]
+    q = torch.randn(s, hq, d, generator=g, device="cuda").to(dtype)
+    out, partial = torch.empty_like(q), torch.full((s * hq * shares * (d + 2),), float("nan"), device="cuda")
+    ops.paged_attention_decode(q, pools[0], pools[1], out, partial, table.cuda(), torch.tensor(kv_lens, dtype=torch.int32, device="cuda"),
+                               d ** -0.5, None, shares)
+    for i, n in enumerate(kv_lens):
+        key = torch.arange(n)
+        k, v = (p[table[i, key // page].long().cuda(), :, (key % page).cuda()].double().repeat_interleave(4, dim=1) for p in pools)
+        w = torch.softmax(torch.einsum("hd,jhd->hj", q[i].double(), k) * d ** -0.5, dim=-1)
+        want = torch.einsum("hj,jhd->hd", w, v)
+        tol = 2e-5 if dtype == torch.float32 else 2.0 ** -6      # bfloat16: the weights and the output rounded once each
+        assert float((out[i].double() - want).abs().max() / want.abs().max()) < tol
