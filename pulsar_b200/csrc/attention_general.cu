@@ -943,6 +943,7 @@ __global__ void qkv_split_write_kernel(const T* __restrict__ qkv, float* __restr
                                        T* __restrict__ v_pool, const int* __restrict__ slots, int Hq, int Hk, int Hv, int Dk, int Dv,
                                        int page_size, const int* __restrict__ positions, float temp_coef, int temp_every,
                                        const PoolBounds bounds) {
+    pdl_trigger();      // a short kernel: the next one may fetch its weights now
     pdl_wait();         // may have come onto the SMs while the product before it was ending: nothing is touched before that one is done
     const int t = blockIdx.x, lane = threadIdx.x & 31;
     const int head = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);

@@ -250,6 +250,7 @@ latent_norms_kernel(const T* __restrict__ q_lat, const float* __restrict__ q_nor
                     const float* __restrict__ norm_w, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                     const int* __restrict__ slots, T* __restrict__ pool, T* __restrict__ latent_out, T* __restrict__ rot_out,
                     const NormsShape sh, const PoolBounds bounds) {
+    pdl_trigger();      // a short kernel: the next one may fetch its weights now
     pdl_wait();         // may have come onto the SMs while the product before it was ending: nothing is touched before that one is done
     __shared__ float scratch[32];
     const int t = blockIdx.x;
@@ -298,6 +299,7 @@ latent_prepare_kernel(const T* __restrict__ q, const T* __restrict__ down, const
                       const float* __restrict__ cos_t, const float* __restrict__ sin_t, const int* __restrict__ slots,
                       T* __restrict__ pool, float* __restrict__ q_out, T* __restrict__ latent_out, T* __restrict__ rot_out,
                       const PrepareShape sh, const PoolBounds bounds) {
+    pdl_trigger();      // a short kernel: the next one may fetch its weights now
     pdl_wait();
     __shared__ float scratch[32];
     const int t = blockIdx.x;

@@ -54,6 +54,7 @@ causal_conv_silu_kernel(const TIn* __restrict__ in, long in_tok, const float* __
                         const float* __restrict__ arena, long slot_stride, long tail_offset, const int* __restrict__ cu_q,
                         const int* __restrict__ seq_of_token, const int* __restrict__ state_slots, T* __restrict__ out,
                         int channels, int n_taps, int n_tokens, int run) {
+    pdl_trigger();      // a short kernel: the next one may fetch its weights now
     pdl_wait();         // may have come onto the SMs while the product before it was ending: nothing is touched before that one is done
     const int t0 = blockIdx.x * run, t1 = min(t0 + run, n_tokens);
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
@@ -101,6 +102,7 @@ selective_scan_kernel(const T* __restrict__ x, const T* __restrict__ xz, const T
                       const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
                       float* __restrict__ arena, T* __restrict__ y, const int* __restrict__ cu_q,
                       const int* __restrict__ state_slots, const ScanShape sh) {
+    pdl_trigger();      // a short kernel: the next one may fetch its weights now
     pdl_wait();         // may have come onto the SMs while the product before it was ending: nothing is touched before that one is done
     constexpr int CH = 128 / G;
     extern __shared__ float smem[];
