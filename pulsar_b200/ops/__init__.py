@@ -771,7 +771,7 @@ def decode_shares(n_seqs: int, n_kv_heads: int, table_tokens: int) -> int:
     splits = decode_splits(n_seqs, n_kv_heads, table_tokens)
     if _FORCED_SPLITS > 0:
         return splits
-    return max(splits, min(table_tokens // 64, 128 // max(1, n_seqs * n_kv_heads)))
+    return max(splits, min(32, table_tokens // 64, 128 // max(1, n_seqs * n_kv_heads)))
 
 
 _TICKETS = 1 << 16
