@@ -36,3 +36,40 @@ def test_chunked_scan_of_aligned_rows(lens, inner, state, dtype):
         got.append((y.clone(), arena))
     assert bool(torch.isfinite(got[0][0].float()).all())
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("n,heads,dim,rot", [(1, 1, 8, 8), (3, 5, 24, 16), (65, 16, 128, 64), (7, 3, 20, 4)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rows_of_the_expanded_form(n, heads, dim, rot, dtype):
+    from pulsar_b200 import ops
+    gen = torch.Generator().manual_seed(n + dim)
+    plain, shared = torch.randn(n, heads, dim, generator=gen).to(dtype), torch.randn(n, rot, generator=gen).to(dtype)
+    want = torch.cat([plain, shared[:, None].expand(n, heads, rot)], dim=-1)
+    q, turn = torch.randn(n, heads * (dim + rot) + 8, generator=gen).to(dtype), torch.rand(n, rot // 2, generator=gen).cuda()
+    for off in (0, 1):
+        keys = _at(torch.zeros(n, heads, dim + rot, dtype=dtype), off)
+        ops.latent_expand_keys(_at(plain, off), _at(shared, off), keys)
+        assert torch.equal(keys.cpu(), want)
+        rows = _at(torch.full((n, heads, dim + rot), float("nan")), off)
+        ops.latent_prepare(_at(q, off)[:, :heads * (dim + rot)], None, None, 1e-6, turn.cos(), turn.sin(), None, None, rows, heads, dim, rot,
+                           8, 16, plain_too=True)
+        assert torch.equal(rows.cpu()[..., :dim], q[:, :heads * (dim + rot)].view(n, heads, dim + rot)[..., :dim].float())
+        assert bool(torch.isfinite(rows).all())
+
+
+@pytest.mark.parametrize("n,width,behind", [(1, 8, 0), (3, 4104, 8), (700, 2048, 2048), (5, 12, 4), (5, 16, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sigmoid_gate_of_aligned_rows(n, width, behind, dtype):
+    from pulsar_b200 import ops
+    gen = torch.Generator().manual_seed(n + width)
+    x, wide = torch.randn(n, width, generator=gen).to(dtype), (8 * torch.randn(n, width + behind, generator=gen)).to(dtype)
+    wide[0, :4] = torch.tensor([float("inf"), -float("inf"), 200.0, -200.0])
+    got = []
+    for off in (0, 1):
+        y = _at(x, off)
+        ops.sigmoid_gate(y, _at(wide, off)[:, :width])
+        got.append(y.clone())
+    assert torch.equal(got[0], got[1])
+    want = x.double() * torch.sigmoid(wide[:, :width].double())
+    tol = 4e-6 if dtype == torch.float32 else 2.0 ** -8         # an exponential, a sum and a quotient in float32; one rounding
+    assert bool(((got[0].cpu().double() - want).abs() <= tol * want.abs() + 1e-38).all())
