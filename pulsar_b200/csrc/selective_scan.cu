@@ -332,6 +332,63 @@ int launch_scan_prompt(const void* x, const void* xz, const void* bc, long bc_to
 // (one more word than 256 per row), so that lanes read neighbouring words and the staging writes hit different banks.
 constexpr int kSpan = 256, kRun = 8, kSpanRow = kSpan + 1, kChunkChannels = 8;
 
+// M states of one channel over a span's runs, side by side: each is a chain of dependent steps (the run, five shuffles, the run again),
+// and a warp that walks M of them has something to issue while one waits.
+// Two cost registers (100 instead of 80, 16 warps an SM instead of 24) and are ahead all the same: 2,048 tokens x 4,096 channels x 16
+// states 243 -> 203 us with a cold L2, 700 tokens 96 -> 84, 64 as before; four are no better (203), two in 80 registers are behind (234).
+// The scalar form (kVec false), whose staging waits for each load, needs the warps: it keeps one (two: 160 -> 221 us with 7 states).
+template <int M>
+__device__ __forceinline__ void walk_states(int n, int S, int w, int lane, const float* bc_s, const float* a_s, float* carry_s,
+                                            const float (&dt)[kRun], const float (&dx)[kRun], float (&acc)[kRun]) {
+    float a[M][kRun], b[M][kRun], P[M], Q[M], carry[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        const float rate = a_s[w * S + n + m];
+        const float* bn = bc_s + (n + m) * kSpanRow + lane;
+        carry[m] = carry_s[w * S + n + m];
+        P[m] = 1.0f;
+        Q[m] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kRun; ++k) {
+            a[m][k] = expf(dt[k] * rate);
+            b[m][k] = dx[k] * bn[k * 32];
+            Q[m] = fmaf(a[m][k], Q[m], b[m][k]);
+            P[m] *= a[m][k];
+        }
+    }
+    // inclusive prefix over the lanes: (P, Q) of all runs up to and including this lane's
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const float Pp = __shfl_up_sync(0xffffffffu, P[m], o), Qp = __shfl_up_sync(0xffffffffu, Q[m], o);
+            if (lane >= o) { Q[m] = fmaf(P[m], Qp, Q[m]); P[m] *= Pp; }
+        }
+    }
+    float st[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        float Pe = __shfl_up_sync(0xffffffffu, P[m], 1), Qe = __shfl_up_sync(0xffffffffu, Q[m], 1);
+        if (lane == 0) { Pe = 1.0f; Qe = 0.0f; }
+        st[m] = fmaf(Pe, carry[m], Qe);                      // the state that enters this lane's run
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {                            // in the states' order: the sums keep theirs
+        const float* cn = bc_s + (S + n + m) * kSpanRow + lane;
+#pragma unroll
+        for (int k = 0; k < kRun; ++k) {
+            st[m] = fmaf(a[m][k], st[m], b[m][k]);
+            acc[k] = fmaf(st[m], cn[k * 32], acc[k]);
+        }
+    }
+    __syncwarp();                                            // every lane has read the carries
+    if (lane == 31) {                                        // whose prefix is the whole span's
+#pragma unroll
+        for (int m = 0; m < M; ++m) carry_s[w * S + n + m] = fmaf(P[m], carry[m], Q[m]);
+    }
+    __syncwarp();
+}
+
 // kVec: rows are read and written 16 bytes at a time (see the launcher).
 template <typename T, bool kVec>
 __global__ void __launch_bounds__(256)
@@ -426,38 +483,11 @@ selective_scan_chunked_kernel(const T* __restrict__ x, const T* __restrict__ xz,
             dx[k] = dt[k] * x_s[w * kSpanRow + k * 32 + lane];
             acc[k] = 0.0f;
         }
-        for (int n = 0; n < S; ++n) {
-            const float rate = a_s[w * S + n];
-            const float* bn = bc_s + n * kSpanRow + lane;
-            const float* cn = bc_s + (S + n) * kSpanRow + lane;
-            float a[kRun], b[kRun];
-            float P = 1.0f, Q = 0.0f;
-#pragma unroll
-            for (int k = 0; k < kRun; ++k) {
-                a[k] = expf(dt[k] * rate);
-                b[k] = dx[k] * bn[k * 32];
-                Q = fmaf(a[k], Q, b[k]);
-                P *= a[k];
-            }
-            // inclusive prefix over the lanes: (P, Q) of all runs up to and including this lane's
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const float Pp = __shfl_up_sync(0xffffffffu, P, o), Qp = __shfl_up_sync(0xffffffffu, Q, o);
-                if (lane >= o) { Q = fmaf(P, Qp, Q); P *= Pp; }
-            }
-            const float carry = carry_s[w * S + n];
-            float Pe = __shfl_up_sync(0xffffffffu, P, 1), Qe = __shfl_up_sync(0xffffffffu, Q, 1);
-            if (lane == 0) { Pe = 1.0f; Qe = 0.0f; }
-            float st = fmaf(Pe, carry, Qe);                  // the state that enters this lane's run
-#pragma unroll
-            for (int k = 0; k < kRun; ++k) {
-                st = fmaf(a[k], st, b[k]);
-                acc[k] = fmaf(st, cn[k * 32], acc[k]);
-            }
-            const float P_all = __shfl_sync(0xffffffffu, P, 31), Q_all = __shfl_sync(0xffffffffu, Q, 31);
-            __syncwarp();                                    // every lane has read the carry
-            if (lane == 0) carry_s[w * S + n] = fmaf(P_all, carry, Q_all);
-        }
+        constexpr int kSideBySide = kVec ? 2 : 1;
+        int n = 0;
+        for (; n + kSideBySide <= S; n += kSideBySide)
+            walk_states<kSideBySide>(n, S, w, lane, bc_s, a_s, carry_s, dt, dx, acc);
+        for (; n < S; ++n) walk_states<1>(n, S, w, lane, bc_s, a_s, carry_s, dt, dx, acc);
 #pragma unroll
         for (int k = 0; k < kRun; ++k) {
             const int at = k * 32 + lane;
