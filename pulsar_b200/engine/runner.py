@@ -287,7 +287,7 @@ class ModelRunner:
             self._graphs.clear()
             self._graph_seen.clear()
             self._graph_epoch = self.scratch_epoch
-        key = (ctx.n_tokens, ctx.n_seqs, int(ctx.logit_rows.numel()), ctx.table_widths,
+        key = (ctx.n_tokens, ctx.n_seqs, int(ctx.logit_rows.numel()), ctx.table_widths, ctx.uneven,
                tuple(int(t.data_ptr()) for t in (ctx.token_ids, ctx.logit_rows)))
         hit = self._graphs.get(key)
         if hit is not None:

@@ -763,15 +763,36 @@ def decode_splits(n_seqs: int, n_kv_heads: int, table_tokens: int = 4096) -> int
     return best
 
 
-def decode_shares(n_seqs: int, n_kv_heads: int, table_tokens: int) -> int:
-    """``decode_splits``, or more of them for a sequence or two: one per 64 tokens (a tile of the kernel) while the
-    blocks are no more than 128.  So few blocks are bound by a block's own walk over its keys, not by the bytes of
-    all: one sequence of 1,000 keys, 12 layers of the 8B sizes, 4 splits 1,078 us a step, 8 1,054, 16 1,047; at 4,000
-    keys 16 are ahead of 32 (1,083, 1,104), with four sequences of 1,000 4 ahead of 9 (1,122, 1,125)."""
+def decode_shares(n_seqs: int, n_kv_heads: int, table_tokens: int, uneven: bool = False) -> int:
+    """``decode_splits``, but for three kinds of steps (times of whole steps of the 8B sizes, 36 layers unless said):
+
+    A sequence or two: one per 64 tokens (a tile of the kernel) while the blocks are no more than 128.  So few blocks
+    are bound by a block's own walk over its keys, not by the bytes of all: one sequence of 1,000 keys, 12 layers, 4
+    splits 1,078 us a step, 8 1,054, 16 1,047; at 4,000 keys 16 are ahead of 32 (1,083, 1,104), with four sequences of
+    1,000 4 ahead of 9 (1,122, 1,125).
+
+    More (sequence, kv head) pairs than slots, over a table of up to 2,048 tokens: one.  Walks that short are over before a
+    thin last round costs what the starts and the merge of the splits do: 40 sequences of 210 to 1,400 keys 5,618 us with 7
+    splits, 4,735 with one, all of 1,400 6,087 and 5,685; 48 of 90 to 600 4,704 with 2, 4,473 with one.
+
+    ``uneven`` (``StepContext.uneven``: the keys of all are well under the longest's times their number) over a longer table:
+    the short ones' blocks end early and leave their slots to others.  Pairs that fit the slots take splits for 384 blocks, a share
+    no shorter than 1,024 tokens of the table, where filling the slots once, as equal ones are best, leaves SMs idle: 16 sequences of
+    560 to 3,700 keys 4,354 us with 2 splits, 4,181 with 3 (all of 3,700: 4,519, 5,050); 24 of 360 to 2,400 4,845 with one,
+    4,749 with 2 (all of 2,400: 5,130, 5,508).  More pairs than slots take no more than two, there is no thin last round to
+    fill: 40 of 390 to 2,600 6,012 us with 7, 5,656 with 2 (all of 2,600: 6,910, 6,844); 44 of 590 to 3,900, the
+    longest first or in any order, 6,596 and 6,384 with 4, 6,394 and 6,472 with 2."""
     splits = decode_splits(n_seqs, n_kv_heads, table_tokens)
     if _FORCED_SPLITS > 0:
         return splits
-    return max(splits, min(32, table_tokens // 64, 128 // max(1, n_seqs * n_kv_heads)))
+    pairs = max(1, n_seqs * n_kv_heads)
+    if pairs > _DECODE_SLOTS and table_tokens <= 2048:
+        return 1
+    if uneven and pairs > _DECODE_SLOTS:
+        splits = min(splits, 2)
+    elif uneven and table_tokens >= 3072:
+        splits = max(splits, min(32, 384 // pairs, table_tokens // 1024))
+    return max(splits, min(32, table_tokens // 64, 128 // pairs))
 
 
 _TICKETS = 1 << 16
@@ -950,7 +971,7 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
     applies (bfloat16, head size 128, pages of 8 or more), else the mma.sync kernel (bfloat16, head
     size 64 or 128), else the generic kernel.  ``PULSAR_ATTENTION=mma`` leaves the tcgen05 kernel out."""
     if ctx.all_decode:
-        n_splits = decode_shares(ctx.n_seqs, cache.k_pool.shape[1], cache.block_table.shape[1] * cache.k_pool.shape[2])
+        n_splits = decode_shares(ctx.n_seqs, cache.k_pool.shape[1], cache.block_table.shape[1] * cache.k_pool.shape[2], ctx.uneven)
         partial = ctx.scratch("attn.partial", (ctx.n_seqs * q.shape[1] * n_splits * (q.shape[2] + 2),), torch.float32)
         paged_attention_decode(q, cache.k_pool, cache.v_pool, out, partial, cache.block_table, ctx.kv_len, scale,
                                window, n_splits)

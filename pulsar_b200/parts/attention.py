@@ -319,7 +319,7 @@ class Attention(Mixer):
                 and ops.decode_qkv_supported(qkv.dtype, s.n_heads, n_kv, s.head_dim, rotary, cache.page_size)):
             # a step of single tokens: the attention kernel normalises, rotates and writes the cache itself
             o = ctx.scratch("attn.o", (n, s.n_heads, s.head_dim))
-            n_splits = ops.decode_shares(ctx.n_seqs, n_kv, cache.block_table.shape[1] * cache.page_size)
+            n_splits = ops.decode_shares(ctx.n_seqs, n_kv, cache.block_table.shape[1] * cache.page_size, ctx.uneven)
             partial = ctx.scratch("attn.partial", (ctx.n_seqs * s.n_heads * n_splits * (s.head_dim + 2),), torch.float32)
             ops.paged_attention_decode_qkv(qkv, self.q_norm, self.k_norm, cos, sin, s.qk_norm_eps or 0.0, cache.slots, cache.k_pool,
                                            cache.v_pool, o, partial, cache.block_table, ctx.kv_len, s.scale, s.window, n_splits)

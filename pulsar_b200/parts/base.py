@@ -77,6 +77,9 @@ class StepContext:
         self.max_q_len = max(host.q_lens) if host.q_lens else 0
         self.max_kv_len = max(host.kv_lens) if host.kv_lens else 0
         self.all_decode = self.max_q_len == 1
+        # whether the sequences hold together less than 0.7 of what they would if all were as long as the longest (part of a
+        # captured step's key: what is decided by it holds for every replay)
+        self.uneven = 10 * sum(host.kv_lens) < 7 * self.max_kv_len * len(host.kv_lens)
         # int32 device arrays
         self.token_ids = self.positions = self.seq_of_token = None      # [N]
         self.position_axes = None               # [axes, N] where the model's positions have more than one axis, else None

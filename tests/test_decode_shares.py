@@ -1,0 +1,27 @@
+"""How many shares a decode step's keys are cut into, and when a step counts as uneven."""
+import types
+
+import pytest
+import torch
+
+
+@pytest.mark.parametrize("n,heads,table,uneven,want", [
+    (1, 8, 1024, False, 16), (1, 1, 100000, False, 32), (4, 8, 1024, True, 4),             # one or two; a short table stays as it was
+    (8, 8, 4096, False, 4), (8, 8, 4096, True, 4), (8, 8, 8192, True, 6), (12, 8, 4096, False, 3), (12, 8, 4096, True, 4),
+    (16, 8, 4096, True, 3), (16, 8, 3072, True, 3), (16, 8, 2048, True, 2), (24, 8, 3072, True, 2), (24, 8, 2048, True, 1),
+    (30, 8, 4096, True, 1), (37, 8, 4096, True, 1), (38, 8, 2048, False, 1), (48, 8, 2048, True, 1), (48, 8, 1024, False, 1),
+    (40, 8, 3072, False, 7), (40, 8, 3072, True, 2), (48, 8, 4096, False, 2), (64, 8, 4096, False, 1), (64, 8, 4096, True, 1)])
+def test_shares_of_a_step(n, heads, table, uneven, want):
+    from pulsar_b200 import ops
+    assert ops.decode_shares(n, heads, table, uneven) == want
+    for batch in range(1, 200, 7):
+        for tokens in (16, 300, 2048, 100000):
+            assert 1 <= ops.decode_shares(batch, heads, tokens, uneven) <= 32
+
+
+@pytest.mark.parametrize("lens,want", [([5], False), ([100, 100], False), ([100, 40], False), ([100, 39], True), ([1, 1, 1000], True)])
+def test_uneven_steps(lens, want):
+    from pulsar_b200.parts.base import HostBatch, StepContext
+    ctx = StepContext(types.SimpleNamespace(dtype=torch.float32, device="cpu"), len(lens), len(lens),
+                      HostBatch([1] * len(lens), lens, [-1] * len(lens)))
+    assert ctx.uneven is want
