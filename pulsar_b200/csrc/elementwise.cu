@@ -123,23 +123,18 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ residual, const T* __
     const int src = rows ? rows[r] : r;
     float* res = residual + (size_t)src * width;
     const T* del = delta ? delta + (size_t)src * width : nullptr;
-    float x[VPT][4], d[VPT][4];
+    float x[VPT][4];
     float local = 0.0f;
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {         // everything the row holds is asked for before anything is written
-        const int i = (threadIdx.x + v * blockDim.x) * 4;
-        if (i < width) {
-            load4(res + i, x[v]);
-            if (del) load4(del + i, d[v]);
-        }
-    }
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
         const int i = (threadIdx.x + v * blockDim.x) * 4;
         if (i < width) {
+            load4(res + i, x[v]);
             if (del) {
+                float d[4];
+                load4(del + i, d);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) x[v][e] += d[v][e];
+                for (int e = 0; e < 4; ++e) x[v][e] += d[e];
             }
             if (write_back) store4(res + i, x[v]);
 #pragma unroll
@@ -520,21 +515,14 @@ PB_EXPORT int pb_add_rmsnorm(int dtype, float* residual, const void* delta, cons
     const bool aligned = (((uintptr_t)residual | (uintptr_t)delta | (uintptr_t)weight | (uintptr_t)out) & 15) == 0;
     if (width % 4 == 0 && width <= 8192 && aligned) {
         const int vecs = width / 4;
-        // A few rows: as many threads as a row has vectors, the shortest way through one row.  Rows for four blocks an SM or more: four
-        // vectors a thread and more blocks an SM, so that some load while others wait for their sum (a prompt of 2,048 tokens, 73 such
-        // launches of 2,048 x 4,096: 25.61 -> 25.42 ms).
-        const int vpt = n_out >= 4 * 148 ? 4 : vecs <= 1024 ? 1 : 2;
-        const int threads = ((vecs + vpt - 1) / vpt + 31) / 32 * 32;
-#define PB_NORM(T, V) return launch_pdl(add_rmsnorm_vec_kernel<T, V>, n_out, threads, 0, stream, residual, (const T*)delta, weight, (T*)out, rows, width, eps, write_back)
+        const int vpt = vecs <= 1024 ? 1 : 2;
+        int threads = ((vecs + vpt - 1) / vpt + 31) / 32 * 32;
         if (dtype == PB_F32) {
-            if (vpt == 1) PB_NORM(float, 1);
-            if (vpt == 2) PB_NORM(float, 2);
-            PB_NORM(float, 4);
+            if (vpt == 1) return launch_pdl(add_rmsnorm_vec_kernel<float, 1>, n_out, threads, 0, stream, residual, (const float*)delta, weight, (float*)out, rows, width, eps, write_back);
+            return launch_pdl(add_rmsnorm_vec_kernel<float, 2>, n_out, threads, 0, stream, residual, (const float*)delta, weight, (float*)out, rows, width, eps, write_back);
         }
-        if (vpt == 1) PB_NORM(__nv_bfloat16, 1);
-        if (vpt == 2) PB_NORM(__nv_bfloat16, 2);
-        PB_NORM(__nv_bfloat16, 4);
-#undef PB_NORM
+        if (vpt == 1) return launch_pdl(add_rmsnorm_vec_kernel<__nv_bfloat16, 1>, n_out, threads, 0, stream, residual, (const __nv_bfloat16*)delta, weight, (__nv_bfloat16*)out, rows, width, eps, write_back);
+        return launch_pdl(add_rmsnorm_vec_kernel<__nv_bfloat16, 2>, n_out, threads, 0, stream, residual, (const __nv_bfloat16*)delta, weight, (__nv_bfloat16*)out, rows, width, eps, write_back);
     }
     const int b = block_for(width);
     if (dtype == PB_F32)

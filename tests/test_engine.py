@@ -592,3 +592,22 @@ def test_layer_sizes_of_the_family(tmp_path_factory, shape, dtype):
     worst = max(helpers.rel_err(row, ref[rid][pos]) for (rid, pos), row in got.items())
     helpers.report(f"layer_sizes[{shape}]", worst, dtype)
     assert worst < helpers.TOL_LARGE[dtype], f"worst relative error {worst:.3e}"
+
+
+@pytest.mark.parametrize("name", ["A", "B"])
+def test_float32_logits_do_not_depend_on_how_a_long_prompt_was_cut(folders, name):
+    """A prompt in one step (more rows than any kernel treats as few) and in portions: the same bits."""
+    from pulsar_b200.engine.runner import StepEntry
+    raw, seed, page = TINY[name]
+    prompt = helpers.random_tokens(random.Random(41), 700, raw["vocab_size"])
+    got = []
+    for cuts in ((700,), (300, 400), (592, 108), (593, 107), (640, 2, 58)):
+        eng = _engine(folders[name], "float32", page, num_pages=128, max_chunk_size=700)
+        at, rows = 0, []
+        for n in cuts:
+            want = [w - at for w in (299, 591, 639, 699) if at <= w < at + n]
+            rows.append(eng.runner.step([StepEntry("p", prompt[at:at + n], want)]).clone())
+            at += n
+        got.append(torch.cat(rows))
+    for other in got[1:]:
+        assert torch.equal(got[0], other)

@@ -120,7 +120,7 @@ def test_heads_linear_of_a_few_tokens(n, heads, k, m, dtype):
     assert bool(((gated.double() - want).abs() <= ((k + 16) * 2.0 ** -24 + (0 if dtype == torch.float32 else 2.0 ** -8)) * size).all())
 
 
-# rows enough for four vectors a thread, widths below, at and above one round of a block, and the last row alone
+# many rows, widths below, at and above one round of a block
 @pytest.mark.parametrize("width", [36, 2048, 4100, 8192])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_add_rmsnorm_of_many_rows(width, dtype):
@@ -135,3 +135,20 @@ def test_add_rmsnorm_of_many_rows(width, dtype):
     want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6) * weight.double()
     tol = 2e-6 if dtype == torch.float32 else 2.0 ** -8         # a sum of up to 8,192 squares, a square root and two products; one rounding
     assert bool(((out.double() - want).abs() <= tol * want.abs() + 1e-30).all())
+
+
+# The order of a row's sum of squares comes from the width alone: a row has the same bits in a step of a few rows as in one of many,
+# so that a float32 prompt's logits do not depend on how it was cut into steps.
+@pytest.mark.parametrize("width", [36, 2048, 4096, 4100, 8192, 8196])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_add_rmsnorm_does_not_depend_on_the_number_of_rows(width, dtype):
+    from pulsar_b200 import ops
+    n, gen = 1300, torch.Generator().manual_seed(width)
+    residual, delta, weight = (torch.randn(*s, generator=gen).cuda() for s in ((n, width), (n, width), (width,)))
+    delta = delta.to(dtype)
+    whole, stream = torch.empty(n, width, dtype=dtype, device="cuda"), residual.clone()
+    ops.add_rmsnorm(stream, delta, weight, 1e-6, whole)
+    for first, rows in ((0, 1), (3, 2), (7, 591), (500, 592), (700, 593)):
+        cut, part = residual[first:first + rows].clone(), torch.empty(rows, width, dtype=dtype, device="cuda")
+        ops.add_rmsnorm(cut, delta[first:first + rows].clone(), weight, 1e-6, part)
+        assert torch.equal(part, whole[first:first + rows]) and torch.equal(cut, stream[first:first + rows])
