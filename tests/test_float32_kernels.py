@@ -101,3 +101,33 @@ def test_decode_attention_of_a_sequence_or_two(kv_lens, hkv, dtype):
         want = torch.einsum("hj,jhd->hd", w, v)
         tol = 2e-5 if dtype == torch.float32 else 2.0 ** -6      # bfloat16: the weights and the output rounded once each
         assert float((out[i].double() - want).abs().max() / want.abs().max()) < tol
+
+
+# single tokens and portions of several sequences, whose rows never share a block: one row a block (few rows), four, and sixteen or eight
+# with tokens that begin anywhere; groups of one, of a part of a block's rows, and of more
+@pytest.mark.parametrize("q_lens,cached", [([3], 40), ([1, 2, 1], 7), ([1] * 9 + [30, 1, 5], 300), ([1] * 33 + [37, 2, 5, 1, 260], 90)])
+@pytest.mark.parametrize("hq,hkv,d,window", [(32, 8, 128, None), (16, 16, 64, 50), (20, 1, 48, None), (6, 2, 32, 33), (18, 6, 256, None)])
+def test_attention_of_a_sequence_does_not_depend_on_the_others(q_lens, cached, hq, hkv, d, window):
+    from pulsar_b200 import ops
+    page, n = 16, sum(q_lens)
+    kv_lens = [q + (cached * (i % 5 + 1)) // 5 for i, q in enumerate(q_lens)]
+    g = torch.Generator(device="cuda").manual_seed(n + d)
+    width = -(-max(kv_lens) // page)
+    table = torch.randperm(len(q_lens) * width, generator=torch.Generator().manual_seed(n)).to(torch.int32).view(len(q_lens), width).cuda()
+    pools = [torch.randn(len(q_lens) * width, hkv, page, d, generator=g, device="cuda") for _ in range(2)]
+    q = torch.randn(n, hq, d, generator=g, device="cuda")
+    as_i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")                       # noqa: E731
+
+    def run(rows, seqs):
+        lens = [q_lens[s] for s in seqs]
+        out = torch.full_like(rows, float("nan"))
+        seq = torch.repeat_interleave(torch.arange(len(seqs), device="cuda"), as_i32(lens)).to(torch.int32)
+        ops.paged_attention_generic(rows, pools[0], pools[1], out, table[seqs].contiguous(), as_i32([sum(lens[:i]) for i in range(len(lens) + 1)]),
+                                    as_i32([kv_lens[s] for s in seqs]), seq, d ** -0.5, window)
+        return out
+
+    whole, at = run(q, list(range(len(q_lens)))), 0
+    assert bool(torch.isfinite(whole).all())
+    for s, m in enumerate(q_lens):
+        assert torch.equal(run(q[at:at + m].contiguous(), [s]), whole[at:at + m])
+        at += m
