@@ -102,7 +102,7 @@ template <> struct Pair<__nv_bfloat16> {
     __device__ __forceinline__ float2 get() const { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
 };
 
-// kPairs: M is even, so that the weights of two neighbouring outputs stand on pair boundaries.
+// kPairs: the weights of two neighbouring outputs are read as one (see heads_pairs).
 template <typename T, typename TO, bool kPairs>
 __global__ void __launch_bounds__(32 * kSlices)
 heads_linear_kernel(const T* __restrict__ a, long a_tok, int a_head, const T* __restrict__ w, TO* __restrict__ out, long o_tok,
@@ -390,6 +390,10 @@ int launch_sigmoid_gate(T* x, const T* gate, long g_tok, int N, int width, cudaS
     return launch_status();
 }
 
+// Whether the weights of two neighbouring outputs stand on a boundary of their pair: M is even and w itself stands on one.  (w may
+// be a view that begins at an odd element; its weights are then read one at a time, as those of an odd M are.)
+bool heads_pairs(const void* w, int M, size_t size) { return M % 2 == 0 && (uintptr_t)w % (2 * size) == 0; }
+
 template <typename T, typename TO>
 int launch_heads(const void* a, long a_tok, int a_head, const void* w, void* out, long o_tok, int o_head, const void* gate,
                  long g_tok, int N, int H, int M, int K, cudaStream_t stream) {
@@ -407,7 +411,7 @@ int launch_heads(const void* a, long a_tok, int a_head, const void* w, void* out
     }();
     if (allowed != cudaSuccess) return (int)allowed;
     dim3 grid((N + kTok - 1) / kTok, H, (M + kOuts - 1) / kOuts);
-    const auto kernel = M % 2 == 0 ? heads_linear_kernel<T, TO, true> : heads_linear_kernel<T, TO, false>;
+    const auto kernel = heads_pairs(w, M, sizeof(T)) ? heads_linear_kernel<T, TO, true> : heads_linear_kernel<T, TO, false>;
     return launch_pdl(kernel, grid, dim3(32 * kSlices), smem, stream, (const T*)a, a_tok, a_head, (const T*)w, (TO*)out, o_tok, o_head,
                       (const T*)gate, g_tok, N, M, K);
 }
@@ -430,6 +434,9 @@ PB_EXPORT int pb_heads_linear(int dtype, int out_dtype, const void* a, long a_to
         return launch_heads<__nv_bfloat16, __nv_bfloat16>(a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, stream);
     return PB_ERR_BAD_DTYPE;
 }
+
+// 1 where pb_heads_linear reads such weights in pairs (a few tokens), 0 where one at a time.
+PB_EXPORT int pb_heads_linear_pairs(int dtype, const void* w, int M) { return heads_pairs(w, M, dtype == PB_F32 ? 4 : 2) ? 1 : 0; }
 
 // q: the projected query rows, head h at q + n * q_tok + h * (dim + rot_dim), its rotated part behind `dim` plain
 // dimensions.  down (may be null: the layer borrows another layer's cache): rows of rank + rot_dim at n * down_tok.
