@@ -138,17 +138,20 @@ __device__ __forceinline__ float squared_relu(float x) {
 // SMs while the kernel before it on the stream is finishing: as soon as every block of that
 // kernel has called pdl_trigger (or exited).  It must call pdl_wait before it touches anything
 // an earlier kernel writes (or reads and later overwrites); pdl_wait returns once the preceding
-// kernel has completed and its writes are visible.  Every kernel of the chain waits first thing,
-// so completion is transitive; kernels trigger late, after their main loop, so that the next
-// kernel's launch overlaps only this kernel's tail.  Both calls do nothing in a kernel that was
-// launched the ordinary way.
+// kernel has completed and its writes are visible.  Every kernel of the chain waits in all of its
+// blocks, so completion is transitive.  Kernels with a main loop trigger late, behind it, so that
+// the next kernel's launch overlaps only this kernel's tail; short ones (norms, prepares, merges)
+// trigger first thing, so several kernels ahead may still be running when a kernel begins: what
+// one reads before pdl_wait has to be finished long before, as loaded weights and the keys of
+// earlier steps are.  Both calls do nothing in a kernel that was launched the ordinary way.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 bool pdl_enabled();      // PULSAR_PDL=0 launches every kernel the ordinary way
 
+// early = false: the ordinary way, behind everything that the stream holds.
 template <typename... KArgs, typename... Args>
-inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+inline int launch_early(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -158,8 +161,13 @@ inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = early && pdl_enabled() ? 1 : 0;
     return (int)cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_early(true, kernel, grid, block, smem, stream, args...);
 }
 
 }  // namespace pb

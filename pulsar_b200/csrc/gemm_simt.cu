@@ -24,10 +24,10 @@ using namespace pb;
 // Bound by reading W once, and with more rows of A by shared memory.  The sums stay chains in ascending k: a chain takes 4 cycles
 // a step, so 128 blocks of 32 weight rows ask for 8 TB/s, above what HBM gives, and a split of K (which would change the sums)
 // is not needed.  W and A come through shared memory in stages of 64 k by 16-byte asynchronous copies of four warps that do
-// nothing else; CW further warps compute, a thread R rows of W times T rows of A.  W depends on no earlier kernel: its first
-// stages are asked for before griddepcontrol.wait.  A 16-byte read of shared memory costs a warp 4 cycles, 2 where neighbouring
-// lanes read the same place (measured), so lanes that share a row of W stand side by side; W's rows stand 68 floats apart, which
-// keeps the others off each other's banks.
+// nothing else; CW further warps compute, a thread R rows of W times T rows of A.  A loaded W depends on no earlier kernel: its first
+// stages are asked for before griddepcontrol.wait (a W that may just have been computed: the ordinary launch, which begins behind
+// it).  A 16-byte read of shared memory costs a warp 4 cycles, 2 where neighbouring lanes read the same place (measured), so lanes
+// that share a row of W stand side by side; W's rows stand 68 floats apart, which keeps the others off each other's banks.
 // us on the sizes of an 8B layer, 64 x 64 tiles of the general kernel before: 6144 x 4096 1 row 21.7 (was 277), 4 rows 27.2, 8 rows
 // 36.7, 16 rows 63; 4096 x 4096 19.3 / 21.6 / 27.4 / 47 (282); 24576 x 4096 66.8 / 74.8 / 103 / 188 (480); 4096 x 12288
 // 43.7 / 50.8 / 69 / 120 (851); 151936 x 4096 376 (6.6 TB/s) / 406 / 562 / 1055.
@@ -153,21 +153,21 @@ simt_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* _
 }
 
 template <int R, int T, int CW, int RST, typename TO>
-int launch_rows_st(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
+int launch_rows_st(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
     constexpr int MR = 32 / (RN / R) * T * CW;
     constexpr size_t smem = sizeof(float) * RST * (RN * RSTRIDE + MR * RK);
     static const cudaError_t allowed =
         cudaFuncSetAttribute(simt_rows_kernel<R, T, CW, RST, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (allowed != cudaSuccess) return (int)allowed;
-    return launch_pdl(simt_rows_kernel<R, T, CW, RST, TO>, dim3((N + RN - 1) / RN), dim3(RLOAD + 32 * CW), smem, stream, A, W, out, M, N, K);
+    return launch_early(loaded, simt_rows_kernel<R, T, CW, RST, TO>, dim3((N + RN - 1) / RN), dim3(RLOAD + 32 * CW), smem, stream, A, W, out, M, N, K);
 }
 
 // With one block an SM or fewer a block's ring has to keep HBM busy by itself: 16 stages instead of 8 (4096 x 4096, one row of A:
 // 19.3 against 19.5 us; 4096 x 12288: 43.9 against 50.3).
 template <int R, int T, int CW, typename TO>
-int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
-    if ((N + RN - 1) / RN <= 148) return launch_rows_st<R, T, CW, 16>(A, W, out, M, N, K, stream);
-    return launch_rows_st<R, T, CW, 8>(A, W, out, M, N, K, stream);
+int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
+    if ((N + RN - 1) / RN <= 148) return launch_rows_st<R, T, CW, 16>(A, W, out, M, N, K, loaded, stream);
+    return launch_rows_st<R, T, CW, 8>(A, W, out, M, N, K, loaded, stream);
 }
 
 // ---------------------------------------------------------------- more rows
@@ -277,13 +277,13 @@ int launch_tile(const float* A, const float* W, TO* out, int M, int N, int K, cu
 
 // float32 operands whose rows are multiples of 16 bytes on 16-byte addresses
 template <typename TO>
-int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
-    if (M == 1) return launch_rows<1, 1, 1>(A, W, out, M, N, K, stream);
-    if (M == 2) return launch_rows<2, 1, 1>(A, W, out, M, N, K, stream);
-    if (M <= 4) return launch_rows<2, 1, 2>(A, W, out, M, N, K, stream);
+int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
+    if (M == 1) return launch_rows<1, 1, 1>(A, W, out, M, N, K, loaded, stream);
+    if (M == 2) return launch_rows<2, 1, 1>(A, W, out, M, N, K, loaded, stream);
+    if (M <= 4) return launch_rows<2, 1, 2>(A, W, out, M, N, K, loaded, stream);
     const bool few = (N + RN - 1) / RN <= 148;
-    if (M <= 8) return few ? launch_rows<2, 1, 4>(A, W, out, M, N, K, stream) : launch_rows<2, 2, 2>(A, W, out, M, N, K, stream);
-    if (M <= 16) return few ? launch_rows<2, 1, 8>(A, W, out, M, N, K, stream) : launch_rows<4, 2, 2>(A, W, out, M, N, K, stream);
+    if (M <= 8) return few ? launch_rows<2, 1, 4>(A, W, out, M, N, K, loaded, stream) : launch_rows<2, 2, 2>(A, W, out, M, N, K, loaded, stream);
+    if (M <= 16) return few ? launch_rows<2, 1, 8>(A, W, out, M, N, K, loaded, stream) : launch_rows<4, 2, 2>(A, W, out, M, N, K, loaded, stream);
     // 64 rows a block where there are blocks for 16 rounds of the SMs (151936 x 4096, 387 rows: 11.3 against 11.9 ms), else 32, whose last
     // rounds are less empty (4096 x 4096: 33 rows 161 against 269 us, 387 rows 356 against 500, the general kernel 656;
     // 24576 x 4096, 387 rows: 1.90 against 2.00 ms, 2.96 before)
@@ -356,16 +356,15 @@ int launch(const void* A, const void* W, void* out, int M, int N, int K, cudaStr
 
 }  // namespace
 
-// a_dtype / w_dtype / out_dtype: PB_F32 or PB_BF16.
-PB_EXPORT int pb_gemm_simt(int a_dtype, int w_dtype, int out_dtype, const void* A, const void* W, void* out,
-                           int M, int N, int K, cudaStream_t stream) {
+static int gemm_simt(int a_dtype, int w_dtype, int out_dtype, const void* A, const void* W, void* out, int M, int N, int K, bool loaded,
+                     cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return PB_ERR_BAD_SIZE;
     if ((a_dtype | w_dtype | out_dtype) & ~1) return PB_ERR_BAD_DTYPE;
     typedef __nv_bfloat16 bf;
     if (a_dtype == PB_F32 && w_dtype == PB_F32 && K % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0) {
-        const int status = out_dtype == PB_F32 ? launch_f32((const float*)A, (const float*)W, (float*)out, M, N, K, stream)
-                                               : launch_f32((const float*)A, (const float*)W, (bf*)out, M, N, K, stream);
+        const int status = out_dtype == PB_F32 ? launch_f32((const float*)A, (const float*)W, (float*)out, M, N, K, loaded, stream)
+                                               : launch_f32((const float*)A, (const float*)W, (bf*)out, M, N, K, loaded, stream);
         if (status != PB_ERR_TOO_LARGE) return status;
     }
     const int key = a_dtype * 4 + w_dtype * 2 + out_dtype;
@@ -380,4 +379,16 @@ PB_EXPORT int pb_gemm_simt(int a_dtype, int w_dtype, int out_dtype, const void* 
         case 7: return launch<bf, bf, bf>(A, W, out, M, N, K, stream);
     }
     return PB_ERR_BAD_DTYPE;
+}
+
+// a_dtype / w_dtype / out_dtype: PB_F32 or PB_BF16.
+PB_EXPORT int pb_gemm_simt(int a_dtype, int w_dtype, int out_dtype, const void* A, const void* W, void* out,
+                           int M, int N, int K, cudaStream_t stream) {
+    return gemm_simt(a_dtype, w_dtype, out_dtype, A, W, out, M, N, K, false, stream);
+}
+
+// The same for a W that no kernel still on the stream writes (a loaded weight): it may be read before those have ended.
+PB_EXPORT int pb_gemm_simt_loaded(int a_dtype, int w_dtype, int out_dtype, const void* A, const void* W, void* out,
+                                  int M, int N, int K, cudaStream_t stream) {
+    return gemm_simt(a_dtype, w_dtype, out_dtype, A, W, out, M, N, K, true, stream);
 }

@@ -73,7 +73,7 @@ heads_linear_wide_kernel(const T* __restrict__ a, long a_tok, int a_head, const 
 
 // A few tokens: bound by the trips to L2, not by bytes (16 heads of 512 x 128 are 2 MB).  A block takes 8 tokens x 64 outputs; its
 // eight warps are slices of K, a lane two neighbouring outputs (one 4-byte load of bfloat16), 16 k asked for at once and the next
-// 16 while these are used.  The weights depend on no earlier kernel: the first batch is asked for before griddepcontrol.wait.
+// 16 while these are used.  `loaded` weights depend on no earlier kernel: the first batch is asked for before griddepcontrol.wait.
 // 8 tokens, 16 heads, bfloat16: 512 -> 128 with the gate 12.7 -> 5.5 us, 128 -> 512 to float32 4.6 -> 2.8 (four slices of single
 // outputs before).
 constexpr int kSlices = 8;
@@ -106,7 +106,7 @@ template <> struct Pair<__nv_bfloat16> {
 template <typename T, typename TO, bool kPairs>
 __global__ void __launch_bounds__(32 * kSlices)
 heads_linear_kernel(const T* __restrict__ a, long a_tok, int a_head, const T* __restrict__ w, TO* __restrict__ out, long o_tok,
-                    int o_head, const T* __restrict__ gate, long g_tok, int N, int M, int K) {
+                    int o_head, const T* __restrict__ gate, long g_tok, int N, int M, int K, bool loaded) {
     extern __shared__ __align__(16) float smem[];
     const int KS = heads_slice(K), KP = KS * kSlices;
     float* a_s = smem;                             // [kTok][KP], zeros behind K
@@ -129,8 +129,9 @@ heads_linear_kernel(const T* __restrict__ a, long a_tok, int a_head, const T* __
         }
     };
     Pair<T> wv[2][kBatch];
-    fetch(wv[0], k0);
+    if (loaded) fetch(wv[0], k0);
     pdl_wait();         // may have come onto the SMs while the product before it was ending: nothing else is touched before that one is done
+    if (!loaded) fetch(wv[0], k0);
     if (K % 4 == 0 && a_tok % 4 == 0 && a_head % 4 == 0 && (uintptr_t)a % 16 == 0) {
         for (int i = threadIdx.x; i < kTok * (KP >> 2); i += blockDim.x) {
             const int tt = i / (KP >> 2), k = i % (KP >> 2) * 4;
@@ -396,7 +397,7 @@ bool heads_pairs(const void* w, int M, size_t size) { return M % 2 == 0 && (uint
 
 template <typename T, typename TO>
 int launch_heads(const void* a, long a_tok, int a_head, const void* w, void* out, long o_tok, int o_head, const void* gate,
-                 long g_tok, int N, int H, int M, int K, cudaStream_t stream) {
+                 long g_tok, int N, int H, int M, int K, bool loaded, cudaStream_t stream) {
     if (N > 2 * kTok) {         // enough token tiles to fill the GPU without cutting K
         dim3 wide((N + kTok - 1) / kTok, H, (M + 127) / 128);
         heads_linear_wide_kernel<T, TO><<<wide, 128, sizeof(float) * kTok * ((K + 3) & ~3), stream>>>(
@@ -413,26 +414,37 @@ int launch_heads(const void* a, long a_tok, int a_head, const void* w, void* out
     dim3 grid((N + kTok - 1) / kTok, H, (M + kOuts - 1) / kOuts);
     const auto kernel = heads_pairs(w, M, sizeof(T)) ? heads_linear_kernel<T, TO, true> : heads_linear_kernel<T, TO, false>;
     return launch_pdl(kernel, grid, dim3(32 * kSlices), smem, stream, (const T*)a, a_tok, a_head, (const T*)w, (TO*)out, o_tok, o_head,
-                      (const T*)gate, g_tok, N, M, K);
+                      (const T*)gate, g_tok, N, M, K, loaded);
 }
 
 }  // namespace
+
+static int heads_linear(int dtype, int out_dtype, const void* a, long a_tok, int a_head, const void* w, void* out, long o_tok, int o_head,
+                        const void* gate, long g_tok, int N, int H, int M, int K, bool loaded, cudaStream_t stream) {
+    if (N <= 0) return 0;
+    if (H <= 0 || M <= 0 || K <= 0 || K > 1024 || (M + 31) / 32 > 65535) return PB_ERR_BAD_SIZE;
+    if (H > 65535) return PB_ERR_TOO_LARGE;
+    if (dtype == PB_F32 && out_dtype == PB_F32)
+        return launch_heads<float, float>(a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, loaded, stream);
+    if (dtype == PB_BF16 && out_dtype == PB_F32)
+        return launch_heads<__nv_bfloat16, float>(a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, loaded, stream);
+    if (dtype == PB_BF16 && out_dtype == PB_BF16)
+        return launch_heads<__nv_bfloat16, __nv_bfloat16>(a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, loaded, stream);
+    return PB_ERR_BAD_DTYPE;
+}
 
 // out[n, h, m] = sum_k a[n, h, k] * w[h, k, m]  (* sigmoid(gate[n, h * M + m]) where a gate is given).
 // a: element (n, h, k) at n * a_tok + h * a_head + k; out likewise with o_tok, o_head; w contiguous [H, K, M].
 // dtype: of a, w and gate; out_dtype: of out (float32, or the same as dtype).
 PB_EXPORT int pb_heads_linear(int dtype, int out_dtype, const void* a, long a_tok, int a_head, const void* w, void* out, long o_tok,
                               int o_head, const void* gate, long g_tok, int N, int H, int M, int K, cudaStream_t stream) {
-    if (N <= 0) return 0;
-    if (H <= 0 || M <= 0 || K <= 0 || K > 1024 || (M + 31) / 32 > 65535) return PB_ERR_BAD_SIZE;
-    if (H > 65535) return PB_ERR_TOO_LARGE;
-    if (dtype == PB_F32 && out_dtype == PB_F32)
-        return launch_heads<float, float>(a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, stream);
-    if (dtype == PB_BF16 && out_dtype == PB_F32)
-        return launch_heads<__nv_bfloat16, float>(a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, stream);
-    if (dtype == PB_BF16 && out_dtype == PB_BF16)
-        return launch_heads<__nv_bfloat16, __nv_bfloat16>(a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, stream);
-    return PB_ERR_BAD_DTYPE;
+    return heads_linear(dtype, out_dtype, a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, false, stream);
+}
+
+// The same for weights that no kernel still on the stream writes (loaded ones): they may be read before those have ended.
+PB_EXPORT int pb_heads_linear_loaded(int dtype, int out_dtype, const void* a, long a_tok, int a_head, const void* w, void* out, long o_tok,
+                                     int o_head, const void* gate, long g_tok, int N, int H, int M, int K, cudaStream_t stream) {
+    return heads_linear(dtype, out_dtype, a, a_tok, a_head, w, out, o_tok, o_head, gate, g_tok, N, H, M, K, true, stream);
 }
 
 // 1 where pb_heads_linear reads such weights in pairs (a few tokens), 0 where one at a time.

@@ -138,7 +138,7 @@ class DecoderModel(Part):
         n, width = residual.shape
         both = ctx.scratch("walk.in", (n, 2 * width))
         ops.concat_streams(residual, delta, origin, both)
-        ops.linear(both, self.walk_in, residual)
+        ops.linear(both, self.walk_in, residual, loaded=True)
         ops.add_bias(residual, self.walk_step[t])
         return None
 
@@ -173,7 +173,7 @@ class DecoderModel(Part):
         logits = ctx.scratch("logits", (rows.numel(), s.vocab_size), torch.float32)
         if rows.numel():
             h = self.final_norm.forward(ctx, residual, delta, rows=rows)
-            ops.linear(h, self.head, logits)
+            ops.linear(h, self.head, logits, loaded=True)
             if s.logit_scale != 1.0 or s.logit_softcap is not None:
                 ops.scale_cap(logits, s.logit_scale, s.logit_softcap)
         return logits

@@ -82,6 +82,7 @@ _SIGNATURES = {
     "pb_set_pool_bounds": [_I, _P],
     "pb_set_gating": [_F, _F, _F],
     "pb_gemm_simt": [_I, _I, _I, _P, _P, _P, _I, _I, _I, _P],
+    "pb_gemm_simt_loaded": [_I, _I, _I, _P, _P, _P, _I, _I, _I, _P],
     "pb_sample": [_P, _I, _I, _P, _P, _P, _P, _I, _P, _P, _P, _P],
     "pb_sample_workspace": [_I],
     "pb_argmax": [_P, _I, _I, _P, _P, _P],
@@ -93,6 +94,7 @@ _SIGNATURES = {
     "pb_paged_attention_general_tc": [_I, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _F, _P, _I, _I, _I, _P, _P, _P, _P],
     "pb_qkv_split_write": [_I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _F, _I, _P],
     "pb_heads_linear": [_I, _I, _P, _L, _I, _P, _P, _L, _I, _P, _L, _I, _I, _I, _I, _P],
+    "pb_heads_linear_loaded": [_I, _I, _P, _L, _I, _P, _P, _L, _I, _P, _L, _I, _I, _I, _I, _P],
     "pb_heads_linear_pairs": [_I, _P, _I],
     "pb_latent_prepare": [_I, _P, _L, _P, _L, _P, _F, _P, _P, _P, _P, _P, _I, _I, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "pb_latent_norms": [_I, _P, _L, _P, _P, _P, _L, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
@@ -161,8 +163,9 @@ def fn(name: str):
         f = getattr(library(), name)
         f.argtypes = _SIGNATURES[name]
         f.restype = _RETURNS.get(name, ctypes.c_int)
-        if profiling.ENABLED and name[3:] in _LAUNCHERS:
-            f = profiling.timed_launcher(name, f)
+        launched = name.removesuffix("_loaded")          # the same kernel
+        if profiling.ENABLED and launched[3:] in _LAUNCHERS:
+            f = profiling.timed_launcher(launched, f)
         _fns[name] = f
     return f
 
@@ -316,14 +319,15 @@ def paged_attention_generic(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch
                                            page_size, float(scale), int(window or 0), stream()), "paged_attention_generic")
 
 
-def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out = a @ w.T in float32 multiply-adds (no tensor cores)."""
+def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, loaded: bool = False) -> None:
+    """out = a @ w.T in float32 multiply-adds (no tensor cores).  ``loaded`` promises that no kernel still on the stream writes
+    ``w``, as none does a model's weights: the product may then read it before the kernels ahead of it have ended."""
     _cuda(a, w, out)
     m, k = a.shape
     n, k2 = w.shape
     assert k2 == k and out.shape == (m, n)
-    check(fn("pb_gemm_simt")(code(a.dtype), code(w.dtype), code(out.dtype), _p(a), _p(w), _p(out), m, n, k, stream()),
-          "gemm_simt")
+    name = "pb_gemm_simt_loaded" if loaded else "pb_gemm_simt"
+    check(fn(name)(code(a.dtype), code(w.dtype), code(out.dtype), _p(a), _p(w), _p(out), m, n, k, stream()), "gemm_simt")
 
 
 _argmax_keys = {}
@@ -676,14 +680,16 @@ def check_wait_words() -> None:
         raise DeviceWaitError(what)
 
 
-def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, loaded: bool = False) -> None:
     """out = a @ w.T.  float32 operands take the float32 CUDA-core product (true 32-bit,
     no reduced-precision mode).  bfloat16 operands: up to 16 rows take this library's
     weight-streaming kernel; more rows take the library product with float32 accumulation,
     as the reference does for every projection (pulsar-core/src/model/qwen3.cpp:82-84:
-    at::linear)."""
+    at::linear).  ``loaded``: as ``gemm_simt`` has it, for float32.  The bfloat16 streaming
+    kernels read ``w`` early in any case: it has to be a weight that was there before the
+    kernels still on the stream were launched."""
     if a.dtype == torch.float32 and w.dtype == torch.float32:
-        gemm_simt(a, w, out)
+        gemm_simt(a, w, out, loaded)
         return
     _cuda(a, w, out)
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
@@ -708,13 +714,13 @@ def _library_product(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> Non
         torch.mm(a, w.t(), out_dtype=torch.float32, out=out)
 
 
-def gated_linear(ctx, a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, gating=None) -> None:
+def gated_linear(ctx, a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, gating=None, loaded: bool = False) -> None:
     """out [M, I] = silu(a Wg^T) * (a Wu^T) with ``w_gate_up`` = gate rows then up rows; with ``gating`` = (limit, alpha,
     shift) the clamped form g * sigmoid(alpha * g) * (u + shift), g = min(a Wg^T, limit), u = clamp(a Wu^T, -limit, limit)
     (alpha infinite: max(g, 0) * (u + shift)).
     In bfloat16, up to 16 rows (the weight-streaming kernel) and more than 128 rows (the tcgen05 kernel)
     take one kernel that never writes the [M, 2I] intermediate; otherwise the product followed by the
-    gating kernel."""
+    gating kernel.  ``loaded``: as ``linear`` has it."""
     if gemm_skinny(a, w_gate_up, out, swiglu=True, gating=gating):
         return
     if gating is None and _stream_wanted(a.shape[0], w_gate_up.shape[0]) and gemm_tcgen05_stream(a, w_gate_up, out, swiglu=True):
@@ -725,7 +731,7 @@ def gated_linear(ctx, a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tenso
     if fused and gemm_tcgen05(a, w_gate_up, out, swiglu=True, gating=gating):
         return
     gate_up = ctx.scratch("mlp.gate_up", (a.shape[0], w_gate_up.shape[0]), a.dtype)
-    linear(a, w_gate_up, gate_up)
+    linear(a, w_gate_up, gate_up, loaded)
     if gating is None:
         silu_mul(gate_up, out)
     elif gating[2] == 1.0:
@@ -1005,7 +1011,7 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
                             ctx.seq_of_token, scale, window)
 
 
-def squared_relu_linear(ctx, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+def squared_relu_linear(ctx, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, loaded: bool = False) -> None:
     """out [M, N] = max(a @ w.T, 0)^2.  In bfloat16, up to 16 rows (the weight-streaming kernel) and more than 128 rows (the
     tcgen05 kernel) apply it in the product's epilogue; otherwise the product leaves float32 rows for the activation kernel."""
     if gemm_skinny(a, w, out, squared_relu=True):
@@ -1014,7 +1020,7 @@ def squared_relu_linear(ctx, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor
     if fused and gemm_tcgen05(a, w, out, squared_relu=True):
         return
     rows = ctx.scratch("mlp.up32", out.shape, torch.float32)
-    linear(a, w, rows)
+    linear(a, w, rows, loaded)
     activation(rows, out, "relu2")
 
 
@@ -1153,10 +1159,12 @@ def qkv_split_write(qkv: torch.Tensor, q_out: torch.Tensor, k_pool: Optional[tor
                                    n_v, key_dim, value_dim, page_size, _p(positions), coef, every, stream()), "qkv_split_write")
 
 
-def heads_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate: Optional[torch.Tensor] = None) -> None:
+def heads_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate: Optional[torch.Tensor] = None,
+                 loaded: bool = False) -> None:
     """out[n, h, :] = a[n, h, :] @ w[h] for every head (float32 sums in ascending k), times sigmoid(gate[n, h, :]) where a
     gate is given.  ``a`` [N, H, K], ``out`` [N, H, M] and ``gate`` [N, H * M] may be views whose last dimension is
-    contiguous; ``w`` [H, K, M] is contiguous.  ``out`` is float32 or of the dtype of ``a`` and ``w``."""
+    contiguous; ``w`` [H, K, M] is contiguous.  ``out`` is float32 or of the dtype of ``a`` and ``w``.  ``loaded``: as
+    ``gemm_simt`` has it."""
     n, h, k = a.shape
     h2, k2, m = w.shape
     assert (h2, k2) == (h, k) and out.shape == (n, h, m) and a.dtype == w.dtype and w.is_contiguous()
@@ -1165,8 +1173,9 @@ def heads_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate: Opti
     if gate is not None:
         assert gate.dtype == a.dtype and gate.shape == (n, h * m) and gate.stride(1) == 1 and gate.is_cuda
         g_tok = gate.stride(0)
-    check(fn("pb_heads_linear")(code(a.dtype), code(out.dtype), _p(a), a.stride(0), a.stride(1), _p(w), _p(out), out.stride(0),
-                                out.stride(1), _p(gate), g_tok, n, h, m, k, stream()), "heads_linear")
+    name = "pb_heads_linear_loaded" if loaded else "pb_heads_linear"
+    check(fn(name)(code(a.dtype), code(out.dtype), _p(a), a.stride(0), a.stride(1), _p(w), _p(out), out.stride(0), out.stride(1),
+                   _p(gate), g_tok, n, h, m, k, stream()), "heads_linear")
 
 
 def latent_prepare(q: torch.Tensor, down: Optional[torch.Tensor], norm_weight: Optional[torch.Tensor], eps: float,

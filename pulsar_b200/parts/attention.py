@@ -225,14 +225,14 @@ class Attention(Mixer):
             qkv = ctx.scratch("attn.qkv32", (n, self.w_qkv.shape[0]), torch.float32)
         else:
             qkv = ctx.scratch("attn.qkv", (n, self.w_qkv.shape[0]))
-        ops.linear(h, self.w_qkv, qkv)
+        ops.linear(h, self.w_qkv, qkv, loaded=True)
         o = self._attend_general(ctx, qkv, cache) if self.general else self._attend(ctx, qkv, cache)
         if s.output_gate or s.gate_per_head:
             columns = s.n_heads * (1 if s.gate_per_head else s.value_dim)
             ops.sigmoid_gate_strided(o.view(n, s.n_heads * s.value_dim), qkv[:, self.gate_at:self.gate_at + columns],
                                      group=s.value_dim if s.gate_per_head else 1)
         out = ctx.scratch("attn.out", (n, s.hidden), torch.float32 if self.output_float32 else None)
-        ops.linear(o.view(n, s.n_heads * s.value_dim), self.w_o, out)
+        ops.linear(o.view(n, s.n_heads * s.value_dim), self.w_o, out, loaded=True)
         if self.output_bias is not None and not self.defer_output_bias:
             ops.add_bias(out, self.output_bias)
         return out
@@ -292,7 +292,7 @@ class Attention(Mixer):
         qkv = ctx.scratch("attn.qkv", (n, (s.n_heads + 2 * n_kv) * s.head_dim))
         prepared = ctx.prepared_norms.pop(id(norm), None)
         if prepared is None or not ops.linear_prenormed(prepared[0], prepared[1], norm.spec.eps, self.w_qkv, qkv):
-            ops.linear(norm.forward(ctx, residual, None), self.w_qkv, qkv)
+            ops.linear(norm.forward(ctx, residual, None), self.w_qkv, qkv, loaded=True)
         o = self._attend(ctx, qkv, cache)
         ctx.prepared_norms.clear()              # the residual changes now
         if not accumulate_and_prepare(ctx, o.view(n, s.n_heads * s.head_dim), self.w_o, residual,

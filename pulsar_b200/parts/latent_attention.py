@@ -124,7 +124,7 @@ class LatentAttention(Mixer):
         s, n, H = self.spec, ctx.n_tokens, self.spec.n_heads
         q_width = self.q_rank or H * (s.head_dim + self.rot_dim)
         proj = ctx.scratch("latent.in", (n, self.w_in.shape[0]))
-        ops.linear(h, self.w_in, proj)
+        ops.linear(h, self.w_in, proj, loaded=True)
         q = proj[:, :q_width]
         down = proj[:, q_width:q_width + self.row] if s.own_kv else None
         gate = proj[:, self.w_in.shape[0] - H * s.value_dim:] if self.gated else None
@@ -142,7 +142,7 @@ class LatentAttention(Mixer):
             ops.latent_norms(q, self.q_norm, q_lat, self.norm_eps, down, self.latent_norm, cos, sin, cache.slots if s.own_kv else None,
                              pool if s.own_kv else None, self.rank, self.rot_dim, cache.page_size, *kept)
             q, down = ctx.scratch("latent.q_up", (n, H * (s.head_dim + self.rot_dim))), None
-            ops.linear(q_lat, self.w_q, q)
+            ops.linear(q_lat, self.w_q, q, loaded=True)
         # A step that brings only whole prompts (every sequence starts at 0) has all its keys among its own tokens: it
         # expands them once (two products for the step) and attends with keys head_dim + rot_dim wide and values value_dim
         # wide, a third of the absorbed form's arithmetic per (query, key) pair.  Every other step (portions behind a
@@ -157,21 +157,21 @@ class LatentAttention(Mixer):
         if head_gate is not None:
             ops.sigmoid_gate_strided(heads.view(n, H * s.value_dim), head_gate, group=s.value_dim)
         out = ctx.scratch("latent.out", (n, s.hidden), torch.float32 if self.output_float32 else None)
-        ops.linear(heads.view(n, H * s.value_dim), self.w_o, out)
+        ops.linear(heads.view(n, H * s.value_dim), self.w_o, out, loaded=True)
         return out
 
     def _absorbed(self, ctx, q, down, gate, cos, sin, cache) -> torch.Tensor:
         s, n, H = self.spec, ctx.n_tokens, self.spec.n_heads
         pool = cache.pools["latent"]
         q_full = ctx.scratch("latent.q", (n, H, self.row), torch.float32)
-        ops.heads_linear(q.view(n, H, s.head_dim + self.rot_dim)[:, :, :s.head_dim], self.w_uk_t, q_full[:, :, :self.rank])
+        ops.heads_linear(q.view(n, H, s.head_dim + self.rot_dim)[:, :, :s.head_dim], self.w_uk_t, q_full[:, :, :self.rank], loaded=True)
         own = down is not None
         ops.latent_prepare(q, down, self.latent_norm, self.norm_eps, cos, sin, cache.slots if own else None, pool if own else None, q_full, H, s.head_dim, self.rot_dim, self.rank, cache.page_size)
         mixed = ctx.scratch("latent.mixed", (n, H, self.rank))
         ops.paged_attention_general(ctx, q_full, pool, pool, mixed, cache.block_table, s.scale, s.window, s.chunk, None,
                                     key_width=self.row, value_width=self.rank, sinks=self.sinks)
         heads = ctx.scratch("latent.heads", (n, H, s.value_dim))
-        ops.heads_linear(mixed, self.w_uv, heads, gate)
+        ops.heads_linear(mixed, self.w_uv, heads, gate, loaded=True)
         return heads
 
     def _step_rows(self, ctx, pool):
@@ -194,9 +194,9 @@ class LatentAttention(Mixer):
             ops.latent_prepare(q, None, None, self.norm_eps, cos, sin, None, None, q_cat, H, s.head_dim, self.rot_dim, self.rank,
                                cache.page_size, plain_too=True)
         k_plain = ctx.scratch("latent.k_plain", (n, H * s.head_dim))
-        ops.linear(latent, self.w_uk_rows, k_plain)
+        ops.linear(latent, self.w_uk_rows, k_plain, loaded=True)
         values = ctx.scratch("latent.values", (n, H * s.value_dim))
-        ops.linear(latent, self.w_uv_rows, values)
+        ops.linear(latent, self.w_uv_rows, values, loaded=True)
         keys = ctx.scratch("latent.keys", (n, H, s.head_dim + self.rot_dim))
         ops.latent_expand_keys(k_plain.view(n, H, s.head_dim), shared, keys)
         # the step's own rows as pages of one token: row t of sequence i is page cu_q[i] + t

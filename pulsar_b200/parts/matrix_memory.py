@@ -75,10 +75,10 @@ class MatrixMemory(Mixer):
     def forward(self, ctx: StepContext, h: torch.Tensor, cache: CacheView) -> torch.Tensor:
         s, n = self.spec, ctx.n_tokens
         rows = ctx.scratch("memory.rows", (n, self.w_in.shape[0]), torch.float32)
-        ops.linear(h, self.w_in, rows)
+        ops.linear(h, self.w_in, rows, loaded=True)
         y = ctx.scratch("memory.y", (n, s.n_heads * s.value_dim))
         ops.matrix_memory(ctx, rows, self.b_i, self.b_f, self.cap, self.norm, s.norm_eps, cache.state, y, s.n_heads, s.head_dim, s.value_dim,
                           self.q_scale, self.denom_eps)
         out = ctx.scratch("memory.out", (n, s.hidden), torch.float32 if self.output_float32 else None)
-        ops.linear(y, self.w_o, out)
+        ops.linear(y, self.w_o, out, loaded=True)
         return out

@@ -57,9 +57,9 @@ class MinGRU(Mixer):
     def forward(self, ctx: StepContext, h: torch.Tensor, cache: CacheView) -> torch.Tensor:
         n = ctx.n_tokens
         proj = ctx.scratch("gru.proj", (n, 3 * self.width), torch.float32)
-        ops.linear(h, self.w_zxg, proj)
+        ops.linear(h, self.w_zxg, proj, loaded=True)
         y = ctx.scratch("gru.y", (n, self.width))
         ops.min_gru(ctx, proj, self.b_z, self.b_x, cache.state, y)
         out = ctx.scratch("gru.out", (n, self.spec.hidden))
-        ops.linear(y, self.w_o, out)
+        ops.linear(y, self.w_o, out, loaded=True)
         return out

@@ -75,7 +75,7 @@ class SwiGLU(FeedForward):
         act = ctx.scratch("mlp.act", (n, s.intermediate))
         prepared = ctx.prepared_norms.pop(id(norm), None) if ops.FUSED_NORM_MLP and self.gating is None else None
         if prepared is None or not ops.linear_prenormed(prepared[0], prepared[1], norm.spec.eps, self.w_gate_up, act, swiglu=True):
-            ops.gated_linear(ctx, norm.forward(ctx, residual, None), self.w_gate_up, act, gating=self.gating)
+            ops.gated_linear(ctx, norm.forward(ctx, residual, None), self.w_gate_up, act, gating=self.gating, loaded=True)
         ctx.prepared_norms.clear()              # the residual changes now
         if not accumulate_and_prepare(ctx, act, self.w_down, residual, next_norm):
             raise ops.KernelError("swiglu: the down projection refused sizes it had declared supported")
@@ -87,12 +87,12 @@ class SwiGLU(FeedForward):
         if self.bias:
             # float32 rows of the product, the biases added before anything is rounded
             gate_up = ctx.scratch("mlp.gate_up32", (n, 2 * s.intermediate), torch.float32)
-            ops.linear(h, self.w_gate_up, gate_up)
+            ops.linear(h, self.w_gate_up, gate_up, loaded=True)
             ops.glu_bias(gate_up, self.b_gate_up, act, self.gating)
         else:
-            ops.gated_linear(ctx, h, self.w_gate_up, act, gating=self.gating)
+            ops.gated_linear(ctx, h, self.w_gate_up, act, gating=self.gating, loaded=True)
         out = ctx.scratch("mlp.out", (n, s.hidden))
-        ops.linear(act, self.w_down, out)
+        ops.linear(act, self.w_down, out, loaded=True)
         if self.output_bias is not None and not self.defer_output_bias:
             ops.add_bias(out, self.output_bias)
         return out
@@ -132,9 +132,9 @@ class ClampedGLU(FeedForward):
     def forward(self, ctx: StepContext, h: torch.Tensor) -> torch.Tensor:
         s, n = self.spec, ctx.n_tokens
         act = ctx.scratch("mlp.act", (n, s.intermediate))
-        ops.gated_linear(ctx, h, self.w_gate_up, act, gating=(self.limit, self.alpha, 1.0))     # the gating in the product's epilogue where it fuses
+        ops.gated_linear(ctx, h, self.w_gate_up, act, gating=(self.limit, self.alpha, 1.0), loaded=True)     # the gating in the product's epilogue where it fuses
         out = ctx.scratch("mlp.out", (n, s.hidden))
-        ops.linear(act, self.w_down, out)
+        ops.linear(act, self.w_down, out, loaded=True)
         return out
 
 
@@ -167,11 +167,11 @@ class ActivatedMLP(FeedForward):
         s, n = self.spec, ctx.n_tokens
         act = ctx.scratch("mlp.act", (n, s.intermediate))
         if s.activation == "relu2":
-            ops.squared_relu_linear(ctx, h, self.w_up, act)
+            ops.squared_relu_linear(ctx, h, self.w_up, act, loaded=True)
         else:
             up = ctx.scratch("mlp.up32", (n, s.intermediate), torch.float32)
-            ops.linear(h, self.w_up, up)
+            ops.linear(h, self.w_up, up, loaded=True)
             ops.activation(up, act, s.activation)
         out = ctx.scratch("mlp.out", (n, s.hidden))
-        ops.linear(act, self.w_down, out)
+        ops.linear(act, self.w_down, out, loaded=True)
         return out

@@ -70,7 +70,7 @@ class Retention(Mixer):
     def forward(self, ctx: StepContext, h: torch.Tensor, cache: CacheView) -> torch.Tensor:
         s, n = self.spec, ctx.n_tokens
         rows = ctx.scratch("retention.rows", (n, self.w_in.shape[0]), torch.float32)
-        ops.linear(h, self.w_in, rows)
+        ops.linear(h, self.w_in, rows, loaded=True)
         cos = sin = None
         rotary = 0
         if self.position is not None:
@@ -80,5 +80,5 @@ class Retention(Mixer):
         ops.retention(ctx, rows, cos, sin, self.decay, cache.state, y, s.n_heads, s.head_dim, s.value_dim, rotary, self.key_scale,
                       s.norm_eps)
         out = ctx.scratch("retention.out", (n, s.hidden), torch.float32 if self.output_float32 else None)
-        ops.linear(y, self.w_o, out)
+        ops.linear(y, self.w_o, out, loaded=True)
         return out

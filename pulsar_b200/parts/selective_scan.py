@@ -78,7 +78,7 @@ class SelectiveScan(Mixer):
     def forward(self, ctx: StepContext, h: torch.Tensor, cache: CacheView) -> torch.Tensor:
         n, w = ctx.n_tokens, self.w
         xz = ctx.scratch("scan.xz", (n, 2 * self.inner))
-        ops.linear(h, w["in"], xz)
+        ops.linear(h, w["in"], xz, loaded=True)
         x = ctx.scratch("scan.x", (n, self.inner))
         ops.causal_conv_silu(ctx, xz, self.inner, w["conv"], w["conv_bias"], cache.state, self.tail_offset, x)
         y = ctx.scratch("scan.y", (n, self.inner))
@@ -88,18 +88,18 @@ class SelectiveScan(Mixer):
             # parallel over tokens where a portion is long, else eight tokens side by side (a captured step of single
             # tokens never comes here)
             r = ctx.scratch("scan.r", (n, self.dt_rank))
-            ops.linear(x, self.w_x_r, r)
+            ops.linear(x, self.w_x_r, r, loaded=True)
             bc = ctx.scratch("scan.bc", (n, 2 * self.n_state))
-            ops.linear(x, self.w_x_bc, bc)
+            ops.linear(x, self.w_x_bc, bc, loaded=True)
             dt_pre = ctx.scratch("scan.dt", (n, self.inner), torch.float32)
-            ops.linear(r, w["dt"], dt_pre)
+            ops.linear(r, w["dt"], dt_pre, loaded=True)
             ops.selective_scan_prompt(ctx, x, xz, bc, dt_pre, w["dt_bias"], w["a_log"], w["d"], cache.state, self.tail_offset,
                                       self.taps, y, chunked=chunked)
         else:
             proj = ctx.scratch("scan.proj", (n, self.dt_rank + 2 * self.n_state))
-            ops.linear(x, w["x"], proj)
+            ops.linear(x, w["x"], proj, loaded=True)
             ops.selective_scan(ctx, x, xz, proj, w["dt"], w["dt_bias"], w["a_log"], w["d"], cache.state, self.tail_offset,
                                self.taps, y)
         out = ctx.scratch("scan.out", (n, self.spec.hidden))
-        ops.linear(y, w["o"], out)
+        ops.linear(y, w["o"], out, loaded=True)
         return out

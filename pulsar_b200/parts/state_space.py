@@ -74,10 +74,10 @@ class StateSpaceDual(Mixer):
     def forward(self, ctx: StepContext, h: torch.Tensor, cache: CacheView) -> torch.Tensor:
         s, n, w = self.spec, ctx.n_tokens, self.w
         rows = ctx.scratch("space.rows", (n, w["in"].shape[0]), torch.float32)
-        ops.linear(h, w["in"], rows)
+        ops.linear(h, w["in"], rows, loaded=True)
         y = ctx.scratch("space.y", (n, self.inner))
         ops.state_space(ctx, rows, w["conv"], w["conv_bias"], w["dt_bias"], w["a_log"], w["d"], w["norm"], self.norm_groups, s.norm_eps,
                         cache.state, y, s.n_heads, self.n_state, s.value_dim, self.n_groups)
         out = ctx.scratch("space.out", (n, s.hidden), torch.float32 if self.output_float32 else None)
-        ops.linear(y, w["o"], out)
+        ops.linear(y, w["o"], out, loaded=True)
         return out

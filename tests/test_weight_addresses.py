@@ -30,3 +30,47 @@ def test_heads_linear_takes_weights_at_any_element(n, heads, k, m, dtype):
         out = torch.empty_like(want)
         ops.heads_linear(a, view, out)
         assert torch.equal(out, want)
+
+
+def test_only_loaded_weights_are_read_before_the_kernels_ahead_have_ended(monkeypatch):
+    """The float32 products and ``heads_linear`` take a ``w`` that an earlier kernel may still be writing unless the caller says
+    that it is a loaded weight."""
+    from pulsar_b200 import ops
+    asked = []
+    monkeypatch.setattr(ops, "fn", lambda name: lambda *args: asked.append(name) or 0)
+    monkeypatch.setattr(ops, "_cuda", lambda *tensors: None)
+    monkeypatch.setattr(ops, "stream", lambda: 0)
+    a, w, out = torch.zeros(2, 8), torch.zeros(4, 8), torch.zeros(2, 4)
+    scratch = type("Ctx", (), {"scratch": lambda self, tag, shape, dtype=None: torch.zeros(shape)})()
+    for call in (lambda **kw: ops.gemm_simt(a, w, out, **kw), lambda **kw: ops.linear(a, w, out, **kw),
+                 lambda **kw: ops.gated_linear(scratch, a, w, torch.zeros(2, 2), **kw)):
+        for kw, name in (({}, "pb_gemm_simt"), (dict(loaded=False), "pb_gemm_simt"), (dict(loaded=True), "pb_gemm_simt_loaded")):
+            asked.clear()
+            call(**kw)
+            assert [n for n in asked if "simt" in n] == [name]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 3, 16])
+def test_a_product_with_a_matrix_that_was_just_computed(m):
+    """``w`` comes from the kernel just before, which lets its successor onto the SMs at its first instruction."""
+    from pulsar_b200 import ops
+    n, k = 4096, 1024
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, ones = torch.randn(m, k, generator=gen, device="cuda"), torch.ones(k, device="cuda")
+    w, out = torch.zeros(n, k, device="cuda"), torch.empty(m, n, device="cuda")
+    heads = torch.empty(m, 4, 1024, device="cuda")
+    for i in range(20):
+        rows = torch.randn(n, k, generator=gen, device="cuda")
+        ops.add_rmsnorm(rows, None, ones, 1e-6, w)
+        ops.linear(a, w, out)
+        first = out.clone()
+        torch.cuda.synchronize()
+        ops.linear(a, w, out)
+        assert torch.equal(out, first)
+        ops.add_rmsnorm(rows, None, ones * 2, 1e-6, w)
+        ops.heads_linear(a.view(m, 1, k).expand(m, 4, k), w.view(4, 1024, 1024), heads)
+        first = heads.clone()
+        torch.cuda.synchronize()
+        ops.heads_linear(a.view(m, 1, k).expand(m, 4, k), w.view(4, 1024, 1024), heads)
+        assert torch.equal(heads, first)
