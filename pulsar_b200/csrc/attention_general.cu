@@ -917,7 +917,7 @@ int dispatch_tiled_bf16(const float* q, const void* k_pool, const void* v_pool, 
     if (!ts.v_in_k) ts.v_row = (ts.g.Dv / 8 | 1) * 8;       // value rows an odd number of 16-byte units apart as well
     const size_t smem = rows_tc_smem(ts);
 #define PB_ROWS_TC(K, V) return launch_rows_tc<K, V>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, row_tiles, ts, smem, stream)
-    if (smem > 0 && smem <= 200 * 1024) {
+    if (smem > 0 && smem <= 200 * 1024 && (uintptr_t)partial % 8 == 0) {                 // partial results are written two floats at a time
         if (ts.g.Dk <= 128 && ts.g.Dv <= 128) PB_ROWS_TC(2, 4);
         if (ts.g.Dk <= 192 && ts.g.Dv <= 128) PB_ROWS_TC(3, 4);
         if (ts.g.Dk <= 320 && ts.g.Dv <= 256) PB_ROWS_TC(5, 8);

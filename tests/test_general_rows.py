@@ -100,6 +100,29 @@ def test_few_rows_on_the_tensor_cores(q_lens, kv_lens, hq, hkv, dk, dv, opts):
     assert float((got[torch.bfloat16].double() - want).abs().max() / want.abs().max()) < 2.0 ** -8
 
 
+@pytest.mark.parametrize("q_lens,kv_lens,hq,hkv,dk,dv", [([1, 1], [1900, 70], 16, 1, 576, 512), ([1, 3], [500, 64], 8, 4, 64, 64)])
+def test_partial_results_at_any_float(q_lens, kv_lens, hq, hkv, dk, dv):
+    """Scratch that begins at an odd float (a view of a caller's own buffer)."""
+    from pulsar_b200 import ops
+    gen = torch.Generator().manual_seed(dk)
+    table, pools = _paged(q_lens, kv_lens, 16, [(hkv, dk)] if dk == 576 else [(hkv, dk), (hkv, dv)], torch.bfloat16, gen)
+    q, n = torch.randn(sum(q_lens), hq, dk, generator=gen).cuda(), sum(q_lens)
+
+    class Shifted(_Ctx):
+        def scratch(self, tag, shape, dtype):
+            assert tag == "attn.general.partial"
+            self.asked = torch.full((shape[0] + 1,), float("nan"), dtype=dtype, device="cuda")
+            return self.asked[1:]
+
+    got = []
+    for ctx in (_Ctx(q_lens, kv_lens), Shifted(q_lens, kv_lens)):
+        out = torch.full((n, hq, dv), float("nan"), device="cuda")
+        ops.paged_attention_general(ctx, q, pools[0], pools[-1], out, table.cuda(), dk ** -0.5, value_width=dv, tensor_cores=False)
+        got.append(out)
+    assert bool(torch.isfinite(ctx.asked[1:3]).all())
+    assert float((got[0] - got[1]).norm() / got[0].norm()) < 3e-6         # the two forms, each 1.5e-6 from float64
+
+
 # 16 tokens and fewer: one and two token tiles, outputs around a block's 64, odd counts, k around the slices and behind their end
 @pytest.mark.parametrize("n,heads,k,m", [(1, 2, 1, 1), (8, 3, 16, 64), (9, 2, 17, 65), (16, 5, 100, 66), (3, 2, 512, 128), (5, 2, 1024, 63)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
