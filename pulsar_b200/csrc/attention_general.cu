@@ -557,9 +557,15 @@ __global__ void general_combine_kernel(const float* __restrict__ partial, T* __r
 constexpr int kSRow = kTile + 4;        // floats of a row of partial scores
 
 // x as a sum of three bfloat16 pairs: element pairs packed as mma wants them.  An infinite number is its own first part and
-// has nothing left.
+// has nothing left.  kLarge: x may be a finite number above bfloat16's largest, which would round to infinity (queries; softmax
+// weights are at most one).
+__device__ __forceinline__ float to_bf16_range(float x) {
+    constexpr float most = 3.3895313892515355e38f;          // bfloat16's largest
+    return fabsf(x) == INFINITY ? x : fminf(fmaxf(x, -most), most);
+}
+template <bool kLarge>
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    hi = pack_bf16(x, y);
+    hi = kLarge ? pack_bf16(to_bf16_range(x), to_bf16_range(y)) : pack_bf16(x, y);
     x = fabsf(x) == INFINITY ? 0.0f : x - __uint_as_float(hi << 16);
     y = fabsf(y) == INFINITY ? 0.0f : y - __uint_as_float(hi & 0xffff0000u);
     mid = pack_bf16(x, y);
@@ -658,7 +664,7 @@ general_rows_tc_kernel(const float* __restrict__ q, const bf16* __restrict__ k_p
             const int r = f & 1, col = ks * 16 + (f >> 1) * 8 + (lane & 3) * 2;
             float2 v = make_float2(0.0f, 0.0f);
             if (ks < steps && pos[r] >= 0) v = *reinterpret_cast<const float2*>(q + ((size_t)tok[r] * sh.Hq + head[r]) * Dk + col);
-            split3(v.x, v.y, qf[0][i][f], qf[1][i][f], qf[2][i][f]);
+            split3<true>(v.x, v.y, qf[0][i][f], qf[1][i][f], qf[2][i][f]);
         }
     }
 
@@ -779,7 +785,7 @@ general_rows_tc_kernel(const float* __restrict__ q, const bf16* __restrict__ k_p
 #pragma unroll
             for (int f = 0; f < 4; ++f) {
                 const int n = 2 * k2 + (f >> 1), r = f & 1;
-                split3(pw[n][2 * r], pw[n][2 * r + 1], pf[k2][0][f], pf[k2][1][f], pf[k2][2][f]);
+                split3<false>(pw[n][2 * r], pw[n][2 * r + 1], pf[k2][0][f], pf[k2][1][f], pf[k2][2][f]);
             }
 #pragma unroll
         for (int i = 0; i < VT; i += 2) {

@@ -100,6 +100,32 @@ def test_few_rows_on_the_tensor_cores(q_lens, kv_lens, hq, hkv, dk, dv, opts):
     assert float((got[torch.bfloat16].double() - want).abs().max() / want.abs().max()) < 2.0 ** -8
 
 
+# queries at the ends of float32: infinite ones (with sigmoid weights, which are then zero or one), and finite ones that round to an
+# infinite bfloat16 and meet keys as small
+@pytest.mark.parametrize("large,sigmoid", [(math.inf, True), (torch.finfo(torch.float32).max, True), (torch.finfo(torch.float32).max, False),
+                                           (3.39e38, False), (-3.4e38, False)])
+def test_queries_at_the_ends_of_float32(large, sigmoid):
+    from pulsar_b200 import ops
+    q_lens, kv_lens, hq, hkv, d, page = [1, 2], [70, 33], 4, 2, 64, 16
+    gen = torch.Generator().manual_seed(3)
+    table, (k_pool, v_pool) = _paged(q_lens, kv_lens, page, [(hkv, d)] * 2, torch.bfloat16, gen)
+    q = torch.randn(3, hq, d, generator=gen).cuda() * 0.1
+    q[:, :, 5] = large
+    k_pool[..., 5] = torch.where(k_pool[..., 5] > 0, 1.0, -1.0) * (1.0 if math.isinf(large) else 2.0 ** -125)       # products of about 8
+    ctx, got, want = _Ctx(q_lens, kv_lens), torch.empty(3, hq, d, device="cuda"), torch.empty(3, hq, d, dtype=torch.float64, device="cuda")
+    ops.paged_attention_general(ctx, q, k_pool, v_pool, got, table.cuda(), 1.0, tensor_cores=False, sigmoid=sigmoid)
+    at = 0
+    for s, (m, kl) in enumerate(zip(q_lens, kv_lens)):
+        k, v = (_keys_of(p, table, s, kl, page).repeat_interleave(2, dim=1) for p in (k_pool, v_pool))
+        hidden = torch.arange(kl, device="cuda")[None] > torch.arange(kl - m, kl, device="cuda")[:, None]
+        sc = torch.einsum("ihd,jhd->hij", q[at:at + m].double(), k)
+        w = torch.sigmoid(sc) * ~hidden if sigmoid else torch.softmax(sc.masked_fill(hidden, -math.inf), dim=-1)
+        want[at:at + m] = torch.einsum("hij,jhv->ihv", w, v)
+        at += m
+    assert bool(torch.isfinite(got).all())
+    assert float((got.double() - want).norm() / want.norm()) < 1e-5       # scores near 9, known to 2^-21 of that: the weights to 5e-6
+
+
 @pytest.mark.parametrize("q_lens,kv_lens,hq,hkv,dk,dv", [([1, 1], [1900, 70], 16, 1, 576, 512), ([1, 3], [500, 64], 8, 4, 64, 64)])
 def test_partial_results_at_any_float(q_lens, kv_lens, hq, hkv, dk, dv):
     """Scratch that begins at an odd float (a view of a caller's own buffer)."""
