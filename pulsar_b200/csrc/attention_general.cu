@@ -488,9 +488,12 @@ general_tiled_kernel(const float* __restrict__ q, const T* __restrict__ k_pool, 
 // out[row] = sum over the splits, in their order, of their partial outputs weighted by exp(m_split - m_all), over the
 // weighted sum of their sums.  One block per (token, head).
 // (With `sigmoid` the partial outputs are added as they are; a row's columns turn back where the launch says so.)
-// Every warp takes the weights of 32 splits side by side, a lane one; a thread's columns of those splits are asked for before the
-// weights are known, so that one trip to L2 brings all of it.
-template <typename T>
+// Every warp takes the weights of up to 32 splits side by side, a lane one; a thread's columns of those splits are asked for before the
+// weights are known, so that one trip to L2 brings all of it.  kSplits (4, 8, 16, 32): the splits a round takes, kCols: the columns a
+// thread takes; both no larger than the launch needs, since every round runs through all its places (us with the attention itself, a loop
+// over the splits, rounds of 32 with two columns always, now: 128 sequences at 300 keys, 16 heads on one of 32 / 64, 4 splits 29.4,
+// 31.3, 27.1; 8 at 500, 128 / 128, 8 splits 24.8, 14.3, 13.4; 32 at 1,000, 16 on one of 576 / 512, 16 splits 111, 43.1, 40.9).
+template <typename T, int kSplits, int kCols>
 __global__ void general_combine_kernel(const float* __restrict__ partial, T* __restrict__ out, const float* __restrict__ sinks,
                                        int n_splits, const GeneralShape sh) {
     pdl_trigger();
@@ -499,41 +502,43 @@ __global__ void general_combine_kernel(const float* __restrict__ partial, T* __r
     const int Hq = sh.Hq, Dv = sh.Dv, lane = threadIdx.x & 31;
     const float* pp = partial + row * n_splits * (Dv + 2);
     float m_all = -INFINITY, l_all = 0.0f;
-    if (!sh.sigmoid && n_splits > 32) {
+    if (!sh.sigmoid && n_splits > kSplits) {
         for (int z = lane; z < n_splits; z += 32) m_all = fmaxf(m_all, pp[(size_t)z * (Dv + 2)]);
         m_all = warp_max(m_all);
     }
-    float o[2] = {0.0f, 0.0f};                               // this thread's columns (at most 512 in blocks of 256)
-    for (int z0 = 0; z0 < n_splits; z0 += 32) {
-        const int nz = min(32, n_splits - z0);
-        float v[2][32];
+    float o[kCols];                                          // this thread's columns
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kCols; ++i) o[i] = 0.0f;
+    for (int z0 = 0; z0 < n_splits; z0 += kSplits) {
+        const int nz = min(kSplits, n_splits - z0);
+        float v[kCols][kSplits];
+#pragma unroll
+        for (int i = 0; i < kCols; ++i) {
             const int c = threadIdx.x + i * blockDim.x;
 #pragma unroll
-            for (int z = 0; z < 32; ++z) v[i][z] = (z < nz && c < Dv) ? pp[(size_t)(z0 + z) * (Dv + 2) + 2 + c] : 0.0f;
+            for (int z = 0; z < kSplits; ++z) v[i][z] = (z < nz && c < Dv) ? pp[(size_t)(z0 + z) * (Dv + 2) + 2 + c] : 0.0f;
         }
         float w = lane < nz ? 1.0f : 0.0f;
         if (!sh.sigmoid) {                                   // uniform over the grid
             const float* mine = pp + (size_t)(z0 + min(lane, nz - 1)) * (Dv + 2);
             const float m = lane < nz ? mine[0] : -INFINITY, l = mine[1];
-            if (n_splits <= 32) m_all = warp_max(m);
+            if (n_splits <= kSplits) m_all = warp_max(m);
             w = m != -INFINITY ? expf(m - m_all) : 0.0f;
             l_all += warp_sum(w != 0.0f ? l * w : 0.0f);
         }
 #pragma unroll
-        for (int z = 0; z < 32; ++z) {
+        for (int z = 0; z < kSplits; ++z) {
             const float wz = __shfl_sync(0xffffffffu, w, z);
             if (wz != 0.0f) {                                // uniform over the warp
-                o[0] = fmaf(v[0][z], wz, o[0]);
-                o[1] = fmaf(v[1][z], wz, o[1]);
+#pragma unroll
+                for (int i = 0; i < kCols; ++i) o[i] = fmaf(v[i][z], wz, o[i]);
             }
         }
     }
     if (sh.sigmoid) l_all = 1.0f;
     else if (sinks) l_all += expf(sinks[row % Hq] - m_all);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kCols; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
         float v = o[i] / l_all;
         if (sh.out_cos) {                                    // uniform over the grid; the pair's other column is the neighbouring lane's
@@ -938,7 +943,12 @@ template <typename T>
 int launch_combine(const float* partial, void* out, const float* sinks, int n_tokens, const TiledShape& ts, cudaStream_t stream) {
     int b = 32;
     while (b < ts.g.Dv && b < 256) b <<= 1;
-    return launch_pdl(general_combine_kernel<T>, dim3(n_tokens * ts.g.Hq), dim3(b), 0, stream, partial, (T*)out, sinks, ts.n_splits, ts.g);
+#define PB_COMBINE(S, C) return launch_pdl(general_combine_kernel<T, S, C>, dim3(n_tokens * ts.g.Hq), dim3(b), 0, stream, partial, (T*)out, sinks, ts.n_splits, ts.g)
+#define PB_COMBINE_COLS(C) { if (ts.n_splits <= 4) PB_COMBINE(4, C); if (ts.n_splits <= 8) PB_COMBINE(8, C); if (ts.n_splits <= 16) PB_COMBINE(16, C); PB_COMBINE(32, C); }
+    if (ts.g.Dv <= b) PB_COMBINE_COLS(1)
+    PB_COMBINE_COLS(2)                                      // widths up to 512 in blocks of 256
+#undef PB_COMBINE_COLS
+#undef PB_COMBINE
 }
 
 // One warp per (token, head) of the fused projection row [q: Hq*Dk | k: Hk*Dk | v: Hv*Dv]:

@@ -201,3 +201,26 @@ def test_add_rmsnorm_does_not_depend_on_the_number_of_rows(width, dtype):
         cut, part = residual[first:first + rows].clone(), torch.empty(rows, width, dtype=dtype, device="cuda")
         ops.add_rmsnorm(cut, delta[first:first + rows].clone(), weight, 1e-6, part)
         assert torch.equal(part, whole[first:first + rows]) and torch.equal(cut, stream[first:first + rows])
+
+
+# the merge of a row's splits: every round length at its edges and more than one round of 32, one and two columns a thread; most of
+# many splits hold no key
+@pytest.mark.parametrize("splits", [2, 4, 5, 8, 9, 16, 17, 32, 33, 64, 70])
+@pytest.mark.parametrize("hq,hkv,dk,dv,opts", [(4, 4, 16, 16, {}), (8, 1, 576, 512, dict(sinks=True)), (6, 2, 320, 256, dict(sigmoid=True, turn=True)),
+                                               (2, 1, 64, 272, dict(turn=True))])
+def test_merge_of_splits(splits, hq, hkv, dk, dv, opts, monkeypatch):
+    from pulsar_b200 import ops
+    q_lens, kv_lens, gen = [1, 3], [530, 40], torch.Generator().manual_seed(splits + dv)
+    table, pools = _paged(q_lens, kv_lens, 16, [(hkv, dk), (hkv, dv)], torch.bfloat16, gen)
+    q, n = torch.randn(4, hq, dk, generator=gen).cuda(), 4
+    sinks = torch.randn(hq, generator=gen).cuda() if opts.get("sinks") else None
+    angle = torch.rand(n, dv // 2, generator=gen).cuda()
+    options = dict(value_width=dv, tensor_cores=False, sinks=sinks, sigmoid=bool(opts.get("sigmoid")),
+                   turn_back=(angle.cos(), angle.sin()) if opts.get("turn") else None)
+    got = []
+    for k in (1, splits):
+        monkeypatch.setattr(ops, "general_splits", lambda blocks, tokens: k)
+        out = torch.full((n, hq, dv), float("nan"), device="cuda")
+        ops.paged_attention_general(_Ctx(q_lens, kv_lens), q, pools[0], pools[1], out, table.cuda(), dk ** -0.5, **options)
+        got.append(out.double())
+    assert float((got[0] - got[1]).norm() / got[0].norm()) < 3e-6         # the same sums in another grouping, each 1.5e-6 from float64
