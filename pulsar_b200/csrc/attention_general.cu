@@ -921,6 +921,9 @@ int dispatch_tiled(const float* q, const void* k_pool, const void* v_pool, void*
 // cores, 8 sequences at 1,900 keys: 16 heads on one row of 576 / 512, 32 splits 60.5 -> 22.7; 16 on 4 heads of 128 / 128, chunks of
 // 1,024, 16 splits 26.7 -> 15.1; the smallest (2 sequences, 8 heads on 4 of 64 / 64, 90 and 333 keys) 7.6 -> 8.2.  Relative error of
 // float32 rows against 64 bits on the first: 5.7e-7 -> 2.0e-7.
+// Keys of 32 and fewer with fewer than four heads to a key/value head stay on the CUDA cores: so few sums a tile do not pay for the
+// tensor-core form's larger blocks once these fill the SMs (4 heads of 32 / 32, 32 sequences at 1,000 keys 32.7 against 34.7, 128 at 300
+// 42.1 against 47.1; one at 1,000 9.9 against 10.9).  With four heads or more, and from keys of 48 on, it is level or ahead.
 int dispatch_tiled_bf16(const float* q, const void* k_pool, const void* v_pool, void* out, float* partial, const int* block_table,
                         const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int row_tiles, TiledShape ts,
                         cudaStream_t stream) {
@@ -928,7 +931,8 @@ int dispatch_tiled_bf16(const float* q, const void* k_pool, const void* v_pool, 
     if (!ts.v_in_k) ts.v_row = (ts.g.Dv / 8 | 1) * 8;       // value rows an odd number of 16-byte units apart as well
     const size_t smem = rows_tc_smem(ts);
 #define PB_ROWS_TC(K, V) return launch_rows_tc<K, V>(q, k_pool, v_pool, out, partial, block_table, cu_q, kv_len, slopes, sinks, row_tiles, ts, smem, stream)
-    if (smem > 0 && smem <= 200 * 1024 && (uintptr_t)partial % 8 == 0) {                 // partial results are written two floats at a time
+    const bool thin = ts.g.Dk <= 32 && ts.g.Hq / ts.g.Hkv < 4;
+    if (smem > 0 && smem <= 200 * 1024 && !thin && (uintptr_t)partial % 8 == 0) {        // partial results are written two floats at a time
         if (ts.g.Dk <= 128 && ts.g.Dv <= 128) PB_ROWS_TC(2, 4);
         if (ts.g.Dk <= 192 && ts.g.Dv <= 128) PB_ROWS_TC(3, 4);
         if (ts.g.Dk <= 320 && ts.g.Dv <= 256) PB_ROWS_TC(5, 8);

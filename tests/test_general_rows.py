@@ -43,7 +43,8 @@ class _Ctx:
     ([1] * 3, [100, 1024, 1025], 16, 4, 128, 128, dict(slopes=True, chunk=64)), ([1, 7], [90, 333], 8, 1, 80, 48, dict(sinks=True)),
     ([1, 5, 2], [64, 37, 300], 12, 4, 64, 64, dict(window=50, keep_first=4, softcap=20.0, sinks=True)),
     ([2, 1], [90, 33], 8, 2, 64, 128, dict(sigmoid=True, turn=True)), ([1, 1], [90, 2333], 8, 4, 64, 64, dict(sigmoid=True, v_share=2)),
-    ([1], [1], 2, 1, 16, 16, {})])
+    ([1], [1], 2, 1, 16, 16, {}), ([1, 2], [300, 40], 4, 1, 32, 32, {}), ([1, 2], [300, 40], 3, 1, 32, 32, {}),
+    ([2, 1], [70, 500], 8, 1, 16, 48, dict(sinks=True))])
 def test_few_rows_on_the_tensor_cores(q_lens, kv_lens, hq, hkv, dk, dv, opts):
     from pulsar_b200 import ops
     gen = torch.Generator().manual_seed(dk + hq)
