@@ -401,12 +401,8 @@ int launch_tc(const void* q, const void* k_pool, const void* v_pool, float* part
     constexpr int pipeline = kStages * 2 * kTile * D * 2;
     constexpr int merge = (kWarps * 16 * D + 2 * kWarps * 16) * 4;
     constexpr int smem = pipeline > merge ? pipeline : merge;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t rc = cudaFuncSetAttribute(decode_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (rc != cudaSuccess) return (int)rc;
-        configured = true;
-    }
+    static SmemLimit limit;
+    if (const int rc = limit.allow(decode_tc_kernel<D>, smem)) return rc;
     // With fewer blocks than SMs (a lone sequence) the two tiles a block has in flight are not enough to hide the
     // memory's latency: such a launch also asks L2 for the two tiles behind them (2.828 against 2.858 ms per step of one
     // sequence).  With more blocks that costs time (3.626 against 3.538 ms at 8 sequences, 10.31 against 9.49 at 64).

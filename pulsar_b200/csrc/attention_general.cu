@@ -863,8 +863,8 @@ template <int KS, int VT>
 int launch_rows_tc(const float* q, const void* k_pool, const void* v_pool, void* out, float* partial, const int* block_table,
                    const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int row_tiles, const TiledShape& ts,
                    size_t smem, cudaStream_t stream) {
-    static const cudaError_t allowed = cudaFuncSetAttribute(general_rows_tc_kernel<KS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (allowed != cudaSuccess) return (int)allowed;
+    static SmemLimit limit;
+    if (const int rc = limit.allow(general_rows_tc_kernel<KS, VT>, 200 * 1024)) return rc;
     return launch_pdl(general_rows_tc_kernel<KS, VT>, dim3(row_tiles, ts.g.Hkv, ts.n_splits), dim3(128), smem, stream, q, (const bf16*)k_pool,
                       (const bf16*)v_pool, (bf16*)out, partial, block_table, cu_q, kv_len, slopes, sinks, ts, pb::pool_bounds_now());
 }
@@ -879,12 +879,8 @@ int launch_tiled(const float* q, const void* k_pool, const void* v_pool, void* o
                  const int* cu_q, const int* kv_len, const float* slopes, const float* sinks, int row_tiles, const TiledShape& ts,
                  cudaStream_t stream) {
     const size_t smem = tiled_smem<T>(ts);
-    static size_t allowed = 48 * 1024;                     // per instantiation
-    if (smem > allowed) {
-        const cudaError_t e = cudaFuncSetAttribute(general_tiled_kernel<T, ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        allowed = smem;
-    }
+    static SmemLimit limit;
+    if (const int rc = limit.allow(general_tiled_kernel<T, ACC>, smem)) return rc;
     dim3 grid(row_tiles, ts.g.Hkv, ts.n_splits);
     return launch_pdl(general_tiled_kernel<T, ACC>, grid, dim3(128), smem, stream, q, (const T*)k_pool, (const T*)v_pool, (T*)out, partial,
                       block_table, cu_q, kv_len, slopes, sinks, ts, pb::pool_bounds_now());

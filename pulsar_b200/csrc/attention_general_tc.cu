@@ -346,12 +346,8 @@ int launch_general_tc(const float* q, const void* k_pool, const void* v_pool, vo
                       cudaStream_t stream) {
     static_assert(DV <= 2 * DK && DK % 16 == 0 && DV % 32 == 0 && DK >= 64 && DV >= 64, "tile shapes");
     constexpr int smem = 2 * kBM * DK * 2 + 2 * kBN * (DK + DV) * 2;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t rc = cudaFuncSetAttribute(general_tc_kernel<DK, DV, kSigmoid>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (rc != cudaSuccess) return (int)rc;
-        configured = true;
-    }
+    static SmemLimit limit;
+    if (const int rc = limit.allow(general_tc_kernel<DK, DV, kSigmoid>, smem)) return rc;
     const long long blocks = (long long)n_q_tiles * sh.Hq;
     if (blocks >= (1LL << 31)) return PB_ERR_TOO_LARGE;
     const dim3 grid((unsigned)blocks);

@@ -254,10 +254,8 @@ int launch_rows(const void* q, const void* k_pool, const void* v_pool, void* out
                 float scale, int window, cudaStream_t stream) {
     const int G = Hq / Hkv, GP = G < ROWS ? G : ROWS, TQ = ROWS / GP;
     const size_t smem = sizeof(float) * ((size_t)ROWS * D + kWarps * ROWS * 32 + 2 * kWarps * ROWS + 2 * ROWS + (size_t)kWarps * ROWS * D);
-    constexpr size_t most = sizeof(float) * (ROWS * 32 * ACC + kWarps * ROWS * 32 + 2 * kWarps * ROWS + 2 * ROWS + kWarps * ROWS * 32 * ACC);
-    static const cudaError_t allowed =
-        cudaFuncSetAttribute(paged_attention_generic_kernel<T, ROWS, ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    if (allowed != cudaSuccess) return (int)allowed;
+    static SmemLimit limit;
+    if (const int rc = limit.allow(paged_attention_generic_kernel<T, ROWS, ACC>, smem)) return rc;
     dim3 grid((n_tokens + TQ - 1) / TQ * TQ, Hkv, (G + GP - 1) / GP);
     if (grid.y > 65535 || grid.z > 65535) return PB_ERR_TOO_LARGE;
     paged_attention_generic_kernel<T, ROWS, ACC><<<grid, kWarps * 32, smem, stream>>>((const T*)q, (const T*)k_pool,

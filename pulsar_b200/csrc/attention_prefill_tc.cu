@@ -246,12 +246,8 @@ int launch_prefill(const void* q, const void* k_pool, const void* v_pool, void* 
                    int page_size, float scale, int window, cudaStream_t stream) {
     constexpr int smem = 2 * 2 * kBN * D * 2;
     const int page_shift = log2_exact(page_size);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t rc = cudaFuncSetAttribute(prefill_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (rc != cudaSuccess) return (int)rc;
-        configured = true;
-    }
+    static SmemLimit limit;
+    if (const int rc = limit.allow(prefill_tc_kernel<D>, smem)) return rc;
     dim3 grid(n_q_tiles, Hq);
     prefill_tc_kernel<D><<<grid, kWarps * 32, smem, stream>>>((const bf16*)q, (const bf16*)k_pool, (const bf16*)v_pool,
                                                               (bf16*)out, block_table, table_stride, cu_q, kv_len, n_seqs,

@@ -480,12 +480,8 @@ PB_EXPORT int pb_paged_attention_prefill_tcgen05(int dtype, const void* q, const
     if (rc != 0) return rc;
     rc = make_map(&mv, v_pool, pool_rows, D, rows_per_load);
     if (rc != 0) return rc;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static SmemLimit limit;
+    if ((rc = limit.allow(prefill_tcgen05_kernel, kSmemBytes)) != 0) return rc;
     Args a;
     a.out = (bf16*)out;
     a.block_table = block_table;

@@ -546,12 +546,8 @@ int launch_dual(const void* q, const void* k_pool, const void* v_pool, void* out
     if (rc != 0) return rc;
     rc = make_map(&mv, v_pool, pool_rows, kD, rows_per_load);
     if (rc != 0) return rc;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_tcgen05_dual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static SmemLimit limit;
+    if ((rc = limit.allow(prefill_tcgen05_dual_kernel, kSmemBytes)) != 0) return rc;
     Args a;
     a.out = (bf16*)out;
     a.block_table = block_table;

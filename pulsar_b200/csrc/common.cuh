@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "device_limit.h"
+
 #define PB_EXPORT extern "C" __attribute__((visibility("default")))
 
 // Refusals (returned instead of a wrong result).
@@ -169,5 +171,16 @@ template <typename... KArgs, typename... Args>
 inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     return launch_early(true, kernel, grid, block, smem, stream, args...);
 }
+
+// `static SmemLimit limit;` beside a launch, one per kernel: limit.allow(kernel, bytes) lets the current device's copy of it
+// take so much dynamic shared memory, and no less than every kernel may (a host call, allowed under capture; nothing once it has been done).
+struct SmemLimit : DeviceLimit {
+    template <typename... KArgs>
+    int allow(void (*kernel)(KArgs...), size_t bytes) {
+        return DeviceLimit::allow(bytes > 48 * 1024 ? bytes : 48 * 1024, [](int* dev) { return (int)cudaGetDevice(dev); }, [&](size_t n) {
+            return (int)cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+        });
+    }
+};
 
 }  // namespace pb

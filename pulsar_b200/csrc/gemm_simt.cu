@@ -156,9 +156,8 @@ template <int R, int T, int CW, int RST, typename TO>
 int launch_rows_st(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
     constexpr int MR = 32 / (RN / R) * T * CW;
     constexpr size_t smem = sizeof(float) * RST * (RN * RSTRIDE + MR * RK);
-    static const cudaError_t allowed =
-        cudaFuncSetAttribute(simt_rows_kernel<R, T, CW, RST, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (allowed != cudaSuccess) return (int)allowed;
+    static SmemLimit limit;
+    if (const int rc = limit.allow(simt_rows_kernel<R, T, CW, RST, TO>, smem)) return rc;
     return launch_early(loaded, simt_rows_kernel<R, T, CW, RST, TO>, dim3((N + RN - 1) / RN), dim3(RLOAD + 32 * CW), smem, stream, A, W, out, M, N, K);
 }
 

@@ -607,20 +607,12 @@ int sm_count() {
 template <int MODE, typename OutT>
 int launch(const CUtensorMap& mx, const CUtensorMap& mw, void* out, int M, int N, int K, const GatedInter inter, int m_tiles, int n_tiles,
            cudaStream_t stream) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t rc = cudaFuncSetAttribute(gemm_tcgen05_kernel<MODE, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        if (rc != cudaSuccess) return (int)rc;
-        configured = true;
-    }
+    static SmemLimit limit;
+    if (const int rc = limit.allow(gemm_tcgen05_kernel<MODE, OutT>, kSmemBytes)) return rc;
     if (M > kBM && pair_enabled()) {
         // more than one tile of tokens: pairs of blocks on tiles of 256 tokens
-        static bool pair_configured = false;
-        if (!pair_configured) {
-            cudaError_t rc = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<MODE, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
-            if (rc != cudaSuccess) return (int)rc;
-            pair_configured = true;
-        }
+        static SmemLimit pair_limit;
+        if (const int rc = pair_limit.allow(gemm_tcgen05_pair_kernel<MODE, OutT>, kPairSmemBytes)) return rc;
         const int pm_tiles = (M + 2 * kBM - 1) / (2 * kBM);
         const long long ptiles = (long long)pm_tiles * n_tiles;
         const int pairs = (int)(ptiles < sm_count() / 2 ? ptiles : sm_count() / 2);
@@ -744,12 +736,8 @@ PB_EXPORT int pb_gemm_tcgen05_grouped(int mode, int out_dtype, const void* x, co
     if (rc != 0) return rc;
 #define PB_GROUPED(MODE, OutT, INTER, NT)                                                                                         \
     {                                                                                                                             \
-        static bool configured = false;                                                                                           \
-        if (!configured) {                                                                                                        \
-            cudaError_t ce = cudaFuncSetAttribute(gemm_tcgen05_grouped_kernel<MODE, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes); \
-            if (ce != cudaSuccess) return (int)ce;                                                                                \
-            configured = true;                                                                                                    \
-        }                                                                                                                         \
+        static SmemLimit limit;                                                                                                   \
+        if (const int e = limit.allow(gemm_tcgen05_grouped_kernel<MODE, OutT>, kSmemBytes)) return e;                             \
         const long long tiles = (long long)max_row_tiles * (NT);                                                                  \
         const int grid = (int)(tiles < sm_count() ? tiles : sm_count());                                                          \
         gemm_tcgen05_grouped_kernel<MODE, OutT><<<grid, kThreads, kSmemBytes, stream>>>(mx, mw, (OutT*)out, N, K, INTER, NT, N,  \

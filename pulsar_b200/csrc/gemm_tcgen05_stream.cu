@@ -432,12 +432,8 @@ int launch(const CUtensorMap& mx, const CUtensorMap& mw, void* out, StreamArgs a
     a.up_offset = stages * stage_bytes;
     a.bar_offset = (a.up_offset + up_bytes + 15) / 16 * 16;
     const int smem_bytes = a.bar_offset + 256 + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t rc = cudaFuncSetAttribute(gemm_tcgen05_stream_kernel<MODE, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (rc != cudaSuccess) return (int)rc;
-        configured = true;
-    }
+    static SmemLimit limit;
+    if (const int rc = limit.allow(gemm_tcgen05_stream_kernel<MODE, OutT>, 227 * 1024)) return rc;
     const long long units = (long long)a.n_tiles * slices;
     const int grid = (int)(units < sm_count() ? units : sm_count());
     return launch_pdl(gemm_tcgen05_stream_kernel<MODE, OutT>, grid, kThreads, smem_bytes, stream, mx, mw, (OutT*)out, a);

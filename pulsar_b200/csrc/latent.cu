@@ -405,12 +405,7 @@ int launch_heads(const void* a, long a_tok, int a_head, const void* w, void* out
         return launch_status();
     }
     const int ks = heads_slice(K);
-    const size_t smem = sizeof(float) * kTok * (ks * kSlices + kSlices * kOuts);
-    static const cudaError_t allowed = [] {
-        const cudaError_t e = cudaFuncSetAttribute(heads_linear_kernel<T, TO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        return e != cudaSuccess ? e : cudaFuncSetAttribute(heads_linear_kernel<T, TO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    }();
-    if (allowed != cudaSuccess) return (int)allowed;
+    const size_t smem = sizeof(float) * kTok * (ks * kSlices + kSlices * kOuts);        // 48 KB with the widest K, 1,024: what every kernel may have
     dim3 grid((N + kTok - 1) / kTok, H, (M + kOuts - 1) / kOuts);
     const auto kernel = heads_pairs(w, M, sizeof(T)) ? heads_linear_kernel<T, TO, true> : heads_linear_kernel<T, TO, false>;
     return launch_pdl(kernel, grid, dim3(32 * kSlices), smem, stream, (const T*)a, a_tok, a_head, (const T*)w, (TO*)out, o_tok, o_head,

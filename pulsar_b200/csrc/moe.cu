@@ -333,12 +333,8 @@ int launch_route(const void* h, const float* router, int* ids, float* weights, i
                  int renormalize, int n_extra, float* extra, int softmax, float renorm_eps, const RouteChoice& choice, cudaStream_t stream) {
     const size_t smem = sizeof(float) * TOK * ((size_t)width + 2 * n_experts + n_extra + choice.n_groups);
     if (smem > 200 * 1024) return PB_ERR_TOO_LARGE;
-    static size_t allowed = 48 * 1024;
-    if (smem > allowed) {
-        const cudaError_t ce = cudaFuncSetAttribute(moe_route_kernel<T, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (ce != cudaSuccess) return (int)ce;
-        allowed = smem;
-    }
+    static SmemLimit limit;
+    if (const int rc = limit.allow(moe_route_kernel<T, TOK>, smem)) return rc;
     int warps = (n_experts + n_extra + kRouteRows - 1) / kRouteRows;      // a warp per group of rows where that fits a block
     if (warps > 16) warps = 16;
     if (warps < TOK) warps = TOK;                                         // warp k picks for token k
@@ -430,15 +426,9 @@ PB_EXPORT int pb_moe_down(int dtype, const void* act, const void* w_down, const 
     const size_t smem = sizeof(float) * (size_t)top * ff;
     if (smem > 200 * 1024) return PB_ERR_TOO_LARGE;
     if (dtype != PB_F32 && dtype != PB_BF16) return PB_ERR_BAD_DTYPE;
-    static size_t allowed[2] = {48 * 1024, 48 * 1024};
-    size_t& mine = allowed[dtype == PB_BF16];
-    if (smem > mine) {
-        const cudaError_t ce = dtype == PB_F32
-            ? cudaFuncSetAttribute(moe_down_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-            : cudaFuncSetAttribute(moe_down_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (ce != cudaSuccess) return (int)ce;
-        mine = smem;
-    }
+    static SmemLimit limit32, limit16;
+    const int rc = dtype == PB_F32 ? limit32.allow(moe_down_kernel<float>, smem) : limit16.allow(moe_down_kernel<__nv_bfloat16>, smem);
+    if (rc != 0) return rc;
     const int warps = 8;
     int by = (width + warps - 1) / warps;
     if (by > 64) by = 64;

@@ -296,14 +296,10 @@ PB_EXPORT int pb_moe_grouped(const void* h, const void* w_gate_up, const void* w
     }
     const GatedInter gating(ff, limit > 0.0f ? limit : __builtin_huge_valf(), alpha, shift);
     constexpr int smem0 = kStages * (kBM + 2 * kBN) * kRow * 2, smem1 = kStages * (kBM + kBN) * kRow * 2;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t ce = cudaFuncSetAttribute(moe_grouped_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem0);
-        if (ce == cudaSuccess) ce = cudaFuncSetAttribute(moe_grouped_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
-        if (ce == cudaSuccess) ce = cudaFuncSetAttribute(moe_grouped_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
-        if (ce != cudaSuccess) return (int)ce;
-        configured = true;
-    }
+    static SmemLimit limit0, limit1, limit2;
+    if (const int e = limit0.allow(moe_grouped_kernel<0>, smem0)) return e;
+    if (const int e = limit1.allow(moe_grouped_kernel<1>, smem1)) return e;
+    if (const int e = limit2.allow(moe_grouped_kernel<2>, smem1)) return e;
     if (ungated)
         rc = launch_pdl(moe_grouped_kernel<2>, dim3(tiles, (ff + kBN - 1) / kBN), dim3(kThreads), smem1, stream, (const bf16*)h, (const bf16*)w_gate_up,
                         (const int*)offsets, (const int*)sorted, (const int*)tile_expert, (const int*)tile_row0, (const int*)meta, (bf16*)act,

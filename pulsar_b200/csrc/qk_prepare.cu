@@ -247,12 +247,8 @@ int launch_whole(const void* rows, long row_stride, const float* q_norm_w, const
     }
     const size_t smem = sizeof(float) * (size_t)widest;
     if (smem > 200 * 1024) return PB_ERR_TOO_LARGE;
-    static size_t allowed = 48 * 1024;                     // per instantiation
-    if (smem > allowed) {
-        const cudaError_t e = cudaFuncSetAttribute(qk_prepare_whole_kernel<TIn, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        allowed = smem;
-    }
+    static SmemLimit limit;
+    if (const int rc = limit.allow(qk_prepare_whole_kernel<TIn, T>, smem)) return rc;
     int threads = 64;
     while (threads < 512 && threads * 8 < widest) threads <<= 1;
     return launch_pdl(qk_prepare_whole_kernel<TIn, T>, dim3(n, sh.Hkv > 0 ? 3 : 1), dim3(threads), smem, stream, (const TIn*)rows,

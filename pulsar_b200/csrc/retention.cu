@@ -345,7 +345,7 @@ template <typename K>
 int allow_smem(K kernel, size_t smem) {
     if (smem <= 48 * 1024) return 0;
     if (smem > 200 * 1024) return PB_ERR_TOO_LARGE;
-    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       // on every launch: the current device's
 }
 
 template <typename T, int PER, int THREADS>

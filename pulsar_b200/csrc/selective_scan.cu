@@ -541,12 +541,8 @@ int launch_scan_chunked(const void* x, const void* xz, const void* bc, long bc_t
     const bool vec = sh.inner % kChunkChannels == 0 && (2 * sh.n_state) % V == 0 && bc_tok % V == 0 && sh.xz_tok % V == 0 &&
                      (((uintptr_t)x | (uintptr_t)xz | (uintptr_t)bc | (uintptr_t)dt_pre | (uintptr_t)y) & 15) == 0;
     const auto kernel = vec ? selective_scan_chunked_kernel<T, true> : selective_scan_chunked_kernel<T, false>;
-    static size_t allowed[2] = {48 * 1024, 48 * 1024};
-    if (smem > allowed[vec]) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        allowed[vec] = smem;
-    }
+    static SmemLimit limits[2];
+    if (const int rc = limits[vec].allow(kernel, smem)) return rc;
     dim3 grid(n_seqs, (sh.inner + kChunkChannels - 1) / kChunkChannels);
     kernel<<<grid, 256, smem, stream>>>((const T*)x, (const T*)xz, (const T*)bc, bc_tok, dt_pre, dt_bias, a_log, d_skip, arena, (T*)y, cu_q,
                                         state_slots, sh);
