@@ -780,7 +780,11 @@ def decode_shares(n_seqs: int, n_kv_heads: int, table_tokens: int, uneven: bool 
 
     More (sequence, kv head) pairs than slots, over a table of up to 2,048 tokens: one.  Walks that short are over before a
     thin last round costs what the starts and the merge of the splits do: 40 sequences of 210 to 1,400 keys 5,618 us with 7
-    splits, 4,735 with one, all of 1,400 6,087 and 5,685; 48 of 90 to 600 4,704 with 2, 4,473 with one.
+    splits, 4,735 with one, all of 1,400 6,087 and 5,685; 48 of 90 to 600 4,704 with 2, 4,473 with one.  But not where all are
+    about as long and the table is longer than 1,024: up to two, since there the last round is thin for as long as the others
+    take (41 of 2,000 6,589 us with one, 6,242 with two, 6,440 with ``decode_splits``' 6; 48 of 2,000 6,694, 6,411, 6,411; 48
+    of 1,500 6,034, 5,907, 5,907; of 1,100 one and two are level).  Up to a tenth more pairs than slots keep one there too,
+    which is no slower than ``decode_splits``' 7 or 8 (38 of 2,000 6,310 and 6,458 us, though 6,089 with two).
 
     ``uneven`` (``StepContext.uneven``: the keys of all are well under the longest's times their number) over a longer table:
     the short ones' blocks end early and leave their slots to others.  Pairs that fit the slots take splits for 384 blocks, a share
@@ -794,7 +798,8 @@ def decode_shares(n_seqs: int, n_kv_heads: int, table_tokens: int, uneven: bool 
         return splits
     pairs = max(1, n_seqs * n_kv_heads)
     if pairs > _DECODE_SLOTS and table_tokens <= 2048:
-        return 1
+        alike = not uneven and table_tokens > 1024 and 10 * pairs > 11 * _DECODE_SLOTS
+        return min(splits, 2) if alike else 1
     if uneven and pairs > _DECODE_SLOTS:
         splits = min(splits, 2)
     elif uneven and table_tokens >= 3072:

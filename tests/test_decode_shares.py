@@ -25,3 +25,12 @@ def test_uneven_steps(lens, want):
     ctx = StepContext(types.SimpleNamespace(dtype=torch.float32, device="cpu"), len(lens), len(lens),
                       HostBatch([1] * len(lens), lens, [-1] * len(lens)))
     assert ctx.uneven is want
+
+
+# more pairs than slots over a short table: sequences of like length behind 1,024 tokens take two where ``decode_splits`` takes two or more
+@pytest.mark.parametrize("n,table,uneven,want", [(38, 2048, False, 1), (40, 2048, False, 1), (41, 2048, False, 2), (44, 2048, False, 2), (48, 2048, False, 2),
+                                                 (55, 2048, False, 2), (56, 2048, False, 1), (64, 2048, False, 1), (44, 2048, True, 1), (48, 1040, False, 2),
+                                                 (48, 1024, False, 1), (44, 600, False, 1), (37, 2048, False, 1)])
+def test_shares_of_more_pairs_than_slots_over_a_short_table(n, table, uneven, want):
+    from pulsar_b200 import ops
+    assert ops.decode_shares(n, 8, table, uneven) == want
