@@ -74,6 +74,9 @@ class ModelRunner:
         # Decode steps (one token per request) are launch-bound: their kernel sequence is
         # captured once per (batch size, block-table width) and replayed.
         self.cuda_graphs = bool(cuda_graphs) and bool(getattr(model, "graph_safe", True)) and not profiling.ENABLED
+        # (group, kv heads) of the caches whose attention may cut its keys by the lengths' unevenness
+        self._sharing = [(g, grp.pools["k"].shape[2]) for g, grp in enumerate(cache.groups) if "k" in (grp.pools or {})] \
+            if getattr(model, "shares_keys", False) else []
         self._graphs: Dict[tuple, Tuple[torch.cuda.CUDAGraph, torch.Tensor, int]] = {}
         self._graph_seen: Dict[tuple, int] = {}
         self._graph_epoch = -1
@@ -208,6 +211,8 @@ class ModelRunner:
         ctx.on_layer = self.layer_hook
         widths = list(widths_c[:n_groups])
         ctx.table_widths = tuple(widths)
+        if ctx.uneven:
+            ctx.uneven = ctx.all_decode and ops.unevenness_matters(s, [(heads, widths[g] * cache.page_size) for g, heads in self._sharing])
         moved = any(e.token_src is not None for e in entries)
         n_arrays = 7 + 2 * n_groups + (2 if moved else 0)
         offsets_c, lengths_c = (ctypes.c_int * n_arrays)(), (ctypes.c_int * n_arrays)()

@@ -91,6 +91,11 @@ class DecoderModel(Part):
         """Whether a step of this model may be captured into a CUDA graph (every part says so)."""
         return all(getattr(b, "graph_safe", True) for b in self.blocks) and getattr(self.final_norm, "graph_safe", True)
 
+    @property
+    def shares_keys(self) -> bool:
+        """Whether any part runs the dense decode attention (see ``Part``)."""
+        return any(getattr(b, "shares_keys", False) for b in self.blocks)
+
     # ---------------------------------------------------------------- weights
     def weight_specs(self) -> List[WeightSpec]:
         s = self.spec

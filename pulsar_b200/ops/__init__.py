@@ -807,6 +807,12 @@ def decode_shares(n_seqs: int, n_kv_heads: int, table_tokens: int, uneven: bool 
     return max(splits, min(32, table_tokens // 64, 128 // pairs))
 
 
+def unevenness_matters(n_seqs: int, shapes) -> bool:
+    """Whether any of the attentions of a step of single tokens, ``shapes`` = (kv heads, tokens of the block table) each, takes
+    other shares because its sequences are of unlike length."""
+    return any(decode_shares(n_seqs, heads, tokens, True) != decode_shares(n_seqs, heads, tokens, False) for heads, tokens in shapes)
+
+
 _TICKETS = 1 << 16
 _decode_tickets = {}
 
@@ -983,7 +989,8 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
     applies (bfloat16, head size 128, pages of 8 or more), else the mma.sync kernel (bfloat16, head
     size 64 or 128), else the generic kernel.  ``PULSAR_ATTENTION=mma`` leaves the tcgen05 kernel out."""
     if ctx.all_decode:
-        n_splits = decode_shares(ctx.n_seqs, cache.k_pool.shape[1], cache.block_table.shape[1] * cache.k_pool.shape[2], ctx.uneven)
+        n_splits = decode_shares(ctx.n_seqs, cache.k_pool.shape[1], cache.block_table.shape[1] * cache.k_pool.shape[2],
+                                 getattr(ctx, "uneven", False))
         partial = ctx.scratch("attn.partial", (ctx.n_seqs * q.shape[1] * n_splits * (q.shape[2] + 2),), torch.float32)
         paged_attention_decode(q, cache.k_pool, cache.v_pool, out, partial, cache.block_table, ctx.kv_len, scale,
                                window, n_splits)

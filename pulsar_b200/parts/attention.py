@@ -89,6 +89,7 @@ class Attention(Mixer):
                             or spec.keep_first or spec.softcap is not None or spec.sinks or spec.fixed_sink is not None
                             or spec.output_gate or self.prepared or self.whole or spec.sigmoid_weights
                             or self.maps > 1 or spec.q_temperature is not None)
+        self.shares_keys = not self.general
         if (self.maps > 1 or spec.q_temperature is not None) and (self.prepared or not spec.own_kv):
             raise ValueError("attention: the differential form and the query temperature go with plain projections of its own keys")
         if spec.q_temperature is not None and not (int(spec.q_temperature[1]) > 0):

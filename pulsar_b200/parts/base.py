@@ -78,7 +78,8 @@ class StepContext:
         self.max_kv_len = max(host.kv_lens) if host.kv_lens else 0
         self.all_decode = self.max_q_len == 1
         # whether the sequences hold together less than 0.7 of what they would if all were as long as the longest (part of a
-        # captured step's key: what is decided by it holds for every replay)
+        # captured step's key: what is decided by it holds for every replay).  The step function takes it back where nothing in
+        # the step is decided by it, so that such steps stay captured while their lengths change.
         self.uneven = 10 * sum(host.kv_lens) < 7 * self.max_kv_len * len(host.kv_lens)
         # int32 device arrays
         self.token_ids = self.positions = self.seq_of_token = None      # [N]
@@ -117,6 +118,10 @@ class Part:
     # whose ``forward`` decides anything on the host from the step's contents (``ctx.host``: lengths, slots) would
     # replay stale decisions: it sets this to False, and a model that holds such a part is never captured.
     graph_safe: bool = True
+
+    # Whether ``forward`` runs the dense decode attention (``ops.attention``), whose shares of the keys may follow ``ctx.uneven``.
+    # A step of a model without such a part has ``uneven`` False.
+    shares_keys: bool = False
 
     def weight_specs(self) -> List[WeightSpec]:
         return []
@@ -193,6 +198,10 @@ class Block(Part):
     @property
     def graph_safe(self) -> bool:
         return all(getattr(p, "graph_safe", True) for p in self.parts)
+
+    @property
+    def shares_keys(self) -> bool:
+        return any(getattr(p, "shares_keys", False) for p in self.parts)
 
     def state_need(self) -> Optional[CacheNeed]:
         """What the arrangement itself carries from token to token for every sequence (``CacheNeed.state``), or None.  The

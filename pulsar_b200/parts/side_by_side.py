@@ -47,6 +47,10 @@ class SideBySide(Mixer):
     def graph_safe(self) -> bool:
         return all(getattr(m, "graph_safe", True) for m in self.members)
 
+    @property
+    def shares_keys(self) -> bool:
+        return any(getattr(m, "shares_keys", False) for m in self.members)
+
     def weight_specs(self) -> List[WeightSpec]:
         return [w for m in self.members for w in m.weight_specs()] + [
             WeightSpec(name, (self.spec.hidden,), role="vector", init="ones_normal") for name in self.norm_names]

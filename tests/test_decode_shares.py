@@ -1,4 +1,5 @@
 """How many shares a decode step's keys are cut into, and when a step counts as uneven."""
+import copy
 import types
 
 import pytest
@@ -34,3 +35,37 @@ def test_uneven_steps(lens, want):
 def test_shares_of_more_pairs_than_slots_over_a_short_table(n, table, uneven, want):
     from pulsar_b200 import ops
     assert ops.decode_shares(n, 8, table, uneven) == want
+
+
+def test_unevenness_counts_only_where_shares_follow_it():
+    from pulsar_b200 import ops
+    assert not ops.unevenness_matters(8, [(8, 1024)]) and not ops.unevenness_matters(8, [(8, 4096)]) and not ops.unevenness_matters(8, [])
+    assert ops.unevenness_matters(16, [(8, 4096)]) and ops.unevenness_matters(44, [(8, 2048)]) and not ops.unevenness_matters(44, [(8, 1024)])
+    assert ops.unevenness_matters(16, [(8, 1024), (8, 4096)]) and not ops.unevenness_matters(16, [(2, 4096)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", ["dense", "general"])
+def test_a_step_stays_captured_while_its_lengths_become_even(sizes, tmp_path):
+    """Four sequences that begin uneven and become even: one capture, whatever the share of keys they hold together."""
+    import helpers
+    from pulsar_b200.engine.engine import Engine
+    from pulsar_b200.engine.runner import StepEntry
+    if sizes == "dense":
+        raw, seed, page = helpers.TINY["F"]
+    else:
+        from test_bubotar import CONFIGS
+        raw, seed, page = CONFIGS["A"]
+    helpers.make_folder(str(tmp_path), copy.deepcopy(raw), seed, store_dtype=torch.bfloat16)
+    engine = Engine(str(tmp_path), dict(dtype="bfloat16", page_size=page, num_pages=128, max_sessions=4, max_running=4, max_chunk_size=256, eos_id=-1))
+    assert engine.model.shares_keys is (sizes == "dense")
+    assert engine.runner._sharing == ([(0, 8)] if sizes == "dense" else [])
+    runner = engine.runner
+    runner.step([StepEntry(i, [1 + i] * n, []) for i, n in enumerate((30, 30, 30, 60))])
+    seen = set()
+    for i in range(30):
+        runner.step([StepEntry(r, [5], [0]) for r in range(4)])
+        lens = [31 + i] * 3 + [61 + i]
+        seen.add(10 * sum(lens) < 7 * max(lens) * 4)
+    assert seen == {True, False}
+    assert len(runner._graphs) == 1 and runner.graph_replays >= 26          # a few eager steps first, while buffers grow
