@@ -189,7 +189,7 @@ def test_add_rmsnorm_of_many_rows(width, dtype):
 
 # The order of a row's sum of squares comes from the width alone: a row has the same bits in a step of a few rows as in one of many,
 # so that a float32 prompt's logits do not depend on how it was cut into steps.
-@pytest.mark.parametrize("width", [36, 2048, 4096, 4100, 8192, 8196])
+@pytest.mark.parametrize("width", [36, 2044, 2048, 3000, 4000, 4096, 4100, 8192, 8196])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_add_rmsnorm_does_not_depend_on_the_number_of_rows(width, dtype):
     from pulsar_b200 import ops
