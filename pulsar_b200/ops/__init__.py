@@ -192,11 +192,14 @@ def code(dtype: torch.dtype) -> int:
         raise KernelError(f"dtype {dtype} is not float32 or bfloat16") from None
 
 
-# The current device's current stream as a number, without the Stream object that torch.cuda.current_stream() makes.
-_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+# The current device's current stream as a number, without the Stream object that torch.cuda.current_stream() makes.  Both are
+# private to PyTorch and a build without CUDA has neither: there the public way says what is missing, at the first launch.
+_raw_stream, _device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
 
 
 def stream() -> int:
+    if _raw_stream is None or _device is None:
+        return torch.cuda.current_stream().cuda_stream
     return _raw_stream(_device())
 
 

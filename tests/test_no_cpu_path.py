@@ -45,3 +45,23 @@ def test_trace_run_and_the_command_line_fail_loudly(tmp_path):
     proc = subprocess.run([sys.executable, os.path.join(ROOT, "bin", "pulsar-generate"), "--model", folder, "--prompt_ids", "1,2,3",
                            "--gen_tokens", "2", "--dtype", "float32"], capture_output=True, text=True, timeout=300)
     assert proc.returncode != 0 and "no CPU path" in (proc.stderr + proc.stdout)
+
+
+def test_the_package_is_imported_where_pytorch_has_no_cuda():
+    """A PyTorch built without CUDA lacks the private functions that name the current stream: importing works all the same, and
+    asking for a stream says what PyTorch says."""
+    program = """
+import torch
+for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"):
+    if hasattr(torch._C, name):
+        delattr(torch._C, name)
+import pulsar_b200
+from pulsar_b200 import ops
+class Stream:
+    cuda_stream = 77
+torch.cuda.current_stream = lambda: Stream
+assert ops.stream() == 77
+print("imported")
+"""
+    done = subprocess.run([sys.executable, "-c", program], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, cwd=ROOT, timeout=300)
+    assert done.returncode == 0 and "imported" in done.stdout, done.stdout
