@@ -153,20 +153,12 @@ simt_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* _
 }
 
 template <int R, int T, int CW, int RST, typename TO>
-int launch_rows_st(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
+int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
     constexpr int MR = 32 / (RN / R) * T * CW;
     constexpr size_t smem = sizeof(float) * RST * (RN * RSTRIDE + MR * RK);
     static SmemLimit limit;
     if (const int rc = limit.allow(simt_rows_kernel<R, T, CW, RST, TO>, smem)) return rc;
     return launch_early(loaded, simt_rows_kernel<R, T, CW, RST, TO>, dim3((N + RN - 1) / RN), dim3(RLOAD + 32 * CW), smem, stream, A, W, out, M, N, K);
-}
-
-// With one block an SM or fewer a block's ring has to keep HBM busy by itself: 16 stages instead of 8 (4096 x 4096, one row of A:
-// 19.3 against 19.5 us; 4096 x 12288: 43.9 against 50.3).
-template <int R, int T, int CW, typename TO>
-int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
-    if ((N + RN - 1) / RN <= 148) return launch_rows_st<R, T, CW, 16>(A, W, out, M, N, K, loaded, stream);
-    return launch_rows_st<R, T, CW, 8>(A, W, out, M, N, K, loaded, stream);
 }
 
 // ---------------------------------------------------------------- more rows
@@ -277,12 +269,16 @@ int launch_tile(const float* A, const float* W, TO* out, int M, int N, int K, cu
 // float32 operands whose rows are multiples of 16 bytes on 16-byte addresses
 template <typename TO>
 int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
-    if (M == 1) return launch_rows<1, 1, 1>(A, W, out, M, N, K, loaded, stream);
-    if (M == 2) return launch_rows<2, 1, 1>(A, W, out, M, N, K, loaded, stream);
-    if (M <= 4) return launch_rows<2, 1, 2>(A, W, out, M, N, K, loaded, stream);
+    // With one block an SM or fewer a block's ring has to keep HBM busy by itself: 16 stages instead of 8 (4096 x 4096, one row of A:
+    // 19.3 against 19.5 us; 4096 x 12288: 43.9 against 50.3).
     const bool few = (N + RN - 1) / RN <= 148;
-    if (M <= 8) return few ? launch_rows<2, 1, 4>(A, W, out, M, N, K, loaded, stream) : launch_rows<2, 2, 2>(A, W, out, M, N, K, loaded, stream);
-    if (M <= 16) return few ? launch_rows<2, 1, 8>(A, W, out, M, N, K, loaded, stream) : launch_rows<4, 2, 2>(A, W, out, M, N, K, loaded, stream);
+#define PB_ROWS(R, T, CW, ST) return launch_rows<R, T, CW, ST>(A, W, out, M, N, K, loaded, stream)
+    if (M == 1) { if (few) PB_ROWS(1, 1, 1, 16); PB_ROWS(1, 1, 1, 8); }
+    if (M == 2) { if (few) PB_ROWS(2, 1, 1, 16); PB_ROWS(2, 1, 1, 8); }
+    if (M <= 4) { if (few) PB_ROWS(2, 1, 2, 16); PB_ROWS(2, 1, 2, 8); }
+    if (M <= 8) { if (few) PB_ROWS(2, 1, 4, 16); PB_ROWS(2, 2, 2, 8); }
+    if (M <= 16) { if (few) PB_ROWS(2, 1, 8, 16); PB_ROWS(4, 2, 2, 8); }
+#undef PB_ROWS
     // 64 rows a block where there are blocks for 16 rounds of the SMs (151936 x 4096, 387 rows: 11.3 against 11.9 ms), else 32, whose last
     // rounds are less empty (4096 x 4096: 33 rows 161 against 269 us, 387 rows 356 against 500, the general kernel 656;
     // 24576 x 4096, 387 rows: 1.90 against 2.00 ms, 2.96 before)
