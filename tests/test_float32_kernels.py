@@ -36,6 +36,25 @@ def test_products_of_rows_and_tiles(m, n, k):
         assert torch.equal(half, out.bfloat16())
 
 
+# every ring of stages turns more than twice, with a ragged tail: 16 and 8 stages of 64 k for every number of rows that streams the
+# weights, three stages of 16 k of the tiles of 64 rows
+@pytest.mark.parametrize("m,n,k", [(m, 130, 2116) for m in range(1, 17)] + [(m, 4800, 1092) for m in range(1, 17)]
+                         + [(65, 153600, 132), (100, 153600, 132), (33, 130, 1092), (100, 321, 2116)])
+def test_products_whose_stages_are_used_again(m, n, k):
+    from pulsar_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(m * 1000 + k)
+    a, w = (torch.randn(r, k, generator=g, device="cuda") for r in (m, n))
+    out, want = torch.full((m, n), float("nan"), device="cuda"), torch.empty(m, n, device="cuda")
+    ops.gemm_simt(_unaligned(a), w, want)
+    for loaded in (False, True):
+        out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        ops.gemm_simt(a, w, out, loaded)
+        assert torch.equal(out, want), "the sums are the general kernel's, bit for bit"
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert bool(((out.double() - ref).abs() <= (k + 1) * 2.0 ** -24 * size).all())       # a chain of k rounded multiply-adds
+
+
 # 16 rows a block (many rows; head sizes up to 64 and 128), 8 (wider heads), 4 (few rows); groups of one to more heads than a block
 # has rows, blocks whose tokens belong to several sequences, windows that begin inside a tile
 @pytest.mark.parametrize("q_lens,kv_lens,hq,hkv,d,page,window", [
