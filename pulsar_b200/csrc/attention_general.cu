@@ -959,7 +959,10 @@ __global__ void qkv_split_write_kernel(const T* __restrict__ qkv, float* __restr
                                        T* __restrict__ v_pool, const int* __restrict__ slots, int Hq, int Hk, int Hv, int Dk, int Dv,
                                        int page_size, const int* __restrict__ positions, float temp_coef, int temp_every,
                                        const PoolBounds bounds) {
-    pdl_trigger();      // a short kernel: the next one may fetch its weights now
+    // A short kernel: the next one may fetch its weights now.  Not where the blocks come in rounds: the next kernel could only come in
+    // the last one, and what every block pays for the word adds up (us, 48 heads of 64 and 16 of 128: 2,048 tokens 21.4 without, 35.6
+    // with it; 256 tokens, 4,096 blocks, 5.1 and 6.1; 64 tokens, 1,024 blocks, 3.4 either way).
+    if (gridDim.x * gridDim.y <= 16 * 148) pdl_trigger();
     pdl_wait();         // may have come onto the SMs while the product before it was ending: nothing is touched before that one is done
     const int t = blockIdx.x, lane = threadIdx.x & 31;
     const int head = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
