@@ -162,7 +162,7 @@ int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, bo
 }
 
 // ---------------------------------------------------------------- more rows
-// Bound by the FMA pipes (59 % of their cycles with 24576 x 1024 weights and 384 rows; the issue slots 71 %).  A block of 128
+// Bound by the FMA pipes (60 % of their cycles with 24576 x 4096 weights and 387 rows; the issue slots 75 %).  A block of 128
 // threads owns 8 TM x 128 outputs, a warp 8 TM x 32, a thread TM x 8 of them (rows ty + 8 i, columns tx + 4 j).  Both operands
 // stand in shared memory as they do in memory, k fastest, so that asynchronous 16-byte copies bring them and a thread reads four
 // k of a row at once: 16 reads per 256 multiply-adds with TM 8.  Rows stand an odd number of 16-byte units apart (no

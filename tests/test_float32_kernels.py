@@ -55,8 +55,8 @@ def test_products_whose_stages_are_used_again(m, n, k):
     assert bool(((out.double() - ref).abs() <= (k + 1) * 2.0 ** -24 * size).all())       # a chain of k rounded multiply-adds
 
 
-# 16 rows a block (many rows; head sizes up to 64 and 128), 8 (wider heads), 4 (few rows); groups of one to more heads than a block
-# has rows, blocks whose tokens belong to several sequences, windows that begin inside a tile
+# 16 rows a block (many rows; head sizes up to 64 and 128), 8 (wider heads), 4 and 1 (few rows); groups of one to more heads than a
+# block has rows, tokens of several sequences, windows that begin inside a tile
 @pytest.mark.parametrize("q_lens,kv_lens,hq,hkv,d,page,window", [
     ([387], [420], 16, 4, 128, 16, None), ([300, 1, 41, 3], [300, 70, 500, 3], 20, 4, 64, 16, 150), ([700], [700], 8, 2, 208, 8, 40),
     ([5, 1, 70], [5, 90, 200], 6, 2, 32, 4, None), ([33], [164], 40, 2, 80, 16, 50), ([260], [261], 36, 1, 48, 4, 33)])
