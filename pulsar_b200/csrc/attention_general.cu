@@ -566,7 +566,7 @@ constexpr int kSRow = kTile + 4;        // floats of a row of partial scores
 // weights are at most one).
 __device__ __forceinline__ float to_bf16_range(float x) {
     constexpr float most = 3.3895313892515355e38f;          // bfloat16's largest
-    return fabsf(x) == INFINITY ? x : fminf(fmaxf(x, -most), most);
+    return fabsf(x) < INFINITY ? fminf(fmaxf(x, -most), most) : x;      // (what is no number stays none)
 }
 template <bool kLarge>
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
@@ -578,6 +578,10 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
     y -= __uint_as_float(mid & 0xffff0000u);
     lo = pack_bf16(x, y);
 }
+
+// A product from its first part and the rest.  An infinite key or value makes the first part what the whole product is; the rest, where
+// it meets zeros and numbers of the other sign, is then NaN or infinite itself and says nothing.
+__device__ __forceinline__ float with_rest(float first, float rest) { return fabsf(first) == INFINITY ? first : first + rest; }
 
 template <int KS, int VT>
 __global__ void __launch_bounds__(128)
@@ -717,7 +721,7 @@ general_rows_tc_kernel(const float* __restrict__ q, const bf16* __restrict__ k_p
 #pragma unroll
             for (int r = 0; r < 2; ++r)
                 *reinterpret_cast<float2*>(s_s + (warp * kRows + (lane >> 2) + 8 * r) * kSRow + n * 8 + (lane & 3) * 2) =
-                    make_float2(sc[n][2 * r] + sr[n][2 * r], sc[n][2 * r + 1] + sr[n][2 * r + 1]);
+                    make_float2(with_rest(sc[n][2 * r], sr[n][2 * r]), with_rest(sc[n][2 * r + 1], sr[n][2 * r + 1]));
         __syncthreads();
 
         // the softmax weights of this thread's two rows: keys 8 n + 2 (lane mod 4) + {0, 1}, the columns of the scores' fragments
@@ -812,8 +816,8 @@ general_rows_tc_kernel(const float* __restrict__ q, const bf16* __restrict__ k_p
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                acc[i][e] += o[0][e] + rest[0][e];
-                acc[i + 1][e] += o[1][e] + rest[1][e];
+                acc[i][e] += with_rest(o[0][e], rest[0][e]);
+                acc[i + 1][e] += with_rest(o[1][e], rest[1][e]);
             }
         }
     }

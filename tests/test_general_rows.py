@@ -127,6 +127,38 @@ def test_queries_at_the_ends_of_float32(large, sigmoid):
     assert float((got.double() - want).norm() / want.norm()) < 1e-5       # scores near 9, known to 2^-21 of that: the weights to 5e-6
 
 
+# infinite numbers in the cache: a key whose score is -infinity weighs nothing (with sigmoid weights one at +infinity weighs one), an
+# infinite value makes its column infinite and no other.  Queries of one bfloat16 (0.25) and of three parts of both signs (0.3); one
+# that is no number beside them takes its own head's row and no other.
+@pytest.mark.parametrize("hq,hkv,dk,dv", [(4, 2, 64, 64), (16, 1, 576, 512)])
+@pytest.mark.parametrize("sigmoid", [False, True])
+def test_infinite_keys_and_values(hq, hkv, dk, dv, sigmoid):
+    from pulsar_b200 import ops
+    kv_lens, page = [70, 33], 16
+    gen = torch.Generator().manual_seed(5)
+    table, (k_pool, v_pool) = _paged([1, 1], kv_lens, page, [(hkv, dk), (hkv, dv)], torch.bfloat16, gen)
+    q = torch.randn(2, hq, dk, generator=gen).cuda() * 0.1
+    q[0, :, 5], q[1, :, 5], q[1, -1, 6] = 0.25, 0.3, math.nan
+    first = table[:, 0].long().cuda()                        # both sequences' first pages
+    k_pool[first, :, 3, 5] = -math.inf
+    if sigmoid:
+        k_pool[first, :, 4, 5] = math.inf
+    v_pool[first, :, 7, 9], v_pool[first, :, 8, 17] = math.inf, -math.inf
+    ctx, got, want = _Ctx([1, 1], kv_lens), torch.empty(2, hq, dv, device="cuda"), torch.empty(2, hq, dv, dtype=torch.float64, device="cuda")
+    ops.paged_attention_general(ctx, q, k_pool, v_pool, got, table.cuda(), 0.5, tensor_cores=False, sigmoid=sigmoid)
+    for s, kl in enumerate(kv_lens):
+        k, v = (_keys_of(p, table, s, kl, page).repeat_interleave(hq // hkv, dim=1) for p in (k_pool, v_pool))
+        sc = torch.einsum("hd,jhd->hj", q[s].double(), k) * 0.5
+        w = torch.sigmoid(sc) if sigmoid else torch.softmax(sc, dim=-1)
+        want[s] = torch.einsum("hj,jhv->hv", w, v)
+    assert bool(torch.isnan(got[1, -1]).all())
+    got, want = (x.view(2 * hq, dv)[:-1] for x in (got, want))
+    fin = torch.isfinite(want)
+    assert not bool(torch.isnan(want).any()) and int((~fin).sum()) == 2 * (2 * hq - 1)
+    assert torch.equal(got[~fin].double(), want[~fin])
+    assert float((got[fin].double() - want[fin]).norm() / want[fin].norm()) < 1e-5       # as at the ends of float32
+
+
 @pytest.mark.parametrize("q_lens,kv_lens,hq,hkv,dk,dv", [([1, 1], [1900, 70], 16, 1, 576, 512), ([1, 3], [500, 64], 8, 4, 64, 64)])
 def test_partial_results_at_any_float(q_lens, kv_lens, hq, hkv, dk, dv):
     """Scratch that begins at an odd float (a view of a caller's own buffer)."""
