@@ -70,8 +70,7 @@ _SIGNATURES = {
     "pb_gemm_tcgen05": [_I, _I, _P, _P, _P, _I, _I, _I, _P],
     "pb_gemm_tcgen05_supported": [_I, _I, _I, _I],
     "pb_gemm_tcgen05_error": [],
-    "pb_gemm_tcgen05_stream": [_I, _I, _P, _P, _P, _I, _I, _I, _P, ctypes.c_longlong, _P, _I, _P],
-    "pb_gemm_tcgen05_stream_workspace": [_I, _I, _I, _I, _P, _P],
+    "pb_gemm_tcgen05_stream": [_I, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "pb_gemm_tcgen05_stream_supported": [_I, _I, _I, _I],
     "pb_gemm_tcgen05_stream_wait_control": [ctypes.c_longlong, _I, _P],
     "pb_gemm_tcgen05_wait_control": [ctypes.c_longlong, _I, _P],
@@ -497,48 +496,34 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bo
     return True
 
 
-# Which products of 17 to 128 tokens take this library's weight-streaming tcgen05 kernel instead of the library
-# product: "auto" those whose weights have tiles for four rounds of all SMs or more (the head: there the kernel's
-# persistent form is ahead of the library, 6.1 against 6.0 TB/s at 64 tokens); "1" all of them (measured behind the
-# library for the projections of a layer at the 8B sizes: see profiles/); "0" none.
+# Which products of 17 to 128 tokens take this library's weight-streaming tcgen05 kernel instead of the library product: "auto" as
+# ``_stream_wanted`` has it; "1" all of them; "0" none.
 STREAM_GEMM = os.environ.get("PULSAR_GEMM_STREAM", "auto")
 _STREAM_MIN_ROWS = 4 * 148 * 128
 
 
-def _stream_wanted(m: int, n: int) -> bool:
+def _stream_wanted(m: int, n: int, k: int, gated: bool = False) -> bool:
+    """Where the weight-streaming kernel is ahead.  It sets up, meets and ends in about 5 us, some of it under the kernels around
+    it; the tokens are read again with every tile of weights, which costs the more the more there are.  us, library / kernel, one
+    launch behind the other: 32 tokens 2048 x 4096 8.1 / 6.9, 160 x 4096 7.0 / 3.9, 8192 x 2048 8.2 / 8.6, 16384 x 2048 gated 15.1 / 13.6,
+    1024 x 1024 3.8 / 4.2; 64 tokens 8192 x 2048 8.5 / 9.9, 8192 x 4096 15.3 / 14.3; 96 tokens 4096 x 8192 16.6 / 15.9, 8192 x 4096
+    15.3 / 16.2, 24576 x 4096 gated 43.4 / 38.7; 128 tokens the same 43.3 / 45.5, 4096 x 8192 16.5 / 18.3.  In a layer of the 8B
+    sizes the kernels before and behind hide more of it: its four products with their norms take 80 us at 48 tokens (library 90)
+    and 83 at 64 (93)."""
     if m > 128 or STREAM_GEMM == "0" or GEMM_BACKEND == "library":
         return False
-    return STREAM_GEMM == "1" or n >= _STREAM_MIN_ROWS
+    if STREAM_GEMM == "1" or n >= _STREAM_MIN_ROWS:
+        return True
+    if m <= 64:
+        return k >= (2048 if m <= 32 else 4096)
+    return k >= 4096 and m <= 112 if gated else k >= 8192 and m <= 96
 
 
-# Float32 partial sums and tile tickets of the product below, one pair per device, grown on demand.  A buffer
-# that was outgrown stays alive: a captured graph may still name it.  Kernels of one stream share the pair (each
-# finishes with it before the next one starts, and leaves the tickets zero).
-_stream_scratch = {}
-_stream_scratch_old = []
-
-
-def _stream_workspace(device: torch.device, mode: int, m: int, n: int, k: int):
-    floats, tickets = ctypes.c_longlong(0), ctypes.c_int(0)
-    fn("pb_gemm_tcgen05_stream_workspace")(mode, m, n, k, ctypes.byref(floats), ctypes.byref(tickets))
-    if floats.value == 0:
-        return None, None
-    have = _stream_scratch.get(device)
-    if have is None or have[0].numel() < floats.value or have[1].numel() < tickets.value:
-        if torch.cuda.is_current_stream_capturing():
-            return None, None                 # no allocation inside a capture: whole tiles this once
-        if have is not None:
-            _stream_scratch_old.append(have)
-        have = (torch.empty(max(floats.value, have[0].numel() if have else 0), dtype=torch.float32, device=device),
-                torch.zeros(max(tickets.value, have[1].numel() if have else 0, 2048), dtype=torch.int32, device=device))
-        _stream_scratch[device] = have
-    return have
-
-
-def gemm_tcgen05_stream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bool = False) -> bool:
+def gemm_tcgen05_stream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bool = False, gating=None, loaded: bool = True) -> bool:
     """The weight-streaming tcgen05 / TMA product for up to 128 tokens (bfloat16 operands, float32 accumulation
-    in tensor memory, K cut into slices whose partial sums meet in a float32 workspace).  ``swiglu`` as in
-    ``gemm_skinny``.  Returns False, having done nothing, when the sizes are not the kernel's."""
+    in tensor memory, K cut into slices whose float32 sums meet in a cluster's shared memory).  ``swiglu`` and ``gating`` as in
+    ``gemm_skinny``; ``loaded``: no kernel still on the stream writes ``w``, which then is read before those have ended.
+    Returns False, having done nothing, when the sizes are not the kernel's."""
     m, k = a.shape
     n = w.shape[0]
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or w.shape[1] != k:
@@ -548,13 +533,10 @@ def gemm_tcgen05_stream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swi
         return False
     _cuda(a, w, out)
     assert out.shape == (m, n // 2 if swiglu else n)
-    work, tickets = _stream_workspace(a.device, mode, m, n, k)
-    status = fn("pb_gemm_tcgen05_stream")(mode, code(out.dtype), _p(a), _p(w), _p(out), m, n, k,
-                                          _p(work) if work is not None else None, work.numel() if work is not None else 0,
-                                          _p(tickets) if tickets is not None else None,
-                                          tickets.numel() if tickets is not None else 0, stream())
+    with _Gating(gating if swiglu else None):
+        status = fn("pb_gemm_tcgen05_stream")(mode, code(out.dtype), _p(a), _p(w), _p(out), m, n, k, int(loaded), stream())
     if status == -3:
-        return False                 # sizes that leave no room for its ring of stages
+        return False                 # addresses that are no multiples of 16
     check(status, "gemm_tcgen05_stream")
     return True
 
@@ -686,10 +668,10 @@ def check_wait_words() -> None:
 def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, loaded: bool = False) -> None:
     """out = a @ w.T.  float32 operands take the float32 CUDA-core product (true 32-bit,
     no reduced-precision mode).  bfloat16 operands: up to 16 rows take this library's
-    weight-streaming kernel; more rows take the library product with float32 accumulation,
-    as the reference does for every projection (pulsar-core/src/model/qwen3.cpp:82-84:
-    at::linear).  ``loaded``: as ``gemm_simt`` has it, for float32.  The bfloat16 streaming
-    kernels read ``w`` early in any case: it has to be a weight that was there before the
+    weight-streaming kernel, up to 128 its tcgen05 form where ``_stream_wanted`` says so; the others take the library product
+    with float32 accumulation, as the reference does for every projection (pulsar-core/src/model/qwen3.cpp:82-84:
+    at::linear).  ``loaded``: as ``gemm_simt`` has it, for float32 and for 17 rows and more.  The bfloat16 streaming
+    kernel of up to 16 rows reads ``w`` early in any case: it has to be a weight that was there before the
     kernels still on the stream were launched."""
     if a.dtype == torch.float32 and w.dtype == torch.float32:
         gemm_simt(a, w, out, loaded)
@@ -699,7 +681,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, loaded: bool = F
         raise KernelError(f"linear: operand dtypes {a.dtype} / {w.dtype} must both be float32 or both bfloat16")
     if gemm_skinny(a, w, out):
         return
-    if _stream_wanted(a.shape[0], w.shape[0]) and gemm_tcgen05_stream(a, w, out):
+    if _stream_wanted(a.shape[0], w.shape[0], w.shape[1]) and gemm_tcgen05_stream(a, w, out, loaded=loaded):
         return
     if GEMM_BACKEND == "tcgen05" and gemm_tcgen05(a, w, out):
         return
@@ -721,15 +703,15 @@ def gated_linear(ctx, a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tenso
     """out [M, I] = silu(a Wg^T) * (a Wu^T) with ``w_gate_up`` = gate rows then up rows; with ``gating`` = (limit, alpha,
     shift) the clamped form g * sigmoid(alpha * g) * (u + shift), g = min(a Wg^T, limit), u = clamp(a Wu^T, -limit, limit)
     (alpha infinite: max(g, 0) * (u + shift)).
-    In bfloat16, up to 16 rows (the weight-streaming kernel) and more than 128 rows (the tcgen05 kernel)
-    take one kernel that never writes the [M, 2I] intermediate; otherwise the product followed by the
+    In bfloat16, up to 16 rows, up to 112 where ``_stream_wanted`` says so (the weight-streaming kernels) and more than 128 rows (the
+    tcgen05 kernel) take one kernel that never writes the [M, 2I] intermediate; otherwise the product followed by the
     gating kernel.  ``loaded``: as ``linear`` has it."""
     if gemm_skinny(a, w_gate_up, out, swiglu=True, gating=gating):
         return
-    if gating is None and _stream_wanted(a.shape[0], w_gate_up.shape[0]) and gemm_tcgen05_stream(a, w_gate_up, out, swiglu=True):
+    if _stream_wanted(a.shape[0], *w_gate_up.shape, True) and gemm_tcgen05_stream(a, w_gate_up, out, swiglu=True, gating=gating, loaded=loaded):
         return
-    # Between 17 and 128 rows the product is still bound by streaming the weights, which the library's small
-    # tiles do faster (4.5 against 3.2 TB/s at the 8B sizes) than the tcgen05 kernel's 128 x 256 tiles.
+    # Up to 128 rows the product is still bound by streaming the weights, which where the kernel above declines the library's small
+    # tiles do faster than the tcgen05 kernel's 128 x 256 tiles.
     fused = GEMM_BACKEND == "tcgen05" or (GEMM_BACKEND == "auto" and a.shape[0] > 128)
     if fused and gemm_tcgen05(a, w_gate_up, out, swiglu=True, gating=gating):
         return
