@@ -53,6 +53,10 @@ __device__ __forceinline__ void unpack_bf16(uint32_t v, float& lo, float& hi) {
     hi = __uint_as_float(v & 0xffff0000u);
 }
 
+// Bit of evict_first: the launch may run while the kernel before it on the stream still does.  That kernel was launched the ordinary
+// way, lets its successor in at its first instruction and touches neither this one's outputs nor what it reads.
+constexpr int kBeside = 256;
+
 template <int D>
 __global__ void __launch_bounds__(kWarps * 32, 2)
 decode_tc_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pool, const bf16* __restrict__ v_pool,
@@ -103,7 +107,11 @@ decode_tc_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pool, co
     for (int i = 0; i < ahead; ++i)
         if (kStages - 1 + i < n_tiles)
             prefetch_kv_tile_l2<D>(k_pool, v_pool, table, (tile0 + kStages - 1 + i) * kTile, begin, end - 1, kvh, Hkv, page_shift, tid, bounds);
-    pdl_wait();
+    // Beside the kernel before (see kBeside): what this one reads was complete before that one began.  The last block alone waits for
+    // it, at its end, so that this kernel is complete no sooner; the others leave their places to the blocks behind them.
+    const bool beside = evict_first & kBeside;
+    const bool last = blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1;
+    if (!beside) pdl_wait();
 
     // Q fragments: rows = query heads of the group (zero beyond G), straight from global memory.
     uint32_t qa[kKSteps][4];
@@ -358,6 +366,7 @@ decode_tc_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pool, co
             if (d == 0) { __stcg(dst + D, m_all * kLn2); __stcg(dst + D + 1, l_all); }   // maximum back in natural-log units
         }
     }
+    if (beside && last) pdl_wait();
     if (tickets == nullptr || direct) return;
     __shared__ unsigned int ticket_s;
     __threadfence();
@@ -396,7 +405,7 @@ decode_tc_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pool, co
 template <int D>
 int launch_tc(const void* q, const void* k_pool, const void* v_pool, float* partial, const int* block_table,
               int table_stride, const int* kv_len, int n_seqs, int Hq, int Hkv, int page_size, float scale, int window,
-              int n_splits, void* out, unsigned int* tickets, cudaStream_t stream, const QkvFuse fuse = QkvFuse{}) {
+              int n_splits, void* out, unsigned int* tickets, cudaStream_t stream, const QkvFuse fuse = QkvFuse{}, bool beside = false) {
     const int page_shift = log2_exact(page_size);
     constexpr int pipeline = kStages * 2 * kTile * D * 2;
     constexpr int merge = (kWarps * 16 * D + 2 * kWarps * 16) * 4;
@@ -415,7 +424,7 @@ int launch_tc(const void* q, const void* k_pool, const void* v_pool, float* part
     }();
     static const int evict_flag = [] { const char* v = getenv("PULSAR_DECODE_EVICT_FIRST"); return (v && v[0] == '0' && v[1] == 0) ? 0 : 1; }();
     const int ahead = forced_ahead >= 0 ? forced_ahead : ((long long)n_splits * Hkv * n_seqs <= sms ? 2 : 0);
-    const int evict_first = evict_flag | (ahead << 4);
+    const int evict_first = evict_flag | (ahead << 4) | (beside ? kBeside : 0);
     dim3 grid(n_splits, Hkv, n_seqs);
     return launch_pdl(decode_tc_kernel<D>, grid, kWarps * 32, smem, stream, (const bf16*)q, (const bf16*)k_pool, (const bf16*)v_pool,
                       partial, block_table, table_stride, kv_len, Hq, Hkv, page_shift, scale, window, n_splits, (bf16*)out, tickets, evict_first,
@@ -467,6 +476,24 @@ PB_EXPORT int pb_paged_attention_decode_tc_fused(int dtype, const void* q, const
                              window, n_splits, out, tickets, stream);
     return launch_tc<128>(q, k_pool, v_pool, partial, block_table, table_stride, kv_len, n_seqs, Hq, Hkv, page_size, scale,
                           window, n_splits, out, tickets, stream);
+}
+
+// The same beside the kernel launched before it (the prefill attention of the step's portions, which leaves SMs idle or ends unevenly):
+// that kernel must have been launched the ordinary way, call griddepcontrol.launch_dependents in every block, and write nothing that
+// this one reads or writes.  tickets null: pb_decode_combine merges the splits.
+PB_EXPORT int pb_paged_attention_decode_tc_beside(int dtype, const void* q, const void* k_pool, const void* v_pool, void* out,
+                                                  float* partial, unsigned int* tickets, const int* block_table,
+                                                  int table_stride, const int* kv_len, int n_seqs, int Hq, int Hkv, int D,
+                                                  int page_size, float scale, int window, int n_splits, cudaStream_t stream) {
+    if (n_seqs <= 0) return 0;
+    if (!pb_decode_tc_supported(dtype, Hq, Hkv, D, page_size) || n_splits <= 0) return PB_ERR_BAD_SIZE;
+    if (Hkv > 65535 || n_seqs > 65535 || (tickets != nullptr && n_splits > 64)) return PB_ERR_TOO_LARGE;
+    const int rc = D == 64 ? launch_tc<64>(q, k_pool, v_pool, partial, block_table, table_stride, kv_len, n_seqs, Hq, Hkv, page_size, scale,
+                                           window, n_splits, tickets ? out : nullptr, tickets, stream, QkvFuse{}, true)
+                           : launch_tc<128>(q, k_pool, v_pool, partial, block_table, table_stride, kv_len, n_seqs, Hq, Hkv, page_size, scale,
+                                            window, n_splits, tickets ? out : nullptr, tickets, stream, QkvFuse{}, true);
+    if (rc != 0 || tickets != nullptr) return rc;
+    return pb_decode_combine(dtype, partial, out, n_seqs * Hq, D, n_splits, stream);
 }
 
 // The same attention for a step of single tokens whose rows come straight from the q/k/v product: qkv [n_seqs]

@@ -115,6 +115,7 @@ __device__ __forceinline__ bool next_item(Work& w, const Args& a) {
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const Args a) {
+    pdl_trigger();      // launched the ordinary way: all it reads is complete, and the decode attention of a mixed step may run beside it
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* q_s = smem;                                 // two tiles

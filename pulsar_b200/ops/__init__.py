@@ -54,6 +54,7 @@ _SIGNATURES = {
     "pb_decode_tc_supported": [_I, _I, _I, _I, _I],
     "pb_paged_attention_decode_tc_qkv": [_I, _P, _P, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
     "pb_paged_attention_decode_tc_fused": [_I, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
+    "pb_paged_attention_decode_tc_beside": [_I, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
     "pb_paged_attention_prefill_tc": [_I, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     "pb_prefill_tc_supported": [_I, _I, _I, _I, _I],
     "pb_prefill_tc_tile": [],
@@ -143,7 +144,7 @@ _fns = {}
 # the entry points that launch kernels (the others answer questions on the host): what PULSAR_PROF=1 times
 _LAUNCHERS = {"embed", "scale_cap", "move_ids", "add_rmsnorm", "rope_table", "qk_norm_rope_write", "silu_mul", "gather_words",
               "paged_attention_generic", "paged_attention_decode", "paged_attention_decode_tc", "paged_attention_decode_tc_fused",
-              "paged_attention_decode_tc_qkv",
+              "paged_attention_decode_tc_qkv", "paged_attention_decode_tc_beside",
               "paged_attention_prefill_tc", "paged_attention_prefill_tcgen05", "gemm_skinny", "gemm_skinny_accumulate",
               "gemm_skinny_scaled", "gemm_tcgen05", "gemm_tcgen05_stream", "gemm_simt", "sample", "argmax", "table_update",
               "paged_attention_general", "paged_attention_general_tiled", "paged_attention_general_tc", "qkv_split_write", "heads_linear", "latent_prepare", "latent_norms", "latent_expand_keys", "sigmoid_gate", "causal_conv_silu",
@@ -814,14 +815,15 @@ def decode_tc_supported(dtype: torch.dtype, n_heads: int, n_kv_heads: int, head_
 def paged_attention_decode(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor,
                            partial: torch.Tensor, block_table: torch.Tensor, kv_len: torch.Tensor, scale: float,
                            window: Optional[int], n_splits: int, tensor_cores: Optional[bool] = None,
-                           fused: Optional[bool] = None) -> None:
+                           fused: Optional[bool] = None, beside: bool = False) -> None:
     """One query token per sequence: q, out [S, Hq, D].  ``partial`` is float32 scratch of at
     least S * Hq * n_splits * (D + 2) elements.  ``tensor_cores``: None picks the tensor-core
     kernel where it applies, False forces the CUDA-core kernel, True insists.  ``fused``: the
     tensor-core kernel finishes the job itself (a single split writes the result; of several the
     last one to finish merges) instead of a second kernel.  None: only for a single split, where
     it saves a launch; with several splits the ticket and fences cost what the combine kernel costs
-    (measured: 5.04 vs 4.99 ms per step at batch 8)."""
+    (measured: 5.04 vs 4.99 ms per step at batch 8).  ``beside``: the tensor-core kernel may run while the kernel launched just
+    before still does; that has to be ``paged_attention_prefill_tcgen05`` over other rows."""
     _cuda(q, k_pool, v_pool, out, partial, block_table, kv_len)
     _check_against(k_pool)
     s, hq, d = q.shape
@@ -834,14 +836,22 @@ def paged_attention_decode(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.
         tensor_cores = decode_tc_supported(q.dtype, hq, hkv, d, page_size)
     if fused is None:
         fused = n_splits == 1
+    assert tensor_cores or not beside
     if tensor_cores and fused and n_splits <= 64 and s * hkv <= _TICKETS:
         tickets = _decode_tickets.get(q.device)
         if tickets is None:
             tickets = _decode_tickets[q.device] = torch.zeros(_TICKETS, dtype=torch.int32, device=q.device)
-        check(fn("pb_paged_attention_decode_tc_fused")(code(q.dtype), _p(q), _p(k_pool), _p(v_pool), _p(out), _p(partial),
+            beside = False                    # what fills them came between
+        check(fn("pb_paged_attention_decode_tc_beside" if beside else "pb_paged_attention_decode_tc_fused")(code(q.dtype), _p(q), _p(k_pool), _p(v_pool), _p(out), _p(partial),
                                                        _p(tickets), _p(block_table), block_table.shape[1], _p(kv_len), s, hq,
                                                        hkv, d, page_size, float(scale), int(window or 0), n_splits, stream()),
               "paged_attention_decode_tc_fused")
+        return
+    if beside:
+        check(fn("pb_paged_attention_decode_tc_beside")(code(q.dtype), _p(q), _p(k_pool), _p(v_pool), _p(out), _p(partial), None,
+                                                        _p(block_table), block_table.shape[1], _p(kv_len), s, hq, hkv, d, page_size,
+                                                        float(scale), int(window or 0), n_splits, stream()),
+              "paged_attention_decode_tc_beside", kernels=2)
         return
     name = "pb_paged_attention_decode_tc" if tensor_cores else "pb_paged_attention_decode"
     check(fn(name)(code(q.dtype), _p(q), _p(k_pool), _p(v_pool), _p(out), _p(partial),
@@ -991,18 +1001,25 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
         while n_dec < len(q_lens) and q_lens[n_dec] == 1:
             n_dec += 1
         table, cu_q, kv_len = cache.block_table, ctx.cu_q, ctx.kv_len
-        if n_dec > 0:
+
+        def decode(beside: bool) -> None:
             n_splits = decode_shares(n_dec, hkv, table.shape[1] * page_size)
             partial = ctx.scratch("attn.partial", (n_dec * q.shape[1] * n_splits * (q.shape[2] + 2),), torch.float32)
             paged_attention_decode(q[:n_dec], cache.k_pool, cache.v_pool, out[:n_dec], partial, table[:n_dec], kv_len[:n_dec],
-                                   scale, window, n_splits)
-            table, cu_q, kv_len, q_lens = table[n_dec:], cu_q[n_dec:], kv_len[n_dec:], q_lens[n_dec:]
+                                   scale, window, n_splits, beside=beside)
+        # A portion of 512 tokens has tiles for 64 SMs only: the decode kernel runs beside the tcgen05 kernel, on the SMs that has left
+        # (7 single tokens beside 505: 62 us a layer one behind the other, 45 beside).
+        beside = n_dec > 0 and use_tcgen05 and decode_tc_supported(q.dtype, q.shape[1], hkv, q.shape[2], page_size)
+        if n_dec > 0 and not beside:
+            decode(False)
         if use_tcgen05:
-            paged_attention_prefill_tcgen05(q, cache.k_pool, cache.v_pool, out, table, cu_q, kv_len,
-                                            prefill_tcgen05_tiles(q_lens), scale, window)
+            paged_attention_prefill_tcgen05(q, cache.k_pool, cache.v_pool, out, table[n_dec:], cu_q[n_dec:], kv_len[n_dec:],
+                                            prefill_tcgen05_tiles(q_lens[n_dec:]), scale, window)
         else:
-            paged_attention_prefill_tc(q, cache.k_pool, cache.v_pool, out, table, cu_q, kv_len, prefill_tc_tiles(q_lens),
-                                       scale, window)
+            paged_attention_prefill_tc(q, cache.k_pool, cache.v_pool, out, table[n_dec:], cu_q[n_dec:], kv_len[n_dec:],
+                                       prefill_tc_tiles(q_lens[n_dec:]), scale, window)
+        if beside:
+            decode(True)
         return
     paged_attention_generic(q, cache.k_pool, cache.v_pool, out, cache.block_table, ctx.cu_q, ctx.kv_len,
                             ctx.seq_of_token, scale, window)
