@@ -17,7 +17,8 @@
 // Every row is worked on by up to 32 blocks (a vocabulary of 150 thousand is 600 KB per row): one
 // kernel for the slices' maxima and sums, three for the histograms (each block first reads the
 // levels above it and decides their bins again, the same way), one for the survivors' masses per
-// slice, whose last block per row draws the token.
+// slice, whose last block per row draws the token.  A row of one slice (up to 2,048 tokens) needs no other block: one kernel
+// takes all the steps, in the same order and with the same sums.
 #include "common.cuh"
 
 #include <climits>
@@ -92,11 +93,12 @@ __device__ __forceinline__ void row_softmax(const float2* part, int slices, floa
     inv_z = 1.0f / z;
 }
 
+// part: the row's slices.
 __device__ __forceinline__ RowParams row_params(int r, const float2* part, int slices, int vocab, const float* temperature,
                                                 const int* top_k, const float* top_p) {
     RowParams p;
     p.inv_t = 1.0f / temperature[r];
-    row_softmax(part + (size_t)r * slices, slices, p.inv_t, p.m, p.inv_z);
+    row_softmax(part, slices, p.inv_t, p.m, p.inv_z);
     p.k = top_k ? top_k[r] : 0;
     const float tp = top_p ? top_p[r] : 1.0f;
     p.use_k = p.k > 0 && p.k < vocab;
@@ -164,16 +166,8 @@ __device__ __forceinline__ void slice_range(int vocab, int slices, int slice, in
     end = min(vocab, begin + per);
 }
 
-__global__ void __launch_bounds__(kSampleThreads)
-sample_stats_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature, SampleWork w) {
-    __shared__ float scratch[32];
-    const int r = blockIdx.y, slices = gridDim.x;
-    const float temp = temperature[r];
-    if (!(temp > 0.0f)) return;
-    const float inv_t = 1.0f / temp;
-    const float* row = logits + (size_t)r * vocab;
-    int begin, end;
-    slice_range(vocab, slices, blockIdx.x, begin, end);
+// Maximum of row[begin, end) and the sum of exp((x - maximum) / T); all threads of the block call it, scratch: 32 floats.
+__device__ __forceinline__ float2 slice_stats(const float* row, int begin, int end, float inv_t, float* scratch) {
     float m = -INFINITY;
     for (int i = begin + threadIdx.x; i < end; i += kSampleThreads) m = fmaxf(m, row[i]);
     m = warp_max(m);
@@ -186,7 +180,65 @@ sample_stats_kernel(const float* __restrict__ logits, int vocab, const float* __
     if (m > -INFINITY)
         for (int i = begin + threadIdx.x; i < end; i += kSampleThreads) z += expf((row[i] - m) * inv_t);
     z = block_sum(z, scratch);
-    if (threadIdx.x == 0) w.part[(size_t)r * slices + blockIdx.x] = make_float2(m, z);
+    return make_float2(m, z);
+}
+
+// The tokens of row[begin, end) whose probability's higher bits equal `prefix` (level 0: all) into the histogram of the level's bits.
+__device__ __forceinline__ void add_to_bins(const float* row, int begin, int end, const RowParams& p, int level, unsigned int prefix,
+                                            unsigned int* h_cnt, unsigned long long* h_mass) {
+    const int shift = 10 * (kLevels - 1 - level);
+    for (int i = begin + threadIdx.x; i < end; i += kSampleThreads) {
+        const float q = prob(row[i], p);
+        const unsigned int key = __float_as_uint(q);
+        if (level == 0 || (key >> (shift + 10)) == prefix) {
+            const unsigned int bin = (key >> shift) & (kBins - 1);
+            atomicAdd(&h_cnt[bin], 1u);
+            atomicAdd(&h_mass[bin], (unsigned long long)(q * kMassScale));
+        }
+    }
+}
+
+// How many of the tokens whose probability EQUALS the threshold survive, the first ones in index order: a sort keeps exactly k
+// tokens and the nucleus rule looks at the mass strictly before each token (pulsar-core/src/runtime/sampler.cpp:30-40), so equal
+// probabilities at the cut are not all in or all out.  carried_*: count and mass of what lies strictly above it.
+__device__ __forceinline__ int survivors_at(float threshold, const RowParams& p, unsigned int carried_cnt, unsigned long long carried_mass) {
+    int allow = INT_MAX;
+    if (p.use_k) allow = p.k - (int)carried_cnt;
+    if (p.use_p) {
+        const unsigned long long each = (unsigned long long)(threshold * kMassScale);
+        const unsigned long long room = p.tp_q >= carried_mass ? p.tp_q - carried_mass : 0;
+        const unsigned long long by_mass = each > 0 ? room / each + 1 : (unsigned long long)INT_MAX;
+        if (by_mass < (unsigned long long)allow) allow = (int)by_mass;
+    }
+    return allow < 1 ? 1 : allow;
+}
+
+// Of one thread's range row[b0, e0): the token at which the cumulative mass, `run` before it, passes the target, the last survivor
+// where none does, -1 without one.  ties: tokens at the threshold before the range.
+__device__ __forceinline__ int pick_in_range(const float* row, int b0, int e0, const RowParams& p, float threshold, int allow, float target,
+                                             float run, int ties) {
+    int last = -1;
+    for (int i = b0; i < e0; ++i) {
+        const float q = prob(row[i], p);
+        if (q > threshold || (q == threshold && ties++ < allow)) {
+            last = i;
+            run += q;
+            if (target < run) return i;
+        }
+    }
+    return last;
+}
+
+__global__ void __launch_bounds__(kSampleThreads)
+sample_stats_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature, SampleWork w) {
+    __shared__ float scratch[32];
+    const int r = blockIdx.y, slices = gridDim.x;
+    const float temp = temperature[r];
+    if (!(temp > 0.0f)) return;
+    int begin, end;
+    slice_range(vocab, slices, blockIdx.x, begin, end);
+    const float2 part = slice_stats(logits + (size_t)r * vocab, begin, end, 1.0f / temp, scratch);
+    if (threadIdx.x == 0) w.part[(size_t)r * slices + blockIdx.x] = part;
 }
 
 // Level L (0 = the highest ten bits): histogram of the probabilities whose higher bits equal the bins picked above.
@@ -201,7 +253,7 @@ sample_hist_kernel(const float* __restrict__ logits, int rows, int vocab, const 
     __shared__ int s_pick;
     const int r = blockIdx.y, slices = gridDim.x;
     if (!(temperature[r] > 0.0f)) return;
-    const RowParams p = row_params(r, w.part, slices, vocab, temperature, top_k, top_p);
+    const RowParams p = row_params(r, w.part + (size_t)r * slices, slices, vocab, temperature, top_k, top_p);
     if (!p.use_k && !p.use_p) return;
     unsigned int carried_cnt = 0;
     unsigned long long carried_mass = 0;
@@ -214,19 +266,9 @@ sample_hist_kernel(const float* __restrict__ logits, int rows, int vocab, const 
     }
     for (int i = threadIdx.x; i < kBins; i += kSampleThreads) { h_cnt[i] = 0; h_mass[i] = 0; }
     __syncthreads();
-    const float* row = logits + (size_t)r * vocab;
     int begin, end;
     slice_range(vocab, slices, blockIdx.x, begin, end);
-    constexpr int kShift = 10 * (kLevels - 1 - LEVEL);
-    for (int i = begin + threadIdx.x; i < end; i += kSampleThreads) {
-        const float q = prob(row[i], p);
-        const unsigned int key = __float_as_uint(q);
-        if (LEVEL == 0 || (key >> (kShift + 10)) == prefix) {
-            const unsigned int bin = (key >> kShift) & (kBins - 1);
-            atomicAdd(&h_cnt[bin], 1u);
-            atomicAdd(&h_mass[bin], (unsigned long long)(q * kMassScale));
-        }
-    }
+    add_to_bins(logits + (size_t)r * vocab, begin, end, p, LEVEL, prefix, h_cnt, h_mass);
     __syncthreads();
     const size_t at = ((size_t)LEVEL * rows + r) * kBins;
     for (int i = threadIdx.x; i < kBins; i += kSampleThreads)
@@ -250,11 +292,8 @@ sample_draw_kernel(const float* __restrict__ logits, int rows, int vocab, const 
     __shared__ Best best_s[32];
     const int r = blockIdx.y, slices = gridDim.x;
     if (!(temperature[r] > 0.0f)) return;
-    const RowParams p = row_params(r, w.part, slices, vocab, temperature, top_k, top_p);
-    // threshold: the smallest surviving probability.  allow: how many of the tokens whose probability EQUALS it
-    // survive, the first ones in index order: a sort keeps exactly k tokens and the nucleus rule looks at the mass
-    // strictly before each token (pulsar-core/src/runtime/sampler.cpp:30-40), so equal probabilities at the cut are
-    // not all in or all out.
+    const RowParams p = row_params(r, w.part + (size_t)r * slices, slices, vocab, temperature, top_k, top_p);
+    // threshold: the smallest surviving probability
     float threshold = 0.0f;
     int allow = INT_MAX;
     if (p.use_k || p.use_p) {
@@ -265,15 +304,7 @@ sample_draw_kernel(const float* __restrict__ logits, int rows, int vocab, const 
             bits = (bits << 10) | (unsigned int)pick_bin(w.cnt + at, w.mass + at, p, carried_cnt, carried_mass, s_cnt, s_mass, &s_pick);
         }
         threshold = __uint_as_float(bits);
-        // carried_*: count and mass of what lies strictly above the threshold (fewer than k, mass <= top_p)
-        if (p.use_k) allow = p.k - (int)carried_cnt;
-        if (p.use_p) {
-            const unsigned long long each = (unsigned long long)(threshold * kMassScale);
-            const unsigned long long room = p.tp_q >= carried_mass ? p.tp_q - carried_mass : 0;
-            const unsigned long long by_mass = each > 0 ? room / each + 1 : (unsigned long long)INT_MAX;
-            if (by_mass < (unsigned long long)allow) allow = (int)by_mass;
-        }
-        if (allow < 1) allow = 1;
+        allow = survivors_at(threshold, p, carried_cnt, carried_mass);
     }
     const float* row = logits + (size_t)r * vocab;
     // thread t owns a contiguous range of the slice's indices.  ``ties_before``: tokens at the threshold in the
@@ -318,18 +349,7 @@ sample_draw_kernel(const float* __restrict__ logits, int rows, int vocab, const 
         int ties = (int)s_cnt[threadIdx.x];
         const float my_mass = mine + (float)max(0, min(my_ties, allow - min(ties, allow))) * threshold;
         if (my_mass > 0.0f && target >= before && target < before + my_mass) {
-            float run = before;
-            int chosen = -1, last = -1;
-            for (int i = b0; i < e0; ++i) {
-                const float q = prob(row[i], p);
-                const bool in = q > threshold || (q == threshold && ties++ < allow);
-                if (in) {
-                    last = i;
-                    run += q;
-                    if (target < run) { chosen = i; break; }
-                }
-            }
-            s_pick = chosen >= 0 ? chosen : last;
+            s_pick = pick_in_range(row, b0, e0, p, threshold, allow, target, before, ties);
         }
         __syncthreads();
         return s_pick;
@@ -372,6 +392,89 @@ sample_draw_kernel(const float* __restrict__ logits, int rows, int vocab, const 
         out[r] = pick;
         w.tickets[r] = 0;
     }
+}
+
+// A row of one slice, all steps in one block: what the kernels above do with slices = 1, the same sums in the same order.  Bound by
+// the chain of its steps: 6 rows of 336 tokens 11.1 us (the five kernels 35.0), 8 rows of 2,048 15.5 (39.8).
+__global__ void __launch_bounds__(kSampleThreads)
+sample_row_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature, const int* __restrict__ top_k,
+                  const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+    __shared__ unsigned int h_cnt[kBins];
+    __shared__ unsigned long long h_mass[kBins];
+    __shared__ unsigned int s_cnt[kSampleThreads];
+    __shared__ unsigned long long s_mass[kSampleThreads];
+    __shared__ float scan_s[kSampleThreads], scratch[32];
+    __shared__ int s_pick;
+    __shared__ float s_total;
+    __shared__ Best best_s[32];
+    const int r = blockIdx.x, t = threadIdx.x;
+    const float temp = temperature[r];
+    if (!(temp > 0.0f)) return;
+    const float* row = logits + (size_t)r * vocab;
+    const float2 part = slice_stats(row, 0, vocab, 1.0f / temp, scratch);
+    const RowParams p = row_params(r, &part, 1, vocab, temperature, top_k, top_p);
+    float threshold = 0.0f;
+    int allow = INT_MAX;
+    if (p.use_k || p.use_p) {
+        unsigned int carried_cnt = 0, bits = 0;
+        unsigned long long carried_mass = 0;
+        for (int l = 0; l < kLevels; ++l) {
+            for (int i = t; i < kBins; i += kSampleThreads) { h_cnt[i] = 0; h_mass[i] = 0; }
+            __syncthreads();
+            add_to_bins(row, 0, vocab, p, l, bits, h_cnt, h_mass);
+            __syncthreads();
+            bits = (bits << 10) | (unsigned int)pick_bin(h_cnt, h_mass, p, carried_cnt, carried_mass, s_cnt, s_mass, &s_pick);
+        }
+        threshold = __uint_as_float(bits);
+        allow = survivors_at(threshold, p, carried_cnt, carried_mass);
+    }
+    const int per = (vocab + kSampleThreads - 1) / kSampleThreads;
+    const int b0 = min(vocab, t * per), e0 = min(vocab, b0 + per);
+    float mine = 0.0f;
+    int my_ties = 0;
+    for (int i = b0; i < e0; ++i) {
+        const float q = prob(row[i], p);
+        if (q > threshold) mine += q;
+        else if (q == threshold) ++my_ties;
+    }
+    __syncthreads();
+    scan_s[t] = mine;
+    s_cnt[t] = (unsigned int)my_ties;
+    __syncthreads();
+    if (t == 0) {      // serial sums over the threads: all above the threshold, and the cumulative mass with the ties that survive
+        float above = 0.0f, run = 0.0f;
+        int ties = 0;
+        for (int k = 0; k < kSampleThreads; k += 8) {
+            float v[8];
+            int n[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { v[e] = scan_s[k + e]; n[e] = (int)s_cnt[k + e]; }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int in = max(0, min(n[e], allow - min(ties, allow)));
+                scan_s[k + e] = run;
+                s_cnt[k + e] = (unsigned int)ties;             // ties before the thread's range
+                above += v[e] + 0.0f * threshold;
+                run += v[e] + (float)in * threshold;
+                ties += n[e];
+            }
+        }
+        // (the mass above travels through 32 bits between the kernels above as it does here)
+        s_total = 0.0f + (above + (float)max(0, min(ties, allow)) * threshold);
+        s_pick = -1;
+    }
+    __syncthreads();
+    const float total = s_total, target = uniform[r] * total, before = scan_s[t];
+    if (total > 0.0f && target < total) {
+        const int ties = (int)s_cnt[t];
+        const float my_mass = mine + (float)max(0, min(my_ties, allow - min(ties, allow))) * threshold;
+        if (my_mass > 0.0f && target >= before && target < before + my_mass)
+            s_pick = pick_in_range(row, b0, e0, p, threshold, allow, target, before, ties);
+    }
+    __syncthreads();
+    int pick = s_pick;
+    if (pick < 0) pick = block_argmax(row, vocab, best_s);      // rounding left the target past the last survivor
+    if (t == 0) out[r] = pick;
 }
 
 // Greedy rows over many blocks: every block reduces a slice of the row to (value, index) and
@@ -457,6 +560,10 @@ PB_EXPORT int pb_sample(const float* logits, int rows, int vocab, const float* t
     }
     int slices = (vocab + 2047) / 2048;
     if (slices > kMaxSlices) slices = kMaxSlices;
+    if (slices == 1) {
+        sample_row_kernel<<<rows, kSampleThreads, 0, stream>>>(logits, vocab, temperature, top_k, top_p, uniform, out);
+        return launch_status();
+    }
     SampleWork w;
     unsigned char* at = static_cast<unsigned char*>(workspace);
     w.mass = reinterpret_cast<unsigned long long*>(at);

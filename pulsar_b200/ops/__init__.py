@@ -335,6 +335,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, loaded: bool 
 
 _argmax_keys = {}
 _sample_work = {}
+_ONE_BLOCK_VOCAB = 2048           # rows this long are one block's work, in one kernel (csrc/sampling.cu)
 
 
 def sample(logits: torch.Tensor, out: torch.Tensor, temperature: Optional[torch.Tensor] = None,
@@ -363,7 +364,7 @@ def sample(logits: torch.Tensor, out: torch.Tensor, temperature: Optional[torch.
         work = _sample_work[logits.device] = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=logits.device)
     filtered = top_k is not None or top_p is not None
     check(fn("pb_sample")(_p(logits), rows, vocab, _p(temperature), _p(top_k), _p(top_p), _p(uniform), 1 if any_greedy else 0,
-                          _p(work), _p(keys), _p(out), stream()), "sample", kernels=(2 if any_greedy else 0) + (5 if filtered else 2))
+                          _p(work), _p(keys), _p(out), stream()), "sample", kernels=(2 if any_greedy else 0) + (1 if vocab <= _ONE_BLOCK_VOCAB else 5 if filtered else 2))
 
 
 class _Gating:
