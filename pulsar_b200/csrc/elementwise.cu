@@ -527,6 +527,12 @@ PB_EXPORT int pb_embed(int dtype, const void* table, const int* ids, float* out,
     return launch_status();
 }
 
+// A copy between the host's pinned memory and the device (either way), in the stream.
+PB_EXPORT int pb_copy(void* dst, const void* src, long long bytes, cudaStream_t stream) {
+    if (bytes <= 0) return bytes == 0 ? 0 : PB_ERR_BAD_SIZE;
+    return (int)cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDefault, stream);
+}
+
 PB_EXPORT int pb_add_rmsnorm(int dtype, float* residual, const void* delta, const float* weight, void* out,
                              const int* rows, int n_out, int width, float eps, int write_back, cudaStream_t stream) {
     if (n_out <= 0) return 0;

@@ -16,7 +16,7 @@ import torch
 from .. import ops, profiling
 from ..cache.manager import CacheManager
 from ..config.engine_config import EngineConfig
-from ..sampling.sampler import GenerationParams, Sampler, make_generator
+from ..sampling.sampler import GenerationParams, Sampler, draw_uniform, make_generator
 from .loading import load_model, torch_dtype
 from .runner import ModelRunner, StepEntry
 from .scheduler import UNREAD, Scheduled, Scheduler, SchedulerError
@@ -31,6 +31,14 @@ class _Session:
     state: str = "idle"           # "idle", "active", "parked"
     scheduled: bool = False       # known to the scheduler
     ended_on_stop: bool = False   # the last turn ended with the stop token
+    redraw: Optional[float] = None      # a number whose draw turned out void: the next draw gives it again
+
+    def draw(self) -> float:
+        """The next uniform number of the request's own generator."""
+        if self.redraw is not None:
+            u, self.redraw = self.redraw, None
+            return u
+        return draw_uniform(self.generator)
 
 
 class EngineFailed(RuntimeError):
@@ -46,7 +54,7 @@ class _Inflight:
     row_of: Dict[int, int]
     host: torch.Tensor                     # pinned; filled when ``event`` has passed
     event: torch.cuda.Event
-    generator_states: Dict[int, torch.Tensor]      # of stochastic sequences, before their draw
+    uniform: List[float]                   # what each row drew (0.0 for greedy sequences)
     status: Optional[torch.Tensor] = None          # pinned; the kernels' wait error words behind this pass
     void: set = field(default_factory=set)         # sequences that had ended before this pass: its token is dropped
 
@@ -103,9 +111,7 @@ class Engine:
         self._mailbox: Dict[int, list] = {}     # events of other sessions seen while one session streams
         self._inflight: Optional[_Inflight] = None          # the pass whose tokens have not been read yet
         self._unclaimed: List[Tuple[int, int, bool]] = []   # events booked outside ``step``
-        self._host_ids: List[Optional[torch.Tensor]] = [None, None, None]
-        self._host_status = [torch.zeros(8, dtype=torch.int32, pin_memory=True) for _ in self._host_ids]
-        self._status_dev = torch.zeros(8, dtype=torch.int32, device=cfg.device)
+        self._host_report: List[Optional[torch.Tensor]] = [None, None, None]      # pinned: error words, then sampled ids
         self._host_next = 0
         self._failed: Optional[BaseException] = None
 
@@ -248,25 +254,23 @@ class Engine:
         self.scheduler.on_step(plan)
         sampled = [e.rid for e in plan if e.sample]
         sessions = [self._sessions[r] for r in sampled]
-        states = {r: s.generator.get_state() for r, s in zip(sampled, sessions) if not s.params.greedy}
+        uniform = [0.0 if s.params.greedy else s.draw() for s in sessions]
         with profiling.scope("launch (sampling)"):
-            ids = self.sampler.sample_on_device(logits, [s.params for s in sessions], [s.generator for s in sessions])
-        slot = self._host_ids[self._host_next]
-        if slot is None or slot.numel() < len(sampled):
-            slot = self._host_ids[self._host_next] = torch.empty(max(64, len(sampled)), dtype=torch.int32, pin_memory=True)
-        status = self._host_status[self._host_next]
-        self._host_next = (self._host_next + 1) % len(self._host_ids)
-        host = slot[:len(sampled)]
-        if sampled:
-            host.copy_(ids, non_blocking=True)
-        # the error words of the kernels with bounded waits travel with the ids: no synchronisation of their own
-        ops.gather_wait_words(self._status_dev)
-        status.copy_(self._status_dev, non_blocking=True)
+            self.sampler.sample_on_device(logits, [s.params for s in sessions], (), uniform)
+        # the error words of the kernels with bounded waits travel with the ids, in one copy: no synchronisation of their own
+        ops.gather_wait_words(self.sampler.head)
+        n_words = Sampler.HEAD + len(sampled)
+        slot = self._host_report[self._host_next]
+        if slot is None or slot.numel() < n_words:
+            slot = self._host_report[self._host_next] = torch.zeros(max(Sampler.HEAD + 64, n_words), dtype=torch.int32, pin_memory=True)
+        self._host_next = (self._host_next + 1) % len(self._host_report)
+        ops.copy_pinned(slot, self.sampler.report(len(sampled)), n_words)
+        status, host = slot[:Sampler.HEAD], slot[Sampler.HEAD:n_words]
         event = torch.cuda.Event()
-        event.record()
+        event.record(ops.current_stream())
         for r in sampled:
             self.scheduler.on_sampled(r)
-        return _Inflight(sampled, {r: i for i, r in enumerate(sampled)}, host, event, states, status)
+        return _Inflight(sampled, {r: i for i, r in enumerate(sampled)}, host, event, uniform, status)
 
     def _collect(self, flight: "_Inflight") -> List[Tuple[int, int, bool]]:
         """Wait for a pass's sampled ids and book them: events ``(seq_id, token, finished)``."""
@@ -286,8 +290,8 @@ class Engine:
             if rid in flight.void:
                 # the sequence had ended with the token before: this pass only cached that token
                 self.scheduler.drop_unread(rid)
-                if rid in flight.generator_states and rid in self._sessions:
-                    self._sessions[rid].generator.set_state(flight.generator_states[rid])
+                if rid in self._sessions and not self._sessions[rid].params.greedy:
+                    self._sessions[rid].redraw = flight.uniform[flight.row_of[rid]]
                 continue
             finished = self.scheduler.on_token(rid, tok, self.eos_id)
             if finished:

@@ -150,6 +150,8 @@ class ModelRunner:
         if not entries:
             raise StepError("a step needs at least one entry")
         seen = set()
+        q_lens, flat_tokens, want_counts, flat_wants, sources = [], [], [], [], []       # of all entries, side by side
+        moved = False
         for e in entries:
             if e.rid in seen:
                 raise StepError(f"request {e.rid!r} appears twice in one step")
@@ -157,7 +159,7 @@ class ModelRunner:
             n_tok = len(e.tokens)
             if n_tok == 0:
                 raise StepError(f"request {e.rid!r}: a step entry needs at least one token")
-            if min(e.tokens) < 0 or max(e.tokens) >= self.vocab:
+            if not (0 <= e.tokens[0] < self.vocab) if n_tok == 1 else min(e.tokens) < 0 or max(e.tokens) >= self.vocab:
                 bad = [t for t in e.tokens if not (0 <= int(t) < self.vocab)][0]
                 raise StepError(f"request {e.rid!r}: token id {bad} outside the vocabulary [0, {self.vocab})")
             if e.token_src is not None and (n_tok != 1 or sampled_ids is None or not (0 <= e.token_src < sampled_ids.numel())):
@@ -170,6 +172,15 @@ class ModelRunner:
             if len(e.want) and (min(e.want) < 0 or max(e.want) >= n_tok):
                 bad = [w for w in e.want if not (0 <= int(w) < n_tok)][0]
                 raise StepError(f"request {e.rid!r}: wanted index {bad} outside its {n_tok} tokens")
+            q_lens.append(n_tok)
+            flat_tokens.extend(map(int, e.tokens))
+            want_counts.append(len(e.want))
+            flat_wants.extend(map(int, e.want))
+            if e.token_src is None:
+                sources.append(-1)
+            else:
+                sources.append(int(e.token_src))
+                moved = True
         # The host runtime checks the whole step's pages and slots before anything changes, grows the
         # requests, and writes the step's index arrays into one pinned buffer:
         # token_ids, positions, seq_of_token [N]; cu_q [S+1]; kv_len, state_slots [S]; logit_rows [R];
@@ -178,19 +189,16 @@ class ModelRunner:
         n_groups = len(cache.groups)
         fresh = [e.rid for e in entries if not cache.has(e.rid)]
         rids = host.longs([cache.native_id(e.rid, create=True) for e in entries])
-        q_lens = [len(e.tokens) for e in entries]
-        n = sum(q_lens)
-        flat_tokens = [int(t) for e in entries for t in e.tokens]
-        flat_wants = [int(w) for e in entries for w in e.want]
-        n_tok, want_n = host.ints(q_lens), host.ints([len(e.want) for e in entries])
+        n = len(flat_tokens)
+        n_tok, want_n = host.ints(q_lens), host.ints(want_counts)
         tokens, wants = host.ints(flat_tokens), host.ints(flat_wants or [0])
-        token_src = host.ints([-1 if e.token_src is None else int(e.token_src) for e in entries])
-        starts, slots = (ctypes.c_int * s)(), (ctypes.c_int * s)()
+        token_src = host.ints(sources)
+        starts_c, slots_c = (ctypes.c_int * s)(), (ctypes.c_int * s)()
         widths_c, bad = (ctypes.c_int * max(1, n_groups))(), ctypes.c_int(-1)
         lib, handle = cache._lib, cache._h
         total = lib.ph_step_plan(handle, s, rids, n_tok, tokens, want_n, wants, token_src,
                                  0 if sampled_ids is None else int(sampled_ids.numel()), self.vocab, self.TABLE_BUCKET,
-                                 starts, slots, widths_c, ctypes.byref(bad))
+                                 starts_c, slots_c, widths_c, ctypes.byref(bad))
         if total < 0:
             for rid in fresh:
                 cache._forget_if_idle(rid)
@@ -204,7 +212,7 @@ class ModelRunner:
             raise StepError(f"the host runtime refused the step (code {total}, entry of request {who!r})")
         for rid in fresh:
             cache.opened_by_runtime(rid)
-        starts, state_slots = list(starts), list(slots)
+        starts, state_slots = list(starts_c), list(slots_c)
         kv_lens = [st + q for st, q in zip(starts, q_lens)]
         host_batch = HostBatch(q_lens, kv_lens, state_slots)
         ctx = StepContext(self, n, s, host_batch)
@@ -213,12 +221,11 @@ class ModelRunner:
         ctx.table_widths = tuple(widths)
         if ctx.uneven:
             ctx.uneven = ctx.all_decode and ops.unevenness_matters(s, [(heads, widths[g] * cache.page_size) for g, heads in self._sharing])
-        moved = any(e.token_src is not None for e in entries)
         n_arrays = 7 + 2 * n_groups + (2 if moved else 0)
         offsets_c, lengths_c = (ctypes.c_int * n_arrays)(), (ctypes.c_int * n_arrays)()
         stage = self._stage(total)
-        rc = lib.ph_step_pack(handle, s, rids, n_tok, tokens, want_n, wants, token_src, (ctypes.c_int * s)(*starts),
-                              (ctypes.c_int * s)(*state_slots), widths_c, stage.data_ptr(), stage.numel(), offsets_c, lengths_c)
+        rc = lib.ph_step_pack(handle, s, rids, n_tok, tokens, want_n, wants, token_src, starts_c, slots_c, widths_c,
+                              stage.data_ptr(), stage.numel(), offsets_c, lengths_c)
         if rc == host.RELEASED_PAGE:
             raise StepError("a position of the step lies in a released page")
         if rc != total:
@@ -229,12 +236,12 @@ class ModelRunner:
             self.scratch_epoch += 1
             self._views.clear()
         dev = self._index_buf
-        dev[:total].copy_(stage[:total], non_blocking=True)
+        ops.copy_pinned(dev, stage, total)
         self.h2d_bytes += total * 4
         ev = self._staging_events[self._staging_slot]
         if ev is None:
             ev = self._staging_events[self._staging_slot] = torch.cuda.Event()
-        ev.record()
+        ev.record(ops.current_stream())
 
         # Views of the device buffer; steady decoding has the same layout every step, so they are kept.
         key = (tuple(lengths), tuple(widths))
@@ -280,8 +287,12 @@ class ModelRunner:
         ``want`` lists.  The tensor is scratch memory: it is valid until the next step."""
         with profiling.scope("pack (index arrays, pages, one copy)"):
             ctx = self.prepare(entries, sampled_ids)
-        with profiling.scope("launch (the model's kernels)"), torch.cuda.device(self.device):
-            logits = self._forward(ctx)
+        with profiling.scope("launch (the model's kernels)"):
+            if torch.cuda.current_device() == self.device.index:
+                logits = self._forward(ctx)
+            else:
+                with torch.cuda.device(self.device):
+                    logits = self._forward(ctx)
         self.steps_run += 1
         return logits
 

@@ -17,7 +17,7 @@ import atexit
 import os
 import sys
 import time
-from contextlib import contextmanager
+from contextlib import contextmanager, nullcontext
 from typing import Dict, List, Tuple
 
 ENABLED = os.environ.get("PULSAR_PROF", "0") not in ("", "0")
@@ -69,12 +69,16 @@ def timed_launcher(name: str, f):
     return call
 
 
-@contextmanager
+_NOT_TIMED = nullcontext()
+
+
 def scope(name: str):
     """Host wall-clock time of a phase."""
-    if not ENABLED:
-        yield
-        return
+    return _timed_scope(name) if ENABLED else _NOT_TIMED
+
+
+@contextmanager
+def _timed_scope(name: str):
     t0 = time.perf_counter()
     try:
         yield

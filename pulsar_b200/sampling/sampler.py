@@ -15,6 +15,7 @@ what else is in the batch.
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
@@ -52,32 +53,71 @@ def make_generator(seed: int) -> torch.Generator:
     return g
 
 
+def draw_uniform(generator: torch.Generator) -> float:
+    return torch.rand(1, generator=generator).item()
+
+
 class Sampler:
+    HEAD = 8
+
     def __init__(self, device):
         self.device = torch.device(device)
-        self._ids: Optional[torch.Tensor] = None
+        # [HEAD words for whoever reads the ids back | the ids]: one copy brings both
+        self._report = torch.zeros(self.HEAD + 64, dtype=torch.int32, device=self.device)
         self.last_ids: Optional[torch.Tensor] = None      # what the last call returned
+        # The rows' parameters travel in one copy from pinned memory, one buffer for each of the last calls: (the memory, the same
+        # as C floats and as C ints, the event behind its last copy).
+        self._staging: List[Optional[tuple]] = [None] * 4
+        self._staging_next = 0
+
+    def report(self, rows: int) -> torch.Tensor:
+        """The head words and the ids of the last call's ``rows`` rows, on the device."""
+        return self._report[:self.HEAD + rows]
+
+    @property
+    def head(self) -> torch.Tensor:
+        return self._report[:self.HEAD]
+
+    def _on_device(self, params: Sequence[GenerationParams], uniform: List[float]) -> torch.Tensor:
+        """float32 [4, rows] on the device: temperatures, top_p, uniform numbers, and the bits of the int32 top_k."""
+        rows, i = len(params), self._staging_next
+        self._staging_next = (i + 1) % len(self._staging)
+        slot = self._staging[i]
+        if slot is not None:
+            slot[3].synchronize()             # the copy out of this buffer, some calls ago
+        if slot is None or slot[0].numel() < 4 * rows:
+            buf = torch.empty(4 * max(rows, 64), dtype=torch.float32, pin_memory=True)
+            at = buf.data_ptr()
+            slot = self._staging[i] = (buf, (ctypes.c_float * buf.numel()).from_address(at), (ctypes.c_int * buf.numel()).from_address(at),
+                                       torch.cuda.Event())
+        buf, floats, ints, event = slot
+        floats[:3 * rows] = [p.temperature for p in params] + [p.top_p for p in params] + uniform
+        ints[3 * rows:4 * rows] = [p.top_k for p in params]
+        out = torch.empty((4, rows), dtype=torch.float32, device=self.device)
+        ops.copy_pinned(out, buf, 4 * rows)
+        event.record(ops.current_stream())
+        return out
 
     def sample_on_device(self, logits: torch.Tensor, params: Sequence[GenerationParams],
-                         generators: Sequence[Optional[torch.Generator]]) -> torch.Tensor:
+                         generators: Sequence[Optional[torch.Generator]], uniform: Optional[List[float]] = None) -> torch.Tensor:
         """One token id per row of ``logits`` (float32 [R, V] on the device), left on the device:
-        an int32 tensor that stays valid until the next call."""
+        an int32 tensor that stays valid until the next call.  ``uniform``: the rows' uniform numbers (0.0 for greedy rows), where
+        the caller has drawn them already."""
         rows = logits.shape[0]
-        assert len(params) == rows and len(generators) == rows
-        if self._ids is None or self._ids.numel() < rows:
-            self._ids = torch.empty(max(rows, 64), dtype=torch.int32, device=self.device)
-        out = self._ids[:rows]
+        assert len(params) == rows and (len(generators) == rows if uniform is None else len(uniform) == rows)
+        if self._report.numel() < self.HEAD + rows:
+            self._report = torch.zeros(self.HEAD + rows, dtype=torch.int32, device=self.device)
+        out = self._report[self.HEAD:self.HEAD + rows]
         self.last_ids = out
         if rows == 0:
             return out
         if all(p.greedy for p in params):
             ops.sample(logits, out)
         else:
-            uniform = [0.0 if p.greedy else float(torch.rand(1, generator=g).item()) for p, g in zip(params, generators)]
-            packed = torch.tensor([[p.temperature for p in params], [p.top_p for p in params], uniform],
-                                  dtype=torch.float32).to(self.device, non_blocking=True)
-            top_k = torch.tensor([p.top_k for p in params], dtype=torch.int32).to(self.device, non_blocking=True)
-            ops.sample(logits, out, packed[0], top_k, packed[1], packed[2], any_greedy=any(p.greedy for p in params))
+            if uniform is None:
+                uniform = [0.0 if p.greedy else draw_uniform(g) for p, g in zip(params, generators)]
+            temperature, top_p, drawn, top_k = self._on_device(params, uniform).unbind(0)
+            ops.sample(logits, out, temperature, top_k.view(torch.int32), top_p, drawn, any_greedy=any(p.greedy for p in params))
         return out
 
     def sample(self, logits: torch.Tensor, params: Sequence[GenerationParams],
