@@ -23,20 +23,25 @@ using namespace pb;
 // ---------------------------------------------------------------- up to 16 rows
 // Bound by reading W once, and with more rows of A by shared memory.  The sums stay chains in ascending k: a chain takes 4 cycles
 // a step, so 128 blocks of 32 weight rows ask for 8 TB/s, above what HBM gives, and a split of K (which would change the sums)
-// is not needed.  W and A come through shared memory in stages of 64 k by 16-byte asynchronous copies of four warps that do
-// nothing else; CW further warps compute, a thread R rows of W times T rows of A.  A loaded W depends on no earlier kernel: its first
+// is not needed.  W and A come through shared memory in stages of RK k by 16-byte asynchronous copies of four warps that do
+// nothing else; CW further warps compute, a thread R rows of W times T rows of A.  Between two stages stands a barrier of the block, and
+// behind it a wait for shared memory that nothing covers (150 cycles together, against the 256 of 64 k's chain): long stages.  (A
+// warp that copies its own rows needs no barrier, but its copies then stand between its chains: 33 us for 4096 x 4096.)
+// A loaded W depends on no earlier kernel: its first
 // stages are asked for before griddepcontrol.wait (a W that may just have been computed: the ordinary launch, which begins behind
 // it).  A 16-byte read of shared memory costs a warp 4 cycles, 2 where neighbouring lanes read the same place (measured), so lanes
-// that share a row of W stand side by side; W's rows stand 68 floats apart, which keeps the others off each other's banks.
-// us on the sizes of an 8B layer, 64 x 64 tiles of the general kernel before: 6144 x 4096 1 row 21.7 (was 277), 4 rows 27.2, 8 rows
-// 36.7, 16 rows 63; 4096 x 4096 19.3 / 21.6 / 27.4 / 47 (282); 24576 x 4096 66.8 / 74.8 / 103 / 188 (480); 4096 x 12288
-// 43.7 / 50.8 / 69 / 120 (851); 151936 x 4096 376 (6.6 TB/s) / 406 / 562 / 1055.
-constexpr int RN = 32, RK = 64, RSTRIDE = RK + 4, RLOAD = 128;
+// that share a row of W stand side by side; W's rows stand four floats more than a multiple of 32 apart, which keeps the others off each
+// other's banks.
+// us on the sizes of an 8B layer (64 x 64 tiles of the general kernel): 6144 x 4096 1 row 19.8 (277), 4 rows 24.4, 8 rows
+// 29.6, 16 rows 58; 4096 x 4096 15.1 / 17.7 / 23.2 / 38.5 (282); 24576 x 4096 64 / 69 / 86 / 174 (480); 4096 x 12288
+// 39.5 / 45.8 / 59.3 / 108 (851); 151936 x 4096 375 (6.6 TB/s) / 387 / 466 to 509 / 969.
+constexpr int RN = 32, RLOAD = 128;
 
-template <int R, int T, int CW, int RST, typename TO>
+template <int R, int T, int CW, int RST, int RK, typename TO>
 __global__ void __launch_bounds__(RLOAD + 32 * CW)
 simt_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out, int M, int N, int K) {
     extern __shared__ __align__(16) float rows_smem[];
+    constexpr int RSTRIDE = RK + 4;
     constexpr int LR = RN / R, LT = 32 / LR, MR = LT * T * CW;      // lanes along the rows of W, along those of A; rows of A held
     float* ws = rows_smem;                                  // [RST][RN][RSTRIDE]
     float* as = ws + RST * RN * RSTRIDE;                    // [RST][MR][RK]
@@ -92,7 +97,7 @@ simt_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* _
     }
 
     const int lane = tid & 31, warp = (tid - RLOAD) >> 5;
-    constexpr int RU = R + T <= 2 ? 4 : R + T <= 4 ? 2 : 1;
+    constexpr int RU = R + T <= 3 ? 4 : 2;                  // k of a batch, in fours
     const int lr = LT == 1 ? lane : LT == 2 ? lane >> 1 : (lane & 1) | lane >> 3 << 1;
     const int m0 = warp * LT * T + (LT == 1 ? 0 : LT == 2 ? lane & 1 : lane >> 1 & 3) * T;
     float acc[R][T];
@@ -152,13 +157,13 @@ simt_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* _
         }
 }
 
-template <int R, int T, int CW, int RST, typename TO>
+template <int R, int T, int CW, int RST, int RK, typename TO>
 int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
     constexpr int MR = 32 / (RN / R) * T * CW;
-    constexpr size_t smem = sizeof(float) * RST * (RN * RSTRIDE + MR * RK);
+    constexpr size_t smem = sizeof(float) * RST * (RN * (RK + 4) + MR * RK);
     static SmemLimit limit;
-    if (const int rc = limit.allow(simt_rows_kernel<R, T, CW, RST, TO>, smem)) return rc;
-    return launch_early(loaded, simt_rows_kernel<R, T, CW, RST, TO>, dim3((N + RN - 1) / RN), dim3(RLOAD + 32 * CW), smem, stream, A, W, out, M, N, K);
+    if (const int rc = limit.allow(simt_rows_kernel<R, T, CW, RST, RK, TO>, smem)) return rc;
+    return launch_early(loaded, simt_rows_kernel<R, T, CW, RST, RK, TO>, dim3((N + RN - 1) / RN), dim3(RLOAD + 32 * CW), smem, stream, A, W, out, M, N, K);
 }
 
 // ---------------------------------------------------------------- more rows
@@ -269,15 +274,16 @@ int launch_tile(const float* A, const float* W, TO* out, int M, int N, int K, cu
 // float32 operands whose rows are multiples of 16 bytes on 16-byte addresses
 template <typename TO>
 int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
-    // With one block an SM or fewer a block's ring has to keep HBM busy by itself: 16 stages instead of 8 (4096 x 4096, one row of A:
-    // 19.3 against 19.5 us; 4096 x 12288: 43.9 against 50.3).
+    // With one block an SM or fewer a block's ring has to keep HBM busy by itself, and its chain is as long as the barriers between its
+    // stages make it: four stages of 256 k, where more blocks an SM take four of 128 (five to eight rows: two of 256).  us, 64 k a stage before: 4096 x 4096 4 rows 21.2 -> 17.6, 8 rows 27.1 -> 23.2; 24576 x 4096 4 rows 74.9 -> 69.2, 8 rows
+    // 103.3 -> 85.7 (93.6 with 128 k), 16 rows 188.5 -> 174; 151936 x 4096 8 rows 618 -> 509; 2048 x 2048 one row 11.9 -> 8.1.
     const bool few = (N + RN - 1) / RN <= 148;
-#define PB_ROWS(R, T, CW, ST) return launch_rows<R, T, CW, ST>(A, W, out, M, N, K, loaded, stream)
-    if (M == 1) { if (few) PB_ROWS(1, 1, 1, 16); PB_ROWS(1, 1, 1, 8); }
-    if (M == 2) { if (few) PB_ROWS(2, 1, 1, 16); PB_ROWS(2, 1, 1, 8); }
-    if (M <= 4) { if (few) PB_ROWS(2, 1, 2, 16); PB_ROWS(2, 1, 2, 8); }
-    if (M <= 8) { if (few) PB_ROWS(2, 1, 4, 16); PB_ROWS(2, 2, 2, 8); }
-    if (M <= 16) { if (few) PB_ROWS(2, 1, 8, 16); PB_ROWS(4, 2, 2, 8); }
+#define PB_ROWS(R, T, CW, ST, RK) return launch_rows<R, T, CW, ST, RK>(A, W, out, M, N, K, loaded, stream)
+    if (M == 1) { if (few) PB_ROWS(1, 1, 1, 4, 256); PB_ROWS(1, 1, 1, 4, 128); }
+    if (M == 2) { if (few) PB_ROWS(2, 1, 1, 4, 256); PB_ROWS(2, 1, 1, 4, 128); }
+    if (M <= 4) { if (few) PB_ROWS(2, 1, 2, 4, 256); PB_ROWS(2, 1, 2, 4, 128); }
+    if (M <= 8) { if (few) PB_ROWS(2, 1, 4, 4, 256); PB_ROWS(2, 2, 2, 2, 256); }
+    if (M <= 16) { if (few) PB_ROWS(2, 1, 8, 4, 256); PB_ROWS(4, 2, 2, 4, 128); }
 #undef PB_ROWS
     // 64 rows a block where there are blocks for 16 rounds of the SMs (151936 x 4096, 387 rows: 11.3 against 11.9 ms), else 32, whose last
     // rounds are less empty (4096 x 4096: 33 rows 161 against 269 us, 387 rows 356 against 500, the general kernel 656;
