@@ -12,9 +12,15 @@
 // Scores, softmax and accumulators are float32 (expf); any group size, any head size
 // that is a multiple of 16 up to 256, float32 or bfloat16 storage, optional window.
 //
+// Bound by latency: a share is a tile or a few of 32 keys a warp.  While all blocks fit the SMs with a tile for each of their warps
+// in shared memory (kStaged), a warp asks for a tile's keys and values at once, by 16-byte asynchronous copies; with more blocks the
+// rows are read as they are needed, which lets an SM hold more blocks.  The heads of a pass have their chains side by side: no branch
+// stands between them.  us with the merge, float32, 8 key heads of 128, groups of 4 (before: rows as needed, heads one after the other):
+// 4 sequences of 460 keys 12.6 (18.0), 2 of 3,000 32.7 (33.9), 8 of 500 19.7 (20.7); 6 of 50, 8 heads of 64, groups of 2, 9.2 (12.3).
+//
 // Role in the reference: pulsar-core/src/kernels/paged_attention.cu:295-412
 // (paged_decode_split_kernel, paged_decode_combine_kernel; auto_splits :432-438).
-#include "common.cuh"
+#include "mma_common.cuh"
 
 #include <cstdlib>
 
@@ -24,8 +30,7 @@ using namespace pb;
 
 constexpr int kWarps = 4;
 constexpr int kMaxD = 256;
-constexpr int kAcc = kMaxD / 32;
-constexpr int kGP = 4;          // query heads handled per pass over the keys
+constexpr int kMaxGP = 4;       // query heads handled per pass over the keys, at most
 
 __device__ __forceinline__ void load_row16(const float* p, float (&f)[8]) {
     const float4 a = *reinterpret_cast<const float4*>(p);
@@ -43,7 +48,9 @@ __device__ __forceinline__ void load_row16(const __nv_bfloat16* p, float (&f)[8]
 }
 
 // partial layout: [S, Hq, n_splits, D + 2] floats: acc[D], m, l
-template <typename T>
+// kGP: query heads of a pass, kAcc: output elements of a lane (D / 32 rounded up).  A pass of fewer heads computes with zeros in the
+// places of the others: no branch stands between the heads' chains, which so run side by side.
+template <typename T, bool kStaged, int kGP, int kAcc>
 __global__ void __launch_bounds__(kWarps * 32)
 decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool,
                     float* __restrict__ partial, const int* __restrict__ block_table, int table_stride,
@@ -56,6 +63,11 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
     float* m_s = p_s + kWarps * kGP * 32;               // [kWarps][kGP]
     float* l_s = m_s + kWarps * kGP;                    // [kWarps][kGP]
     float* acc_s = l_s + kWarps * kGP;                  // [kWarps][kGP][D]
+    // staged: [kWarps][K, V][32 keys], rows 16 bytes more than D elements apart (off each other's banks)
+    const int row_bytes = D * (int)sizeof(T) + 16;
+    unsigned char* k_tile = reinterpret_cast<unsigned char*>(acc_s + kWarps * kGP * D) + (threadIdx.x >> 5) * 2 * 32 * row_bytes;
+    unsigned char* v_tile = k_tile + 32 * row_bytes;
+    pdl_wait();
 
     const int split = blockIdx.x, kvh = blockIdx.y, s = blockIdx.z;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -69,12 +81,36 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
     const int* table = block_table + (size_t)s * table_stride;
     const int stride = D + 2;
 
+    auto place = [&](int j) -> size_t {                 // where key j's row begins in the pools
+        int page = table[j / page_size];
+        if (!page_ok(page, bounds)) page = 0;
+        return (((size_t)page * Hkv + kvh) * page_size + j % page_size) * D;
+    };
+    // The warp's tile of keys and values from j0 on: every lane a key's place, the copies of a row side by side.
+    auto ask = [&](int j0) {
+        const size_t at = j0 + lane < end ? place(j0 + lane) : 0;
+        const int n_here = min(32, end - j0), chunks = D * (int)sizeof(T) / 16;      // 16-byte pieces of a row
+        const uint32_t k_dst = smem_u32(k_tile), v_dst = smem_u32(v_tile);
+        for (int r = 0; r < n_here; ++r) {
+            const size_t row = __shfl_sync(0xffffffffu, at, r);
+            for (int c = lane; c < 2 * chunks; c += 32) {
+                const bool is_v = c >= chunks;
+                const int piece = is_v ? c - chunks : c;
+                cp_async16((is_v ? v_dst : k_dst) + r * row_bytes + piece * 16,
+                           reinterpret_cast<const unsigned char*>((is_v ? v_pool : k_pool) + row) + piece * 16, true);
+            }
+        }
+    };
     for (int g0 = 0; g0 < G; g0 += kGP) {
         const int gn = min(kGP, G - g0);
+        if (kStaged) {
+            if (begin + warp * 32 < end) ask(begin + warp * 32);
+            cp_async_commit();
+        }
         __syncthreads();
-        for (int i = threadIdx.x; i < gn * D; i += blockDim.x) {
+        for (int i = threadIdx.x; i < kGP * D; i += blockDim.x) {
             const int g = i / D, d = i - g * D;
-            q_s[g * D + d] = to_float(q[((size_t)s * Hq + kvh * G + g0 + g) * D + d]) * scale;
+            q_s[g * D + d] = g < gn ? to_float(q[((size_t)s * Hq + kvh * G + g0 + g) * D + d]) * scale : 0.0f;
         }
         __syncthreads();
 
@@ -87,6 +123,10 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
         }
 
         for (int j0 = begin + warp * 32; j0 < end; j0 += kWarps * 32) {
+            if (kStaged) {
+                cp_async_wait<0>();
+                __syncwarp();
+            }
             const int j = j0 + lane;
             const bool valid = j < end;
             float sc[kGP];
@@ -94,47 +134,65 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
             for (int g = 0; g < kGP; ++g) sc[g] = 0.0f;
             size_t at = 0;                                  // where the key's row begins in the pools
             if (valid) {
-                int page = table[j / page_size];
-                if (!page_ok(page, bounds)) page = 0;
-                at = (((size_t)page * Hkv + kvh) * page_size + j % page_size) * D;
-                const T* kr = k_pool + at;
-                // 32 elements of the row asked for before the first is used (a trip to L2 per 32 elements instead of one per 8)
-                for (int d0 = 0; d0 < D; d0 += 32) {
-                    float kf[4][8];
+                if (!kStaged) at = place(j);
+                const T* kr = kStaged ? reinterpret_cast<const T*>(k_tile + lane * row_bytes) : k_pool + at;
+                // D is a multiple of 16.  A round's elements are asked for before those of the round before are used: 16 of them where
+                // they stand in shared memory, 32 where every round is a trip to L2.
+                constexpr int kRound = kStaged ? 16 : 32;
+                float kf[kRound / 8][8];
+                auto fetch = [&](int d0) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < kRound / 8; ++u)
                         if (d0 + 8 * u < D) load_row16(kr + d0 + 8 * u, kf[u]);
+                };
+                fetch(0);
+                for (int d0 = 0; d0 < D; d0 += kRound) {
+                    float now[kRound];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int d = d0 + 8 * u;
-                        if (d >= D) break;
+                    for (int e = 0; e < kRound; ++e) now[e] = kf[e / 8][e % 8];
+                    fetch(d0 + kRound);
 #pragma unroll
-                        for (int g = 0; g < kGP; ++g) {
-                            if (g < gn) {
-                                const float4 qa = *reinterpret_cast<const float4*>(q_s + g * D + d);
-                                const float4 qb = *reinterpret_cast<const float4*>(q_s + g * D + d + 4);
-                                sc[g] = fmaf(qa.x, kf[u][0], sc[g]); sc[g] = fmaf(qa.y, kf[u][1], sc[g]);
-                                sc[g] = fmaf(qa.z, kf[u][2], sc[g]); sc[g] = fmaf(qa.w, kf[u][3], sc[g]);
-                                sc[g] = fmaf(qb.x, kf[u][4], sc[g]); sc[g] = fmaf(qb.y, kf[u][5], sc[g]);
-                                sc[g] = fmaf(qb.z, kf[u][6], sc[g]); sc[g] = fmaf(qb.w, kf[u][7], sc[g]);
-                            }
-                        }
+                    for (int e = 0; e < kRound; e += 4) {
+                        if (e % 16 == 0 && d0 + e >= D) break;
+                        float4 qv[kGP];
+#pragma unroll
+                        for (int g = 0; g < kGP; ++g) qv[g] = *reinterpret_cast<const float4*>(q_s + g * D + d0 + e);
+#pragma unroll
+                        for (int g = 0; g < kGP; ++g) sc[g] = fmaf(qv[g].x, now[e], sc[g]);
+#pragma unroll
+                        for (int g = 0; g < kGP; ++g) sc[g] = fmaf(qv[g].y, now[e + 1], sc[g]);
+#pragma unroll
+                        for (int g = 0; g < kGP; ++g) sc[g] = fmaf(qv[g].z, now[e + 2], sc[g]);
+#pragma unroll
+                        for (int g = 0; g < kGP; ++g) sc[g] = fmaf(qv[g].w, now[e + 3], sc[g]);
                     }
                 }
             }
             __syncwarp();
+            float top[kGP], sum[kGP];
+#pragma unroll
+            for (int g = 0; g < kGP; ++g) top[g] = valid ? sc[g] : -INFINITY;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int g = 0; g < kGP; ++g) top[g] = fmaxf(top[g], __shfl_xor_sync(0xffffffffu, top[g], o));
 #pragma unroll
             for (int g = 0; g < kGP; ++g) {
-                if (g < gn) {
-                    const float m_new = fmaxf(m_run[g], warp_max(valid ? sc[g] : -INFINITY));
-                    const float pv = valid ? expf(sc[g] - m_new) : 0.0f;
-                    const float corr = expf(m_run[g] - m_new);
-                    l_run[g] = l_run[g] * corr + warp_sum(pv);
-                    m_run[g] = m_new;
+                top[g] = fmaxf(m_run[g], top[g]);
+                sum[g] = valid ? expf(sc[g] - top[g]) : 0.0f;
+                p_s[(warp * kGP + g) * 32 + lane] = sum[g];
+            }
 #pragma unroll
-                    for (int i = 0; i < kAcc; ++i) acc[g][i] *= corr;
-                    p_s[(warp * kGP + g) * 32 + lane] = pv;
-                }
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int g = 0; g < kGP; ++g) sum[g] += __shfl_xor_sync(0xffffffffu, sum[g], o);
+#pragma unroll
+            for (int g = 0; g < kGP; ++g) {
+                const float corr = expf(m_run[g] - top[g]);
+                l_run[g] = l_run[g] * corr + sum[g];
+                m_run[g] = top[g];
+#pragma unroll
+                for (int i = 0; i < kAcc; ++i) acc[g][i] *= corr;
             }
             __syncwarp();
             const int n_here = min(32, end - j0);
@@ -143,7 +201,8 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
                 float vf[4][kAcc];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const T* vr = v_pool + __shfl_sync(0xffffffffu, at, min(k0 + u, n_here - 1));
+                    const int r = min(k0 + u, n_here - 1);
+                    const T* vr = kStaged ? reinterpret_cast<const T*>(v_tile + r * row_bytes) : v_pool + __shfl_sync(0xffffffffu, at, r);
 #pragma unroll
                     for (int i = 0; i < kAcc; ++i) {
                         const int d = lane + 32 * i;
@@ -152,16 +211,21 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    if (k0 + u >= n_here) break;
+                    float pk[kGP];
 #pragma unroll
-                    for (int g = 0; g < kGP; ++g) {
-                        if (g < gn) {
-                            const float pk = p_s[(warp * kGP + g) * 32 + k0 + u];
+                    for (int g = 0; g < kGP; ++g) pk[g] = p_s[(warp * kGP + g) * 32 + k0 + u];
+                    if (k0 + u < n_here) {
 #pragma unroll
-                            for (int i = 0; i < kAcc; ++i) acc[g][i] = fmaf(pk, vf[u][i], acc[g][i]);
-                        }
+                        for (int g = 0; g < kGP; ++g)
+#pragma unroll
+                            for (int i = 0; i < kAcc; ++i) acc[g][i] = fmaf(pk[g], vf[u][i], acc[g][i]);
                     }
                 }
+            }
+            if (kStaged) {
+                __syncwarp();                           // the tile is done with
+                if (j0 + kWarps * 32 < end) ask(j0 + kWarps * 32);
+                cp_async_commit();
             }
         }
 
@@ -195,6 +259,7 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const
             if (d == 0) { dst[D] = m_all; dst[D + 1] = l_all; }
         }
     }
+    pdl_trigger();
 }
 
 // One block per (sequence, head): the weights exp(m_i - m_all) of the splits are computed
@@ -253,7 +318,31 @@ __global__ void decode_combine_kernel(const float* __restrict__ partial, T* __re
 }
 
 size_t split_smem(int D) {
-    return sizeof(float) * ((size_t)kGP * D + kWarps * kGP * 32 + 2 * kWarps * kGP + (size_t)kWarps * kGP * D);
+    return sizeof(float) * ((size_t)kMaxGP * D + kWarps * kMaxGP * 32 + 2 * kWarps * kMaxGP + (size_t)kWarps * kMaxGP * D);
+}
+
+template <typename T, int kGP, int kAcc>
+int launch_split(const void* q, const void* k_pool, const void* v_pool, float* partial, const int* block_table, int table_stride,
+                 const int* kv_len, int n_seqs, int Hq, int Hkv, int D, int page_size, float scale, int window, int n_splits, cudaStream_t stream) {
+    const size_t plain = split_smem(D), staged = plain + (size_t)kWarps * 2 * 32 * (D * sizeof(T) + 16);
+    const dim3 grid(n_splits, Hkv, n_seqs);
+    const bool aligned = (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
+    const long long at_once = 148 * (227 * 1024 / (long long)(staged + 1024));
+    if (aligned && (long long)n_splits * Hkv * n_seqs <= at_once) {
+        static SmemLimit limit;
+        if (const int rc = limit.allow(decode_split_kernel<T, true, kGP, kAcc>, staged)) return rc;
+        return launch_pdl(decode_split_kernel<T, true, kGP, kAcc>, grid, kWarps * 32, staged, stream, (const T*)q, (const T*)k_pool, (const T*)v_pool,
+                          partial, block_table, table_stride, kv_len, Hq, Hkv, D, page_size, scale, window, n_splits, pool_bounds_now());
+    }
+    return launch_pdl(decode_split_kernel<T, false, kGP, kAcc>, grid, kWarps * 32, plain, stream, (const T*)q, (const T*)k_pool, (const T*)v_pool,
+                      partial, block_table, table_stride, kv_len, Hq, Hkv, D, page_size, scale, window, n_splits, pool_bounds_now());
+}
+
+// The heads of a pass by the group's size, a lane's elements by the head's.
+template <typename T, typename... Args>
+int launch_split_for(int G, int D, Args... args) {
+    if (G <= 2) return D <= 64 ? launch_split<T, 2, 2>(args...) : D <= 128 ? launch_split<T, 2, 4>(args...) : launch_split<T, 2, 8>(args...);
+    return D <= 64 ? launch_split<T, 4, 2>(args...) : D <= 128 ? launch_split<T, 4, 4>(args...) : launch_split<T, 4, 8>(args...);
 }
 
 }  // namespace
@@ -271,22 +360,14 @@ PB_EXPORT int pb_paged_attention_decode(int dtype, const void* q, const void* k_
     if (n_seqs <= 0) return 0;
     if (D <= 0 || D % 16 || D > kMaxD || Hkv <= 0 || Hq % Hkv || page_size <= 0 || n_splits <= 0) return PB_ERR_BAD_SIZE;
     if (Hkv > 65535 || n_seqs > 65535 || n_splits > 64) return PB_ERR_TOO_LARGE;
-    const size_t smem = split_smem(D);
-    dim3 grid(n_splits, Hkv, n_seqs);
-    if (dtype == PB_F32) {
-        decode_split_kernel<float><<<grid, kWarps * 32, smem, stream>>>((const float*)q, (const float*)k_pool,
-            (const float*)v_pool, partial, block_table, table_stride, kv_len, Hq, Hkv, D, page_size, scale, window, n_splits,
-            pb::pool_bounds_now());
-        decode_combine_kernel<float><<<n_seqs * Hq, 128, 0, stream>>>(partial, (float*)out, D, n_splits);
-    } else if (dtype == PB_BF16) {
-        decode_split_kernel<__nv_bfloat16><<<grid, kWarps * 32, smem, stream>>>((const __nv_bfloat16*)q,
-            (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, partial, block_table, table_stride, kv_len, Hq, Hkv, D,
-            page_size, scale, window, n_splits, pb::pool_bounds_now());
-        decode_combine_kernel<__nv_bfloat16><<<n_seqs * Hq, 128, 0, stream>>>(partial, (__nv_bfloat16*)out, D, n_splits);
-    } else {
-        return PB_ERR_BAD_DTYPE;
-    }
-    return launch_status();
+    if (dtype != PB_F32 && dtype != PB_BF16) return PB_ERR_BAD_DTYPE;
+    const int rc = dtype == PB_F32 ? launch_split_for<float>(Hq / Hkv, D, q, k_pool, v_pool, partial, block_table, table_stride, kv_len, n_seqs, Hq,
+                                                             Hkv, D, page_size, scale, window, n_splits, stream)
+                                   : launch_split_for<__nv_bfloat16>(Hq / Hkv, D, q, k_pool, v_pool, partial, block_table, table_stride, kv_len,
+                                                                     n_seqs, Hq, Hkv, D, page_size, scale, window, n_splits, stream);
+    if (rc != 0) return rc;
+    if (dtype == PB_F32) return launch_pdl(decode_combine_kernel<float>, n_seqs * Hq, 128, 0, stream, partial, (float*)out, D, n_splits);
+    return launch_pdl(decode_combine_kernel<__nv_bfloat16>, n_seqs * Hq, 128, 0, stream, partial, (__nv_bfloat16*)out, D, n_splits);
 }
 
 // ---------------------------------------------------------------------------------------

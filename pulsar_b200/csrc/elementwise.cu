@@ -213,6 +213,8 @@ __global__ void qk_norm_rope_write_kernel(const T* __restrict__ qkv, T* __restri
                                           const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                           const float* __restrict__ q_weight, const float* __restrict__ k_weight,
                                           float eps, int Hq, int Hkv, int D, int rotary, int page_size, const PoolBounds bounds) {
+    pdl_trigger();
+    pdl_wait();
     const int t = blockIdx.x;
     const int lane = threadIdx.x & 31;
     const int head = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -368,6 +370,8 @@ qk_norm_rope_write_bf16_d128_kernel(const uint32_t* __restrict__ qkv, uint32_t* 
 // out[t, i] = silu(gu[t, i]) * gu[t, I + i], silu(z) = z / (1 + exp(-z)); one rounding.
 template <typename T>
 __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, int inter, size_t total) {
+    pdl_trigger();      // a few microseconds: let the next product start fetching its weights
+    pdl_wait();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
         const size_t t = idx / inter;
@@ -380,6 +384,8 @@ __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, i
 
 // The same on 16-byte vectors of bfloat16 (inter % 8 == 0, 16-byte aligned rows).
 __global__ void silu_mul_bf16x8_kernel(const uint4* __restrict__ gu, uint4* __restrict__ out, int inter8, size_t total8) {
+    pdl_trigger();      // a few microseconds: let the next product start fetching its weights
+    pdl_wait();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total8;
          idx += (size_t)gridDim.x * blockDim.x) {
         const size_t t = idx / inter8;
@@ -591,14 +597,13 @@ PB_EXPORT int pb_qk_norm_rope_write(int dtype, const void* qkv, void* q_out, voi
     }
     dim3 grid(n, (heads + warps - 1) / warps);
     if (dtype == PB_F32)
-        qk_norm_rope_write_kernel<float><<<grid, warps * 32, 0, stream>>>((const float*)qkv, (float*)q_out, (float*)k_pool, (float*)v_pool,
-            slots, cos_t, sin_t, q_weight, k_weight, eps, Hq, Hkv, D, rotary, page_size, pb::pool_bounds_now());
-    else if (dtype == PB_BF16)
-        qk_norm_rope_write_kernel<__nv_bfloat16><<<grid, warps * 32, 0, stream>>>((const __nv_bfloat16*)qkv, (__nv_bfloat16*)q_out,
-            (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, slots, cos_t, sin_t, q_weight, k_weight, eps, Hq, Hkv, D, rotary, page_size,
-            pb::pool_bounds_now());
-    else return PB_ERR_BAD_DTYPE;
-    return launch_status();
+        return launch_pdl(qk_norm_rope_write_kernel<float>, grid, warps * 32, 0, stream, (const float*)qkv, (float*)q_out, (float*)k_pool, (float*)v_pool,
+                          slots, cos_t, sin_t, q_weight, k_weight, eps, Hq, Hkv, D, rotary, page_size, pb::pool_bounds_now());
+    if (dtype == PB_BF16)
+        return launch_pdl(qk_norm_rope_write_kernel<__nv_bfloat16>, grid, warps * 32, 0, stream, (const __nv_bfloat16*)qkv, (__nv_bfloat16*)q_out,
+                          (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, slots, cos_t, sin_t, q_weight, k_weight, eps, Hq, Hkv, D, rotary, page_size,
+                          pb::pool_bounds_now());
+    return PB_ERR_BAD_DTYPE;
 }
 
 PB_EXPORT int pb_silu_mul(int dtype, const void* gate_up, void* out, int n, int inter, cudaStream_t stream) {
@@ -610,9 +615,9 @@ PB_EXPORT int pb_silu_mul(int dtype, const void* gate_up, void* out, int n, int 
     if (dtype == PB_BF16 && inter % 8 == 0 && ((uintptr_t)gate_up & 15) == 0 && ((uintptr_t)out & 15) == 0) {
         size_t total8 = total / 8, blocks8 = (total8 + b - 1) / b;
         if (blocks8 > 148 * 16) blocks8 = 148 * 16;
-        silu_mul_bf16x8_kernel<<<(int)blocks8, b, 0, stream>>>((const uint4*)gate_up, (uint4*)out, inter / 8, total8);
-    } else if (dtype == PB_F32) silu_mul_kernel<float><<<(int)blocks, b, 0, stream>>>((const float*)gate_up, (float*)out, inter, total);
-    else if (dtype == PB_BF16) silu_mul_kernel<__nv_bfloat16><<<(int)blocks, b, 0, stream>>>((const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, inter, total);
-    else return PB_ERR_BAD_DTYPE;
-    return launch_status();
+        return launch_pdl(silu_mul_bf16x8_kernel, (int)blocks8, b, 0, stream, (const uint4*)gate_up, (uint4*)out, inter / 8, total8);
+    }
+    if (dtype == PB_F32) return launch_pdl(silu_mul_kernel<float>, (int)blocks, b, 0, stream, (const float*)gate_up, (float*)out, inter, total);
+    if (dtype == PB_BF16) return launch_pdl(silu_mul_kernel<__nv_bfloat16>, (int)blocks, b, 0, stream, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, inter, total);
+    return PB_ERR_BAD_DTYPE;
 }
