@@ -9,7 +9,7 @@
 //
 // Three kernels:
 //   * simt_rows_kernel (up to 16 rows of A, float32 operands): streams the weights, bound by HBM;
-//   * simt_tile_kernel (more rows, float32 operands): bound by the FMA pipes;
+//   * simt_tile_kernel (more rows, float32 operands): bound by the FMA pipes and the register file;
 //   * gemm_simt_kernel: everything else (bfloat16 operands, rows of K that are no multiple of 16 bytes).
 //
 // The reference uses at::linear here (cuBLAS SGEMM in float32,
@@ -251,23 +251,125 @@ __device__ __forceinline__ void tile_block(const float* __restrict__ A, const fl
     }
 }
 
-template <int TM, typename TO>
+// 32 rows by 128 columns with paired multiply-adds (fma.rn.f32x2: two sums of neighbouring columns, each rounded by itself, so the same
+// bits).  From registers alone single multiply-adds reach 52 TFLOP/s here, paired ones 63: three operands a lane and cycle are more than
+// the register file gives.  A pair wants neighbouring columns in neighbouring registers, so both operands stand with k slowest in
+// shared memory: 16-byte loads of four k bring them to registers while the stage before is computed, and four stores turn them (columns
+// shifted by the k's quad, which spreads the stores over the banks).  A thread takes rows 4 ty .. 4 ty + 3 and columns 4 tx .. + 3 and 16 + 4 tx ..
+// + 3 of its warp's 32; its a values are doubled into pairs.  us, single multiply-adds before: 24576 x 4096 with 387 rows 1,898 -> 1,732,
+// 4096 x 4096 357 -> 338, 6144 x 4096 634 -> 493.  With 64 rows a block 1,838, with pairs along the rows 1,883.
+constexpr int PK = 32, PM = 32;
+__device__ __forceinline__ unsigned long long pair_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+template <typename TO>
+__device__ __forceinline__ void pair_block(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out,
+                                           int M, int N, int K, float* smem) {
+    constexpr int kStage = PK * (PM + GN), QK = PK / 4;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = lane >> 1 & 3, ty = (lane & 1) | lane >> 3 << 1;
+    const int row0 = blockIdx.x * PM, col0 = blockIdx.y * GN, n_kt = (K + PK - 1) / PK;
+    const int q = tid % QK, r0 = tid / QK;                   // this thread's quad of k and its first row of 16 a round
+    float4 ra[PM / 16], rw[GN / 16];
+    auto fetch = [&](int kt) {
+        const int k = kt * PK + q * 4;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < PM / 16; ++e) {
+            const int r = row0 + r0 + 16 * e;
+            ra[e] = r < M && k < K ? *reinterpret_cast<const float4*>(A + (size_t)r * K + k) : zero;
+        }
+#pragma unroll
+        for (int e = 0; e < GN / 16; ++e) {
+            const int r = col0 + r0 + 16 * e;
+            rw[e] = r < N && k < K ? *reinterpret_cast<const float4*>(W + (size_t)r * K + k) : zero;
+        }
+    };
+    auto put = [&](float* dst, int rows, int at, const float4& v) {
+        dst += q * 4 * rows + (at ^ 8 * (q & 3));
+        dst[0] = v.x; dst[rows] = v.y; dst[2 * rows] = v.z; dst[3 * rows] = v.w;
+    };
+    auto stash = [&](int stage) {
+        float* as = smem + stage * kStage;
+#pragma unroll
+        for (int e = 0; e < PM / 16; ++e) put(as, PM, r0 + 16 * e, ra[e]);
+#pragma unroll
+        for (int e = 0; e < GN / 16; ++e) put(as + PK * PM, GN, r0 + 16 * e, rw[e]);
+    };
+    unsigned long long acc[4][4];                            // [row][pair of columns]
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+    fetch(0);
+    stash(0);
+    __syncthreads();
+    for (int kt = 0; kt < n_kt; ++kt) {
+        if (kt + 1 < n_kt) fetch(kt + 1);
+        const float* as = smem + (kt & 1) * kStage;
+        const float* ws = as + PK * PM + warp * 32;
+#pragma unroll
+        for (int k = 0; k < PK; ++k) {
+            const int shift = 8 * (k >> 2 & 3);
+            const float4 a = *reinterpret_cast<const float4*>(as + k * PM + ((ty * 4) ^ shift));
+            const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(ws + k * GN + ((tx * 4) ^ shift));
+            const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(ws + k * GN + ((tx * 4 + 16) ^ shift));
+            const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                unsigned long long d;
+                asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(av[i]));
+                acc[i][0] = pair_fma(d, w0.x, acc[i][0]);
+                acc[i][1] = pair_fma(d, w0.y, acc[i][1]);
+                acc[i][2] = pair_fma(d, w1.x, acc[i][2]);
+                acc[i][3] = pair_fma(d, w1.y, acc[i][3]);
+            }
+        }
+        if (kt + 1 < n_kt) stash((kt + 1) & 1);
+        __syncthreads();
+    }
+    const bool vector = N % 4 == 0 && (uintptr_t)out % (4 * sizeof(TO)) == 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = row0 + ty * 4 + i;
+        if (r >= M) continue;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = col0 + warp * 32 + tx * 4 + 16 * h;
+            float v[4];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[i][2 * h]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[i][2 * h + 1]));
+            TO* o = out + (size_t)r * N + c;
+            if (vector && c < N) store_quad(o, v);
+            else
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (c + e < N) o[e] = from_float<TO>(v[e]);
+        }
+    }
+}
+
+template <int TM, bool kPairs, typename TO>
 __global__ void __launch_bounds__(128, TM == 8 ? 3 : 4)
 simt_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out, int M, int N, int K) {
     constexpr int GM = 8 * TM;
     __shared__ __align__(16) float tile_smem[Tile<GM>::GST * (GM + GN) * Tile<GM>::GSTRIDE];
     const int left = M - (int)blockIdx.x * GM;
     if (TM == 8 && left > 32) tile_block<GM, TM, TO>(A, W, out, M, N, K, tile_smem);
+    else if (kPairs && left > 16) pair_block<TO>(A, W, out, M, N, K, tile_smem);
     else if (left > 16) tile_block<GM, 4, TO>(A, W, out, M, N, K, tile_smem);
     else if (left > 8) tile_block<GM, 2, TO>(A, W, out, M, N, K, tile_smem);
     else tile_block<GM, 1, TO>(A, W, out, M, N, K, tile_smem);
 }
 
-template <int TM, typename TO>
+template <int TM, bool kPairs, typename TO>
 int launch_tile(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
     dim3 grid((M + 8 * TM - 1) / (8 * TM), (N + GN - 1) / GN);
     if (grid.y > 65535) return PB_ERR_TOO_LARGE;
-    simt_tile_kernel<TM, TO><<<grid, 128, 0, stream>>>(A, W, out, M, N, K);
+    static_assert(TM == 4 || !kPairs, "pairs are computed by blocks of 32 rows");
+    simt_tile_kernel<TM, kPairs, TO><<<grid, 128, 0, stream>>>(A, W, out, M, N, K);
     return launch_status();
 }
 
@@ -288,8 +390,11 @@ int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, boo
     // 64 rows a block where there are blocks for 16 rounds of the SMs (151936 x 4096, 387 rows: 11.3 against 11.9 ms), else 32, whose last
     // rounds are less empty (4096 x 4096: 33 rows 161 against 269 us, 387 rows 356 against 500, the general kernel 656;
     // 24576 x 4096, 387 rows: 1.90 against 2.00 ms, 2.96 before)
-    if ((long)((M + 63) / 64) * ((N + GN - 1) / GN) >= 16 * 148) return launch_tile<8>(A, W, out, M, N, K, stream);
-    return launch_tile<4>(A, W, out, M, N, K, stream);
+    if ((long)((M + 63) / 64) * ((N + GN - 1) / GN) >= 16 * 148) return launch_tile<8, false>(A, W, out, M, N, K, stream);
+    // Pairs where an SM has two blocks and more, whose loads then cover each other's (4096 x 12288, 200 rows: 773 us both ways): with
+    // one, the asynchronous copies are ahead (100 rows 448 against 609; 6144 x 4096, 64 rows 153 against 218).
+    if ((long)((M + 31) / 32) * ((N + GN - 1) / GN) > 148) return launch_tile<4, true>(A, W, out, M, N, K, stream);
+    return launch_tile<4, false>(A, W, out, M, N, K, stream);
 }
 
 // ---------------------------------------------------------------- any operands
