@@ -23,6 +23,8 @@ import torch
 
 from .. import ops
 
+_MAX_TOP_K = 2 ** 31 - 1           # the kernels count in 32 bits
+
 
 @dataclass
 class GenerationParams:
@@ -36,10 +38,19 @@ class GenerationParams:
             raise ValueError(f"top_p must lie in (0, 1], found {self.top_p}")
         if self.top_k < 0:
             raise ValueError(f"top_k must be >= 0, found {self.top_k}")
+        if not self.greedy and not self.top_k <= _MAX_TOP_K:
+            raise ValueError(f"top_k must be at most {_MAX_TOP_K}, found {self.top_k}")
 
     @property
     def greedy(self) -> bool:
         return not (self.temperature > 0.0)
+
+    def device_top_k(self) -> int:
+        """``top_k`` as the kernels take it (a greedy row has no use for its own)."""
+        k = 0 if self.greedy else int(self.top_k)
+        if not -_MAX_TOP_K - 1 <= k <= _MAX_TOP_K:
+            raise ValueError(f"top_k must be at most {_MAX_TOP_K}, found {self.top_k}")
+        return k
 
 
 def make_generator(seed: int) -> torch.Generator:
@@ -92,7 +103,7 @@ class Sampler:
                                        torch.cuda.Event())
         buf, floats, ints, event = slot
         floats[:3 * rows] = [p.temperature for p in params] + [p.top_p for p in params] + uniform
-        ints[3 * rows:4 * rows] = [p.top_k for p in params]
+        ints[3 * rows:4 * rows] = [p.device_top_k() for p in params]
         out = torch.empty((4, rows), dtype=torch.float32, device=self.device)
         ops.copy_pinned(out, buf, 4 * rows)
         event.record(ops.current_stream())
