@@ -52,10 +52,8 @@ class _Inflight:
     """A forward pass whose sampled ids are on their way to the host."""
     sampled: List[int]                     # sequences sampled in it, in the order of its rows
     row_of: Dict[int, int]
-    host: torch.Tensor                     # pinned; filled when ``event`` has passed
-    event: torch.cuda.Event
+    report: "ops.Pinned"                   # the kernels' wait error words behind this pass, then its sampled ids
     uniform: List[float]                   # what each row drew (0.0 for greedy sequences)
-    status: Optional[torch.Tensor] = None          # pinned; the kernels' wait error words behind this pass
     void: set = field(default_factory=set)         # sequences that had ended before this pass: its token is dropped
 
 
@@ -111,7 +109,7 @@ class Engine:
         self._mailbox: Dict[int, list] = {}     # events of other sessions seen while one session streams
         self._inflight: Optional[_Inflight] = None          # the pass whose tokens have not been read yet
         self._unclaimed: List[Tuple[int, int, bool]] = []   # events booked outside ``step``
-        self._host_report: List[Optional[torch.Tensor]] = [None, None, None]      # pinned: error words, then sampled ids
+        self._host_report: List[Optional[ops.Pinned]] = [None, None, None]
         self._host_next = 0
         self._failed: Optional[BaseException] = None
 
@@ -260,31 +258,28 @@ class Engine:
         # the error words of the kernels with bounded waits travel with the ids, in one copy: no synchronisation of their own
         ops.gather_wait_words(self.sampler.head)
         n_words = Sampler.HEAD + len(sampled)
-        slot = self._host_report[self._host_next]
-        if slot is None or slot.numel() < n_words:
-            slot = self._host_report[self._host_next] = torch.zeros(max(Sampler.HEAD + 64, n_words), dtype=torch.int32, pin_memory=True)
+        report = self._host_report[self._host_next]
+        if report is None or report.host.numel() < n_words:
+            report = self._host_report[self._host_next] = ops.Pinned(max(Sampler.HEAD + 64, n_words), torch.int32)
         self._host_next = (self._host_next + 1) % len(self._host_report)
-        ops.copy_pinned(slot, self.sampler.report(len(sampled)), n_words)
-        status, host = slot[:Sampler.HEAD], slot[Sampler.HEAD:n_words]
-        event = torch.cuda.Event()
-        event.record(ops.current_stream())
+        report.from_device(self.sampler.report(len(sampled)), n_words)
         for r in sampled:
             self.scheduler.on_sampled(r)
-        return _Inflight(sampled, {r: i for i, r in enumerate(sampled)}, host, event, uniform, status)
+        return _Inflight(sampled, {r: i for i, r in enumerate(sampled)}, report, uniform)
 
     def _collect(self, flight: "_Inflight") -> List[Tuple[int, int, bool]]:
         """Wait for a pass's sampled ids and book them: events ``(seq_id, token, finished)``."""
         with profiling.scope("read (wait for the sampled ids)"):
-            flight.event.synchronize()
-        if flight.status is not None:
-            what = ops.describe_wait_words(flight.status[:ops.N_WAIT_WORDS].tolist())
-            if what is not None:
-                # the pass's tokens come from a kernel that gave up: none of them is booked, and nothing runs after it
-                self._failed = ops.DeviceWaitError(what)
-                self._inflight = None
-                raise EngineFailed(f"a forward pass did not complete: {what}") from self._failed
+            flight.report.wait()
+        words = flight.report.host[:Sampler.HEAD + len(flight.sampled)].tolist()
+        what = ops.describe_wait_words(words[:ops.N_WAIT_WORDS])
+        if what is not None:
+            # the pass's tokens come from a kernel that gave up: none of them is booked, and nothing runs after it
+            self._failed = ops.DeviceWaitError(what)
+            self._inflight = None
+            raise EngineFailed(f"a forward pass did not complete: {what}") from self._failed
         events = []
-        for rid, tok in zip(flight.sampled, flight.host.tolist()):
+        for rid, tok in zip(flight.sampled, words[Sampler.HEAD:]):
             if rid not in self.scheduler.seqs:
                 continue                            # released while the pass was in flight
             if rid in flight.void:

@@ -65,8 +65,7 @@ class ModelRunner:
         self._scratch: Dict[tuple, torch.Tensor] = {}
         self._scratch_views: Dict[tuple, Dict[tuple, torch.Tensor]] = {}      # of each buffer, by shape
         self.scratch_epoch = 0
-        self._staging: List[Optional[torch.Tensor]] = [None] * self.N_STAGING
-        self._staging_events: List[Optional[torch.cuda.Event]] = [None] * self.N_STAGING
+        self._staging: List[Optional[ops.Pinned]] = [None] * self.N_STAGING
         self._staging_next = 0
         self._index_buf: Optional[torch.Tensor] = None
         self._views: Dict[tuple, list] = {}
@@ -128,17 +127,15 @@ class ModelRunner:
             return CacheView("state", state=self.cache.state[entry], page_size=self.cache.page_size)
         return CacheView("none", page_size=self.cache.page_size)
 
-    def _stage(self, n_ints: int) -> torch.Tensor:
+    def _stage(self, n_ints: int) -> "ops.Pinned":
         i = self._staging_next
         self._staging_next = (i + 1) % self.N_STAGING
-        if self._staging_events[i] is not None:
-            self._staging_events[i].synchronize()
-        buf = self._staging[i]
-        if buf is None or buf.numel() < n_ints:
-            buf = torch.empty(max(n_ints, 4096), dtype=torch.int32, pin_memory=True)
-            self._staging[i] = buf
-        self._staging_slot = i
-        return buf
+        stage = self._staging[i]
+        if stage is not None:
+            stage.wait()
+        if stage is None or stage.host.numel() < n_ints:
+            stage = self._staging[i] = ops.Pinned(max(n_ints, 4096), torch.int32)
+        return stage
 
     # ------------------------------------------------------------------ the step
     def prepare(self, entries: Sequence[StepEntry], sampled_ids: Optional[torch.Tensor] = None) -> StepContext:
@@ -225,7 +222,7 @@ class ModelRunner:
         offsets_c, lengths_c = (ctypes.c_int * n_arrays)(), (ctypes.c_int * n_arrays)()
         stage = self._stage(total)
         rc = lib.ph_step_pack(handle, s, rids, n_tok, tokens, want_n, wants, token_src, starts_c, slots_c, widths_c,
-                              stage.data_ptr(), stage.numel(), offsets_c, lengths_c)
+                              stage.host.data_ptr(), stage.host.numel(), offsets_c, lengths_c)
         if rc == host.RELEASED_PAGE:
             raise StepError("a position of the step lies in a released page")
         if rc != total:
@@ -236,12 +233,8 @@ class ModelRunner:
             self.scratch_epoch += 1
             self._views.clear()
         dev = self._index_buf
-        ops.copy_pinned(dev, stage, total)
+        stage.to_device(dev, total)
         self.h2d_bytes += total * 4
-        ev = self._staging_events[self._staging_slot]
-        if ev is None:
-            ev = self._staging_events[self._staging_slot] = torch.cuda.Event()
-        ev.record(ops.current_stream())
 
         # Views of the device buffer; steady decoding has the same layout every step, so they are kept.
         key = (tuple(lengths), tuple(widths))

@@ -223,11 +223,38 @@ def _p(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
-def copy_pinned(dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
-    """The first ``n`` elements of ``src`` to ``dst``, one of them on the device and the other in pinned host memory, in the stream; the
-    host does not wait.  What slices and ``Tensor.copy_`` do, at a third of their host time."""
-    assert dst.is_cuda != src.is_cuda and dst.dtype == src.dtype and 0 <= n <= min(dst.numel(), src.numel()) and dst.is_contiguous() and src.is_contiguous()
-    check(fn("pb_copy")(dst.data_ptr(), src.data_ptr(), n * src.element_size(), stream()), "copy", kernels=0)
+class Pinned:
+    """Pinned host memory whose copies to and from the device take a third of the host time of slices and ``Tensor.copy_``.  PyTorch's
+    host allocator, which would give the memory to another tensor as soon as this one is gone, does not hear of such copies: so the last
+    one is waited for before that."""
+
+    def __init__(self, numel: int, dtype: torch.dtype):
+        self.host = torch.zeros(numel, dtype=dtype, pin_memory=True)
+        self.event = torch.cuda.Event()            # behind the last copy
+
+    def _copy(self, dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
+        assert dst.is_cuda != src.is_cuda and dst.dtype == src.dtype and 0 <= n <= min(dst.numel(), src.numel()) and dst.is_contiguous() and src.is_contiguous()
+        try:
+            check(fn("pb_copy")(dst.data_ptr(), src.data_ptr(), n * src.element_size(), stream()), "copy", kernels=0)
+        finally:
+            self.event.record(current_stream())
+
+    def to_device(self, dst: torch.Tensor, n: int) -> None:
+        """The first ``n`` elements to ``dst``, in the stream; the host does not wait."""
+        self._copy(dst, self.host, n)
+
+    def from_device(self, src: torch.Tensor, n: int) -> None:
+        """The first ``n`` elements of ``src`` to this memory, in the stream; they are here once ``wait`` returns."""
+        self._copy(self.host, src, n)
+
+    def wait(self) -> None:
+        self.event.synchronize()
+
+    def __del__(self):
+        try:
+            self.event.synchronize()
+        except Exception:                          # never made whole, or a process that is on its way out
+            pass
 
 
 def embed(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, scale: float = 1.0) -> None:

@@ -77,7 +77,7 @@ class Sampler:
         self._report = torch.zeros(self.HEAD + 64, dtype=torch.int32, device=self.device)
         self.last_ids: Optional[torch.Tensor] = None      # what the last call returned
         # The rows' parameters travel in one copy from pinned memory, one buffer for each of the last calls: (the memory, the same
-        # as C floats and as C ints, the event behind its last copy).
+        # as C floats and as C ints).
         self._staging: List[Optional[tuple]] = [None] * 4
         self._staging_next = 0
 
@@ -95,18 +95,16 @@ class Sampler:
         self._staging_next = (i + 1) % len(self._staging)
         slot = self._staging[i]
         if slot is not None:
-            slot[3].synchronize()             # the copy out of this buffer, some calls ago
-        if slot is None or slot[0].numel() < 4 * rows:
-            buf = torch.empty(4 * max(rows, 64), dtype=torch.float32, pin_memory=True)
-            at = buf.data_ptr()
-            slot = self._staging[i] = (buf, (ctypes.c_float * buf.numel()).from_address(at), (ctypes.c_int * buf.numel()).from_address(at),
-                                       torch.cuda.Event())
-        buf, floats, ints, event = slot
+            slot[0].wait()                        # the copy out of this buffer, some calls ago
+        if slot is None or slot[0].host.numel() < 4 * rows:
+            buf = ops.Pinned(4 * max(rows, 64), torch.float32)
+            at, n = buf.host.data_ptr(), buf.host.numel()
+            slot = self._staging[i] = (buf, (ctypes.c_float * n).from_address(at), (ctypes.c_int * n).from_address(at))
+        buf, floats, ints = slot
         floats[:3 * rows] = [p.temperature for p in params] + [p.top_p for p in params] + uniform
         ints[3 * rows:4 * rows] = [p.device_top_k() for p in params]
         out = torch.empty((4, rows), dtype=torch.float32, device=self.device)
-        ops.copy_pinned(out, buf, 4 * rows)
-        event.record(ops.current_stream())
+        buf.to_device(out, 4 * rows)
         return out
 
     def sample_on_device(self, logits: torch.Tensor, params: Sequence[GenerationParams],
