@@ -234,6 +234,14 @@ class Pinned:
 
     def _copy(self, dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
         assert dst.is_cuda != src.is_cuda and dst.dtype == src.dtype and 0 <= n <= min(dst.numel(), src.numel()) and dst.is_contiguous() and src.is_contiguous()
+        where = dst.device if dst.is_cuda else src.device
+        if _device is None or where.index != _device():            # the stream is that of the tensor's device, whichever is current
+            with torch.cuda.device(where):
+                self._launch(dst, src, n)
+        else:
+            self._launch(dst, src, n)
+
+    def _launch(self, dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
         try:
             check(fn("pb_copy")(dst.data_ptr(), src.data_ptr(), n * src.element_size(), stream()), "copy", kernels=0)
         finally:
