@@ -95,10 +95,21 @@ __device__ __forceinline__ void peer_push(uint32_t addr, uint32_t bar, const uin
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
                  ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(bar) : "memory");
 }
-// mbar_wait on a barrier that other blocks of the cluster arrive at: their writes before it are visible behind it.
+// mbar_wait on a barrier that other blocks of the cluster arrive at: what they wrote or read before is ordered before what follows.
+// (By the wait itself: a fence behind both waits costs every thread, gate/up 24576 x 4096 with 48 tokens 34.9 us against 32.2.)
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    if (!mbar_wait(bar, parity, abort_flag)) return false;
-    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+    if (mbar_try_wait_cluster(bar, parity)) return true;
+    const long long t0 = clock64(), limit = __ldg(&g_wait_limit);
+    while (!mbar_try_wait_cluster(bar, parity)) {
+        if (*abort_flag) return false;
+        if (clock64() - t0 > limit) return false;
+    }
     return true;
 }
 
@@ -304,7 +315,7 @@ gemm_tcgen05_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
                 const int quads = (min(a.pass, a.M - first) + 3) / 4, share = (quads + a.slices - 1) / a.slices;
                 const int own = max(0, min(share, quads - rank * share));
                 // what the pass before laid down has been read by all blocks of the cluster
-                ok = named_barrier_all(4, 128, mbar_wait(part_empty, (pass & 1) ^ 1, abort_flag));
+                ok = named_barrier_all(4, 128, mbar_wait_cluster(part_empty, (pass & 1) ^ 1, abort_flag));
                 if (!ok) break;
                 if (etid == 0) mbar_expect_tx(part_full, a.slices * own * a.rows * 16);
                 int owner = 0, slot = 0;
