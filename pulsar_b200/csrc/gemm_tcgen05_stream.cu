@@ -359,16 +359,17 @@ gemm_tcgen05_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
     if (a.slices > 1 && (warp < 2 || warp == 6)) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemColumns));
-    // A block that ends has what its peers sent it, and sends nothing to one that has ended.  One that gave up waits for its
-    // copies in flight, and for its peers, which may still send to it.
-    if (*abort_flag) {
+    // A block that gave up lets its copies and products in flight land before it frees what they write.
+    const bool gave_up = *abort_flag != 0;
+    if (gave_up)
         for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-        if (a.slices > 1) {
-            __syncthreads();
-            asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
-            asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-        }
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemColumns));
+    // A block that ends has what its peers sent it, and sends nothing to one that has ended.  One that gave up waits for its peers, which
+    // may still send to it.
+    if (gave_up && a.slices > 1) {
+        __syncthreads();
+        asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     }
 }
 

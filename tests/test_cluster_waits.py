@@ -15,3 +15,10 @@ def test_waits_for_other_blocks_are_ordered_for_the_whole_cluster():
     waits = re.findall(r"(mbar_wait\w*)\((part_\w+)", _text("gemm_tcgen05_stream.cu"))
     assert sorted({bar for _, bar in waits}) == ["part_empty", "part_full"]
     assert {call for call, _ in waits} == {"mbar_wait_cluster"}
+
+
+def test_tensor_memory_is_freed_behind_the_work_in_flight():
+    """A block that gave up a wait lets its copies and products land before it frees the tensor memory that they write."""
+    for name in ("gemm_tcgen05.cu", "gemm_tcgen05_stream.cu", "attention_prefill_tcgen05.cu", "attention_prefill_tcgen05_dual.cu"):
+        order = re.findall(r"__nanosleep|tcgen05\.dealloc", _text(name))
+        assert order and order == ["__nanosleep", "tcgen05.dealloc"] * (len(order) // 2), name
