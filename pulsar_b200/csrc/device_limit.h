@@ -1,5 +1,5 @@
-// A kernel's limit of dynamic shared memory as it has been raised so far, per device: the limit belongs to a device's
-// copy of the kernel, so a process that launches on a second GPU has to raise it there too.  Plain C++ (the calls that
+// What a process keeps per device about its launches.  A kernel's limit of dynamic shared memory as it has been raised so far: the limit
+// belongs to a device's copy of the kernel, so a process that launches on a second GPU has to raise it there too.  Plain C++ (the calls that
 // ask for the current device and set the limit are the caller's), any number of threads.
 #pragma once
 
@@ -31,6 +31,28 @@ private:
     static constexpr int kDevices = 64;
     std::atomic<size_t> held_[kDevices] = {};
     std::mutex lock_;
+};
+
+// A number above 0 that belongs to a device and is asked for once on each: how many of a launch's clusters it holds, say.
+class DeviceCount {
+public:
+    // The current device's number, or 0 where it cannot be had; that is not remembered, so the next call asks again.  device(int*) gives
+    // the current device, ask(int*) its number; both return 0 or an error.
+    template <typename Device, typename Ask>
+    int get(Device device, Ask ask) {
+        int dev = 0, n = 0;
+        if (device(&dev) != 0) return 0;
+        const bool kept = dev >= 0 && dev < kDevices;               // more devices than are kept account of are asked every time
+        if (kept) n = known_[dev].load(std::memory_order_relaxed);
+        if (n > 0) return n;
+        if (ask(&n) != 0 || n <= 0) return 0;
+        if (kept) known_[dev].store(n, std::memory_order_relaxed);
+        return n;
+    }
+
+private:
+    static constexpr int kDevices = 64;
+    std::atomic<int> known_[kDevices] = {};
 };
 
 }  // namespace pb

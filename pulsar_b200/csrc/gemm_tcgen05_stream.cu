@@ -32,7 +32,6 @@
 #include "tcgen05_common.cuh"
 
 #include <algorithm>
-#include <atomic>
 #include <cstdlib>
 
 namespace {
@@ -412,18 +411,14 @@ cudaLaunchConfig_t stream_config(cudaLaunchAttribute (&attr)[2], int slices, int
 // clusters, so not every SM can be used by every size).
 template <int MODE, typename OutT>
 int resident_clusters(int slices) {
-    static std::atomic<int> known[kMaxSlices + 1];
-    int n = known[slices].load(std::memory_order_relaxed);
-    if (n == 0) {
+    static DeviceCount known[kMaxSlices + 1];
+    return known[slices].get([](int* dev) { return (int)cudaGetDevice(dev); }, [&](int* n) {
         cudaLaunchAttribute attr[2];
         const cudaLaunchConfig_t cfg = stream_config(attr, slices, slices, kSmem, false, nullptr);
-        if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_stream_kernel<MODE, OutT>, &cfg) != cudaSuccess || n <= 0) {
-            (void)cudaGetLastError();
-            n = -1;
-        }
-        known[slices].store(n, std::memory_order_relaxed);
-    }
-    return n;
+        const cudaError_t rc = cudaOccupancyMaxActiveClusters(n, gemm_tcgen05_stream_kernel<MODE, OutT>, &cfg);
+        if (rc != cudaSuccess) (void)cudaGetLastError();
+        return (int)rc;
+    });
 }
 
 // How a problem is cut: slices of K, rows of a tile.  The cost is what a block walks through one after the other, in rows of 128 k:
@@ -433,14 +428,15 @@ int resident_clusters(int slices) {
 // 128 rows 9.7, 3 x 96 10.5; 6144 x 4096 2 x 96 11.8, 3 x 96 14.2; gate/up 24576 x 4096 2 x 112 32.1, 2 x 128 32.6, 4 x 128 38.7;
 // 4096 x 12288 4 x 128 18.5, 2 x 128 21.5.
 template <int MODE, typename OutT>
-bool cut(StreamArgs& a, int k_tiles) {
+int cut(StreamArgs& a, int k_tiles) {          // the clusters that the device holds, 0: none of any size
     static const int slices_forced = forced("PULSAR_STREAM_SLICES");
     const int width = MODE == kSwiGLU ? a.inter.n : a.N, quads = a.n_pad / 4;
     float best = 0.0f;
+    int clusters = 0;
     for (int s = 1; s <= kMaxSlices && s <= k_tiles; ++s) {
         if (slices_forced > 0 && s != std::min(slices_forced, std::min(kMaxSlices, k_tiles))) continue;
         const int n = resident_clusters<MODE, OutT>(s);
-        if (n <= 0) continue;
+        if (n == 0) continue;
         for (int rows = kRows; rows >= 48; rows -= 16) {
             const int cols = MODE == kSwiGLU ? rows / 2 : rows, tiles = (width + cols - 1) / cols, rest = tiles % n;
             float rounds = (float)(tiles / n);
@@ -448,18 +444,18 @@ bool cut(StreamArgs& a, int k_tiles) {
             const float walk = (float)((k_tiles + s - 1) / s * (rows + a.n_pad / 2));
             const float add = (s > 1 ? 250.0f : 100.0f) + 4.0f * quads + 33.0f * ((quads + s - 1) / s);
             const float cost = rounds * fmaxf(walk, add) + add;
-            if (best == 0.0f || cost < best) { best = cost; a.slices = s; a.rows = rows; a.n_tiles = tiles; }
+            if (best == 0.0f || cost < best) { best = cost; clusters = n; a.slices = s; a.rows = rows; a.n_tiles = tiles; }
         }
     }
-    return best > 0.0f;
+    return clusters;
 }
 
 template <int MODE, typename OutT>
 int launch(const void* x, const void* w, void* out, StreamArgs a, bool loaded, cudaStream_t stream) {
     static SmemLimit limit;
     if (const int rc = limit.allow(gemm_tcgen05_stream_kernel<MODE, OutT>, kSmem)) return rc;
-    if (!cut<MODE, OutT>(a, (a.K + kBK - 1) / kBK)) return (int)cudaErrorNotSupported;
-    const int n = resident_clusters<MODE, OutT>(a.slices);
+    const int n = cut<MODE, OutT>(a, (a.K + kBK - 1) / kBK);
+    if (n == 0) return PB_ERR_BAD_SIZE;            // declined: the caller has another product
     const int stage_bytes = (a.rows + a.n_pad) * kBK * 2;
     const int bar_bytes = (2 * kMaxStages + 6) * 8 + 16, room = kSmem - 1024 - bar_bytes;
     // The MMAs read kRows rows from an atom's first: what lies behind the last stage, up to there, belongs to the block as well.

@@ -589,7 +589,7 @@ def gemm_tcgen05_stream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swi
     with _Gating(gating if swiglu else None):
         status = fn("pb_gemm_tcgen05_stream")(mode, code(out.dtype), _p(a), _p(w), _p(out), m, n, k, int(loaded), stream())
     if status == -3:
-        return False                 # addresses that are no multiples of 16
+        return False                 # addresses that are no multiples of 16, or a device that holds no cluster of its blocks
     check(status, "gemm_tcgen05_stream")
     return True
 

@@ -76,6 +76,65 @@ def test_limits_are_kept_per_device(tmp_path):
     assert done.returncode == 0, done.stdout
 
 
+COUNTS = r"""
+#include "device_limit.h"
+#include <cstdio>
+#include <cstdlib>
+#include <thread>
+#include <vector>
+static thread_local int current = 0;
+static std::atomic<int> asked;
+static int device(int* d) { if (current < 0) return 100; *d = current; return 0; }
+static int ask(int* n) { ++asked; *n = 10 * (current + 1); return 0; }
+static int fail(int* n) { ++asked; *n = 5; return 2; }
+static int none(int* n) { ++asked; *n = 0; return 0; }
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::exit(1); } } while (0)
+
+int main() {
+    static pb::DeviceCount a, b;
+    // a failure and an answer of none are not remembered; each device has its own number, asked for once
+    CHECK(a.get(device, fail) == 0 && a.get(device, none) == 0 && asked == 2);
+    for (int round = 0; round < 3; ++round)
+        for (current = 0; current < 3; ++current) CHECK(a.get(device, ask) == 10 * (current + 1));
+    CHECK(asked == 5);
+    current = 1;
+    CHECK(a.get(device, fail) == 20 && b.get(device, fail) == 0);
+    current = -1;
+    CHECK(a.get(device, ask) == 0);
+    current = 70;
+    CHECK(a.get(device, ask) == 710 && a.get(device, ask) == 710 && asked == 8);
+    std::vector<std::thread> threads;
+    for (int t = 0; t < 8; ++t)
+        threads.emplace_back([t] { current = 10 + t % 4; for (int i = 0; i < 10000; ++i) CHECK(b.get(device, ask) == 10 * (current + 1)); });
+    for (auto& t : threads) t.join();
+    return 0;
+}
+"""
+
+
+def test_counts_are_kept_per_device(tmp_path):
+    cxx = shutil.which(os.environ.get("CXX", "g++")) or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    src = tmp_path / "counts.cpp"
+    src.write_text(COUNTS)
+    subprocess.run([cxx, "-std=c++17", "-O2", "-pthread", "-I", CSRC, str(src), "-o", str(tmp_path / "counts")], check=True)
+    done = subprocess.run([str(tmp_path / "counts")], stdout=subprocess.PIPE, text=True, timeout=120)
+    assert done.returncode == 0, done.stdout
+
+
+def test_nothing_is_asked_of_a_device_once_for_the_whole_process():
+    """How many clusters a device holds belongs to the device: no launcher keeps the answer in a static of its own."""
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name)) as f:
+                text = f.read()
+            for at in re.finditer(r"cudaOccupancyMaxActiveClusters\(", text):
+                before = text[max(0, at.start() - 600):at.start()]
+                before = before[before.rfind("\n}") + 1:]
+                assert "static std::atomic" not in before and "DeviceCount" in before, name
+
+
 def test_no_launch_remembers_a_raised_limit_for_the_whole_process():
     """Every launch with more shared memory than any kernel may have raises the limit through ``SmemLimit``, or on every call."""
     for name in sorted(os.listdir(CSRC)):
