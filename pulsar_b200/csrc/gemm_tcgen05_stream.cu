@@ -421,12 +421,28 @@ int resident_clusters(int slices) {
     });
 }
 
+// Shared memory of a block besides the alignment of its ring: barriers, and what is left for stages and partial sums.
+constexpr int kBarBytes = (2 * kMaxStages + 6) * 8 + 16, kRoom = kSmem - 1024 - kBarBytes;
+
+// Bytes of the partial sums of `pass` tokens.
+inline int sum_bytes(int pass, int slices, int rows) { return (pass / 4 + slices - 1) / slices * slices * rows * 16; }
+
+// Tokens whose partial sums are laid down at once: all, or 64 where all leave fewer than three stages.
+inline int pass_tokens(int n_pad, int slices, int rows) {
+    return n_pad > 64 && kRoom - sum_bytes(n_pad, slices, rows) < 3 * (rows + n_pad) * kBK * 2 ? 64 : n_pad;
+}
+
 // How a problem is cut: slices of K, rows of a tile.  The cost is what a block walks through one after the other, in rows of 128 k:
-// its tiles, the last round counted by how full it is but as no less than half a round (an SM alone pulls twice its share of HBM; with
-// many tokens, whose loads come from L2, less), times the k-tiles of its slice, times the tile's rows and half a row for every
-// token; or what the exchange and the adding up take, by its share of the tokens, where that is longer; and that once more, behind the last tile.  Measured (us, 8B sizes, 48 tokens): 4096 x 4096 4 slices x
-// 128 rows 9.7, 3 x 96 10.5; 6144 x 4096 2 x 96 11.8, 3 x 96 14.2; gate/up 24576 x 4096 2 x 112 32.1, 2 x 128 32.6, 4 x 128 38.7;
-// 4096 x 12288 4 x 128 18.5, 2 x 128 21.5.
+//   - the k-tiles of its slice times the tile's rows and half a row for every token, for its first tile;
+//   - that for every further tile, or what the sums of a tile take where that is longer.  All of a tile's sums pass through every
+//     block's epilogue however many slices there are, once for each pass (gate/up 28672 x 4096, 111 tokens, tiles of 128 rows: 4.7 rounds of 3
+//     slices 73 us, 3 of 2 slices 48; 76000 x 2048, 128 tokens: 1, 2, 4, 8 slices 65, 90, 142, 297);
+//   - the last round by how full it is, but as no less than half a round (an SM alone pulls twice its share of HBM; with many tokens,
+//     whose loads come from L2, less);
+//   - the exchange behind the last tile, by the block's share of the tokens.
+// The weights of these were fitted to the times of all cuts of 30 products with 32 to 128 tokens: the chosen one is on average 2.7 % behind
+// the best (9.0 % while the sums were taken to cost less the more slices share them).  us at 48 tokens: 4096 x 4096 4 slices x 128 rows
+// 8.9; 6144 x 4096 2 x 96 11.3; gate/up 24576 x 4096 2 x 112 32.2; 4096 x 12288 4 x 128 19.1.
 template <int MODE, typename OutT>
 int cut(StreamArgs& a, int k_tiles) {          // the clusters that the device holds, 0: none of any size
     static const int slices_forced = forced("PULSAR_STREAM_SLICES");
@@ -437,13 +453,15 @@ int cut(StreamArgs& a, int k_tiles) {          // the clusters that the device h
         if (slices_forced > 0 && s != std::min(slices_forced, std::min(kMaxSlices, k_tiles))) continue;
         const int n = resident_clusters<MODE, OutT>(s);
         if (n == 0) continue;
+        const int slice_tiles = (k_tiles + s - 1) / s, share = (quads + s - 1) / s;
         for (int rows = kRows; rows >= 48; rows -= 16) {
             const int cols = MODE == kSwiGLU ? rows / 2 : rows, tiles = (width + cols - 1) / cols, rest = tiles % n;
+            const int passes = pass_tokens(a.n_pad, s, rows) < a.n_pad ? 2 : 1;
             float rounds = (float)(tiles / n);
             if (rest > 0) rounds += fminf(1.0f, fmaxf((float)rest / n, 0.5f + a.n_pad / 256.0f));
-            const float walk = (float)((k_tiles + s - 1) / s * (rows + a.n_pad / 2));
-            const float add = (s > 1 ? 250.0f : 100.0f) + 4.0f * quads + 33.0f * ((quads + s - 1) / s);
-            const float cost = rounds * fmaxf(walk, add) + add;
+            const float walk = (float)(slice_tiles * (rows + a.n_pad / 2));
+            const float sums = s > 1 ? 600.0f * passes + 80.0f * quads : 450.0f * passes + 64.0f * quads;
+            const float cost = fminf(rounds, 1.0f) * walk + fmaxf(rounds - 1.0f, 0.0f) * fmaxf(walk, sums) + 150.0f * passes + 20.0f * share;
             if (best == 0.0f || cost < best) { best = cost; clusters = n; a.slices = s; a.rows = rows; a.n_tiles = tiles; }
         }
     }
@@ -457,25 +475,19 @@ int launch(const void* x, const void* w, void* out, StreamArgs a, bool loaded, c
     const int n = cut<MODE, OutT>(a, (a.K + kBK - 1) / kBK);
     if (n == 0) return PB_ERR_BAD_SIZE;            // declined: the caller has another product
     const int stage_bytes = (a.rows + a.n_pad) * kBK * 2;
-    const int bar_bytes = (2 * kMaxStages + 6) * 8 + 16, room = kSmem - 1024 - bar_bytes;
     // The MMAs read kRows rows from an atom's first: what lies behind the last stage, up to there, belongs to the block as well.
     const int beyond = (a.rows + kRows) * kAtom * 2 + 1024;
-    // Partial sums of all tokens at once, or of 64 where that leaves fewer than three stages.
-    int stages = 0, part_bytes = 0;
-    for (int pass = a.n_pad; stages < 3 && pass > 0; pass = pass > 64 ? 64 : 0) {
-        a.pass = pass;
-        part_bytes = (pass / 4 + a.slices - 1) / a.slices * a.slices * a.rows * 16;
-        stages = (room - part_bytes) / stage_bytes;
-        if (stages > kMaxStages) stages = kMaxStages;
-        while (stages > 0 && (stages - 1) * stage_bytes + beyond > kSmem) --stages;
-    }
+    a.pass = pass_tokens(a.n_pad, a.slices, a.rows);
+    const int part_bytes = sum_bytes(a.pass, a.slices, a.rows);
+    int stages = std::min((kRoom - part_bytes) / stage_bytes, kMaxStages);
+    while (stages > 0 && (stages - 1) * stage_bytes + beyond > kSmem) --stages;
     static const int stages_forced = forced("PULSAR_STREAM_STAGES");
     if (stages_forced > 0 && stages_forced < stages) stages = stages_forced;
     if (stages < 2) return PB_ERR_BAD_SIZE;
     a.stages = stages;
     a.part_offset = stages * stage_bytes;
     a.bar_offset = a.part_offset + part_bytes;
-    int smem = a.bar_offset + bar_bytes + 1024;
+    int smem = a.bar_offset + kBarBytes + 1024;
     if (smem < (stages - 1) * stage_bytes + beyond) smem = (stages - 1) * stage_bytes + beyond;
     CUtensorMap mx, mw;
     if (const int rc = make_map(&mx, x, a.M, a.K, a.n_pad)) return rc;
@@ -493,6 +505,21 @@ PB_EXPORT int pb_gemm_tcgen05_stream_supported(int mode, int M, int N, int K) {
     if (M <= 0 || M > 128 || N <= 0 || K <= 0 || (K % 8)) return 0;
     if (mode == kSwiGLU) return (N % 2 == 0) ? 1 : 0;
     return mode == kPlain ? 1 : 0;
+}
+
+// slices and rows: how the product is cut on the current device.  Returns the clusters that it holds, 0 where the product is declined.
+PB_EXPORT int pb_gemm_tcgen05_stream_cut(int mode, int M, int N, int K, int* slices, int* rows) {
+    if (!pb_gemm_tcgen05_stream_supported(mode, M, N, K)) return 0;
+    StreamArgs a{};
+    a.N = N;
+    a.n_pad = (M + 15) / 16 * 16;
+    a.inter = GatedInter(mode == kSwiGLU ? N / 2 : 0);
+    static SmemLimit limits[2];
+    if (mode == kSwiGLU ? limits[0].allow(gemm_tcgen05_stream_kernel<kSwiGLU, bf16>, kSmem) : limits[1].allow(gemm_tcgen05_stream_kernel<kPlain, bf16>, kSmem)) return 0;
+    const int n = mode == kSwiGLU ? cut<kSwiGLU, bf16>(a, (K + kBK - 1) / kBK) : cut<kPlain, bf16>(a, (K + kBK - 1) / kBK);
+    *slices = a.slices;
+    *rows = a.rows;
+    return n;
 }
 
 // limit > 0: the new limit of the kernel's bounded waits in clock cycles; error >= 0: the new value of the error

@@ -74,6 +74,7 @@ _SIGNATURES = {
     "pb_gemm_tcgen05_stream": [_I, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "pb_copy": [_P, _P, ctypes.c_longlong, _P],
     "pb_gemm_tcgen05_stream_supported": [_I, _I, _I, _I],
+    "pb_gemm_tcgen05_stream_cut": [_I, _I, _I, _I, _P, _P],
     "pb_gemm_tcgen05_stream_wait_control": [ctypes.c_longlong, _I, _P],
     "pb_gemm_tcgen05_wait_control": [ctypes.c_longlong, _I, _P],
     "pb_gemm_tcgen05_wait_selftest": [_P],

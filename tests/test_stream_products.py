@@ -69,3 +69,23 @@ def test_linear_takes_it_and_gives_the_library_products_result(m, n, k, monkeypa
     ops.linear(a, odd, out)
     assert taken == [True, False]
     assert float((out.double() - ref).abs().max() / ref.abs().max()) < 2.0 ** -8
+
+
+# every block's epilogue takes all of a tile's sums, however many slices share them: no more slices than the walk over a tile pays for
+@pytest.mark.parametrize("gated,m,n,k,most", [(1, 111, 28672, 4096, 2), (1, 111, 22016, 4096, 2), (1, 97, 16384, 2048, 1), (0, 128, 76000, 2048, 1),
+                                              (0, 112, 128256, 2048, 1), (1, 48, 24576, 4096, 2), (0, 48, 4096, 12288, 4), (0, 17, 160, 4096, 8)])
+def test_a_product_is_cut_into_no_more_slices_than_its_sums_allow(gated, m, n, k, most):
+    import ctypes
+    from pulsar_b200 import ops
+    slices, rows = ctypes.c_int(), ctypes.c_int()
+    assert ops.fn("pb_gemm_tcgen05_stream_cut")(gated, m, n, k, ctypes.byref(slices), ctypes.byref(rows)) > 0
+    assert 1 <= slices.value <= most and rows.value % 16 == 0 and 48 <= rows.value <= 128
+    a, w, ref, size = _operands(m, n, k)
+    out = torch.full((m, n // 2 if gated else n), float("nan"), device="cuda")
+    assert ops.gemm_tcgen05_stream(a, w, out, swiglu=bool(gated))
+    if gated:
+        ref = torch.nn.functional.silu(ref[:, :n // 2]) * ref[:, n // 2:]
+        assert float((out.double() - ref).abs().max()) < 2e-4
+    else:
+        assert bool(((out.double() - ref).abs() <= k * 2.0 ** -23 * size).all())
+    ops.check_wait_words()
