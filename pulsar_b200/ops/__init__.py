@@ -553,24 +553,30 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bo
 # Which products of 17 to 128 tokens take this library's weight-streaming tcgen05 kernel instead of the library product: "auto" as
 # ``_stream_wanted`` has it; "1" all of them; "0" none.
 STREAM_GEMM = os.environ.get("PULSAR_GEMM_STREAM", "auto")
-_STREAM_MIN_ROWS = 4 * 148 * 128
+_STREAM_MIN_ROWS = 4 * 148 * 128        # heads: tiles for four rounds of all SMs
 
 
 def _stream_wanted(m: int, n: int, k: int, gated: bool = False) -> bool:
-    """Where the weight-streaming kernel is ahead.  It sets up, meets and ends in about 5 us, some of it under the kernels around
-    it; the tokens are read again with every tile of weights, which costs the more the more there are.  us, library / kernel, one
-    launch behind the other: 32 tokens 2048 x 4096 8.1 / 6.9, 160 x 4096 7.0 / 3.9, 8192 x 2048 8.2 / 8.6, 16384 x 2048 gated 15.1 / 13.6,
-    1024 x 1024 3.8 / 4.2; 64 tokens 8192 x 2048 8.5 / 9.9, 8192 x 4096 15.3 / 14.3; 96 tokens 4096 x 8192 16.6 / 15.9, 8192 x 4096
-    15.3 / 16.2, 24576 x 4096 gated 43.4 / 38.7; 128 tokens the same 43.3 / 45.5, 4096 x 8192 16.5 / 18.3.  In a layer of the 8B
-    sizes the kernels before and behind hide more of it: its four products with their norms take 80 us at 48 tokens (library 90)
-    and 83 at 64 (93)."""
+    """Where the weight-streaming kernel is ahead of the library's product (and the gating kernel behind that) between a norm and another
+    product, as in a layer: much of its 5 us of setting up, meeting and ending is hidden by the kernels around it, some 3 us more than
+    of the library's.  The tokens are read again with every tile of weights and the sums pass through every block, which costs the more
+    the more tokens there are.  us, the three kernels with the library's product / with this one: 32 tokens 8192 x 2048 20.4 / 18.5,
+    2048 x 2048 13.7 / 11.9 (48 tokens 12.3 / 13.7), 6144 x 4096 27.8 / 22.9; 64 tokens 6144 x 4096 28.3 / 26.1, 10240 x 4096 38.5 / 35.2, 4096 x
+    12288 59.6 / 52.4; 80 tokens 6144 x 4096 28.5 / 28.3; 96 tokens 4096 x 12288 58.7 / 57.9, 14336 x 8192 91.4 / 91.0, 28672 x 8192 178.8 /
+    195.5.  Gated: 48 tokens 16384 x 2048 27.4 / 25.8, 5632 x 2048 16.5 / 19.4; 96 tokens 22016 x 4096 61.5 / 56.5, 8192 x 4096 29.7 / 30.2;
+    112 tokens 28672 x 4096 79.6 / 76.9, 22016 x 4096 60.6 / 61.3, 11264 x 4096 35.9 / 41.0; 128 tokens 61.0 / 68.1 with 22016.  Heads: 96 tokens
+    151936 x 4096 222 / 209, x 1024 64 / 60, 76000 x 2048 58.5 / 58.4, x 512 18 / 29; 128 tokens 151936 x 4096 228 / 232, x 1024 67 / 82."""
     if m > 128 or STREAM_GEMM == "0" or GEMM_BACKEND == "library":
         return False
-    if STREAM_GEMM == "1" or n >= _STREAM_MIN_ROWS:
+    if STREAM_GEMM == "1":
         return True
+    if n >= _STREAM_MIN_ROWS:
+        return k >= 1024 and m <= 96
     if m <= 64:
         return k >= (2048 if m <= 32 else 4096)
-    return k >= 4096 and m <= 112 if gated else k >= 8192 and m <= 96
+    if gated:
+        return k >= 4096 and (m <= 96 or (m <= 112 and n >= 16384))
+    return k >= 8192 and m <= 96 and n <= 16384
 
 
 def gemm_tcgen05_stream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bool = False, gating=None, loaded: bool = True) -> bool:
