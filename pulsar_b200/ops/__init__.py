@@ -1060,6 +1060,9 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
         while n_dec < len(q_lens) and q_lens[n_dec] == 1:
             n_dec += 1
         table, cu_q, kv_len = cache.block_table, ctx.cu_q, ctx.kv_len
+        behind = (table, cu_q, kv_len, q_lens)                    # of the portions (a slice costs the host more than a microsecond a layer)
+        if n_dec > 0:
+            behind = (table[n_dec:], cu_q[n_dec:], kv_len[n_dec:], q_lens[n_dec:])
 
         def decode(beside: bool) -> None:
             n_splits = decode_shares(n_dec, hkv, table.shape[1] * page_size)
@@ -1072,11 +1075,9 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
         if n_dec > 0 and not beside:
             decode(False)
         if use_tcgen05:
-            paged_attention_prefill_tcgen05(q, cache.k_pool, cache.v_pool, out, table[n_dec:], cu_q[n_dec:], kv_len[n_dec:],
-                                            prefill_tcgen05_tiles(q_lens[n_dec:]), scale, window)
+            paged_attention_prefill_tcgen05(q, cache.k_pool, cache.v_pool, out, *behind[:3], prefill_tcgen05_tiles(behind[3]), scale, window)
         else:
-            paged_attention_prefill_tc(q, cache.k_pool, cache.v_pool, out, table[n_dec:], cu_q[n_dec:], kv_len[n_dec:],
-                                       prefill_tc_tiles(q_lens[n_dec:]), scale, window)
+            paged_attention_prefill_tc(q, cache.k_pool, cache.v_pool, out, *behind[:3], prefill_tc_tiles(behind[3]), scale, window)
         if beside:
             decode(True)
         return
