@@ -377,10 +377,23 @@ int launch_tile(const float* A, const float* W, TO* out, int M, int N, int K, cu
 template <typename TO>
 int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, bool loaded, cudaStream_t stream) {
     // With one block an SM or fewer a block's ring has to keep HBM busy by itself, and its chain is as long as the barriers between its
-    // stages make it: four stages of 256 k, where more blocks an SM take four of 128 (five to eight rows: two of 256).  us, 64 k a stage before: 4096 x 4096 4 rows 21.2 -> 17.6, 8 rows 27.1 -> 23.2; 24576 x 4096 4 rows 74.9 -> 69.2, 8 rows
-    // 103.3 -> 85.7 (93.6 with 128 k), 16 rows 188.5 -> 174; 151936 x 4096 8 rows 618 -> 509; 2048 x 2048 one row 11.9 -> 8.1.
+    // stages make it: four stages of 256 k, where more blocks an SM take four of 128 (five to eight rows: two of 256).  us, 64 k a stage:
+    // 4096 x 4096 4 rows 21.2 -> 17.6, 8 rows 27.1 -> 23.2; 24576 x 4096 4 rows 74.9 -> 69.2, 8 rows 103.3 -> 85.7 (93.6 with 128 k),
+    // 16 rows 188.5 -> 174; 151936 x 4096 8 rows 618 -> 509; 2048 x 2048 one row 11.9 -> 8.1.
+    // Stages of 64 k under a short K: a long stage is waited for and multiplied whole however few of its k there are.  us with 64 k / with
+    // long stages: 1024 x 64 1 row 1.4 / 1.8, 8 rows 1.3 / 2.8, x 128 2 rows 1.8 / 1.9, 4 rows 1.9 / 2.1, 8 rows 1.9 / 2.7, 16 rows 3.0 / 3.5,
+    // x 192 4 rows 2.3 / 2.1, x 320 8 rows 3.6 / 4.7, x 512 4.9 / 4.7, x 576 6.2 / 7.2, 16 rows 10.3 / 8.7; 8192 x 192 16 rows 5.4 / 6.4.
     const bool few = (N + RN - 1) / RN <= 148;
+    const bool brief = M <= 2 ? K <= 64 : M <= 4 ? K <= (few ? 128 : 64) : M <= 8 ? K < (few ? 640 : 384) && K % 256 != 0
+                              : K <= 128 || (!few && K < 384 && K % 128 != 0);
 #define PB_ROWS(R, T, CW, ST, RK) return launch_rows<R, T, CW, ST, RK>(A, W, out, M, N, K, loaded, stream)
+    if (brief) {
+        if (M == 1) PB_ROWS(1, 1, 1, 8, 64);
+        if (M == 2) PB_ROWS(2, 1, 1, 8, 64);
+        if (M <= 4) PB_ROWS(2, 1, 2, 8, 64);
+        if (M <= 8) { if (few) PB_ROWS(2, 1, 4, 16, 64); PB_ROWS(2, 2, 2, 8, 64); }
+        if (M <= 16) { if (few) PB_ROWS(2, 1, 8, 16, 64); PB_ROWS(4, 2, 2, 8, 64); }
+    }
     if (M == 1) { if (few) PB_ROWS(1, 1, 1, 4, 256); PB_ROWS(1, 1, 1, 4, 128); }
     if (M == 2) { if (few) PB_ROWS(2, 1, 1, 4, 256); PB_ROWS(2, 1, 1, 4, 128); }
     if (M <= 4) { if (few) PB_ROWS(2, 1, 2, 4, 256); PB_ROWS(2, 1, 2, 4, 128); }
