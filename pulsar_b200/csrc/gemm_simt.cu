@@ -167,22 +167,18 @@ int launch_rows(const float* A, const float* W, TO* out, int M, int N, int K, bo
 }
 
 // ---------------------------------------------------------------- more rows
-// Bound by the FMA pipes (60 % of their cycles with 24576 x 4096 weights and 387 rows; the issue slots 75 %).  A block of 128
-// threads owns 8 TM x 128 outputs, a warp 8 TM x 32, a thread TM x 8 of them (rows ty + 8 i, columns tx + 4 j).  Both operands
-// stand in shared memory as they do in memory, k fastest, so that asynchronous 16-byte copies bring them and a thread reads four
-// k of a row at once: 16 reads per 256 multiply-adds with TM 8.  Rows stand an odd number of 16-byte units apart (no
-// bank conflicts), and of the 8 x 4 lanes of a warp neighbours share a row or a column (see above).  Two stages of 32 k with 32 rows
-// (half the barriers of three stages of 16: 24576 x 4096 with 387 rows 2.03 -> 1.90 ms, 4096 x 4096 389 -> 356 us), three of 16 with
-// 64 rows (more would not fit).  A block
-// whose last rows lie behind M computes 8 or 16 rows instead.  k slowest in shared memory (copies of 4 bytes) was slower (35 against 39
-// TFLOP/s at 24576 x 4096, 387 rows), packed pairs of multiply-adds are not faster than single ones on this chip (61 against 65).
-constexpr int GN = 128;
-template <int GM> struct Tile { static constexpr int GK = GM == 64 ? 16 : 32, GST = GM == 64 ? 3 : 2, GSTRIDE = GK + 4; };
+// Bound by the FMA pipes and the register file.  A block of 128 threads owns 32 x 128 outputs, a warp 32 x 32, a thread 4 x 8.  Of the
+// 8 x 4 lanes of a warp neighbours share a row or a column (see above).  This form, with single multiply-adds, serves where an SM has
+// one block, and the last rows: a block whose last rows lie behind M computes 8 or 16.  Both operands stand in shared memory as they do
+// in memory, k fastest, so that asynchronous 16-byte copies bring them and a thread reads four k of a row at once (rows ty + 8 i,
+// columns tx + 4 j).  Rows stand an odd number of 16-byte units apart (no bank conflicts).  Two stages of 32 k: half the barriers of
+// three stages of 16 (24576 x 4096 with 387 rows 2.03 -> 1.90 ms, 4096 x 4096 389 -> 356 us).
+constexpr int GM = 32, GN = 128, GK = 32, GST = 2, GSTRIDE = GK + 4;
 
-template <int GM, int NI, typename TO>
+template <int NI, typename TO>
 __device__ __forceinline__ void tile_block(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out,
                                            int M, int N, int K, float* smem) {
-    constexpr int GK = Tile<GM>::GK, GST = Tile<GM>::GST, GSTRIDE = Tile<GM>::GSTRIDE, LR = 128 / (GK / 4);
+    constexpr int LR = 128 / (GK / 4);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = lane >> 1 & 3, ty = (lane & 1) | lane >> 3 << 1;
     const int row0 = blockIdx.x * GM, col0 = blockIdx.y * GN;
@@ -258,7 +254,6 @@ __device__ __forceinline__ void tile_block(const float* __restrict__ A, const fl
 // shifted by the k's quad, which spreads the stores over the banks).  A thread takes rows 4 ty .. 4 ty + 3 and columns 4 tx .. + 3 and 16 + 4 tx ..
 // + 3 of its warp's 32; its a values are doubled into pairs.  us, single multiply-adds before: 24576 x 4096 with 387 rows 1,898 -> 1,732,
 // 4096 x 4096 357 -> 338, 6144 x 4096 634 -> 493.  With 64 rows a block 1,838, with pairs along the rows 1,883.
-constexpr int PK = 32, PM = 32;
 __device__ __forceinline__ unsigned long long pair_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
@@ -267,17 +262,17 @@ __device__ __forceinline__ unsigned long long pair_fma(unsigned long long a, uns
 template <typename TO>
 __device__ __forceinline__ void pair_block(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out,
                                            int M, int N, int K, float* smem) {
-    constexpr int kStage = PK * (PM + GN), QK = PK / 4;
+    constexpr int kStage = GK * (GM + GN), QK = GK / 4;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = lane >> 1 & 3, ty = (lane & 1) | lane >> 3 << 1;
-    const int row0 = blockIdx.x * PM, col0 = blockIdx.y * GN, n_kt = (K + PK - 1) / PK;
+    const int row0 = blockIdx.x * GM, col0 = blockIdx.y * GN, n_kt = (K + GK - 1) / GK;
     const int q = tid % QK, r0 = tid / QK;                   // this thread's quad of k and its first row of 16 a round
-    float4 ra[PM / 16], rw[GN / 16];
+    float4 ra[GM / 16], rw[GN / 16];
     auto fetch = [&](int kt) {
-        const int k = kt * PK + q * 4;
+        const int k = kt * GK + q * 4;
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int e = 0; e < PM / 16; ++e) {
+        for (int e = 0; e < GM / 16; ++e) {
             const int r = row0 + r0 + 16 * e;
             ra[e] = r < M && k < K ? *reinterpret_cast<const float4*>(A + (size_t)r * K + k) : zero;
         }
@@ -294,9 +289,9 @@ __device__ __forceinline__ void pair_block(const float* __restrict__ A, const fl
     auto stash = [&](int stage) {
         float* as = smem + stage * kStage;
 #pragma unroll
-        for (int e = 0; e < PM / 16; ++e) put(as, PM, r0 + 16 * e, ra[e]);
+        for (int e = 0; e < GM / 16; ++e) put(as, GM, r0 + 16 * e, ra[e]);
 #pragma unroll
-        for (int e = 0; e < GN / 16; ++e) put(as + PK * PM, GN, r0 + 16 * e, rw[e]);
+        for (int e = 0; e < GN / 16; ++e) put(as + GK * GM, GN, r0 + 16 * e, rw[e]);
     };
     unsigned long long acc[4][4];                            // [row][pair of columns]
 #pragma unroll
@@ -309,11 +304,11 @@ __device__ __forceinline__ void pair_block(const float* __restrict__ A, const fl
     for (int kt = 0; kt < n_kt; ++kt) {
         if (kt + 1 < n_kt) fetch(kt + 1);
         const float* as = smem + (kt & 1) * kStage;
-        const float* ws = as + PK * PM + warp * 32;
+        const float* ws = as + GK * GM + warp * 32;
 #pragma unroll
-        for (int k = 0; k < PK; ++k) {
+        for (int k = 0; k < GK; ++k) {
             const int shift = 8 * (k >> 2 & 3);
-            const float4 a = *reinterpret_cast<const float4*>(as + k * PM + ((ty * 4) ^ shift));
+            const float4 a = *reinterpret_cast<const float4*>(as + k * GM + ((ty * 4) ^ shift));
             const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(ws + k * GN + ((tx * 4) ^ shift));
             const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(ws + k * GN + ((tx * 4 + 16) ^ shift));
             const float av[4] = {a.x, a.y, a.z, a.w};
@@ -351,25 +346,22 @@ __device__ __forceinline__ void pair_block(const float* __restrict__ A, const fl
     }
 }
 
-template <int TM, bool kPairs, typename TO>
-__global__ void __launch_bounds__(128, TM == 8 ? 3 : 4)
+template <bool kPairs, typename TO>
+__global__ void __launch_bounds__(128, 4)
 simt_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, TO* __restrict__ out, int M, int N, int K) {
-    constexpr int GM = 8 * TM;
-    __shared__ __align__(16) float tile_smem[Tile<GM>::GST * (GM + GN) * Tile<GM>::GSTRIDE];
+    __shared__ __align__(16) float tile_smem[GST * (GM + GN) * GSTRIDE];
     const int left = M - (int)blockIdx.x * GM;
-    if (TM == 8 && left > 32) tile_block<GM, TM, TO>(A, W, out, M, N, K, tile_smem);
-    else if (kPairs && left > 16) pair_block<TO>(A, W, out, M, N, K, tile_smem);
-    else if (left > 16) tile_block<GM, 4, TO>(A, W, out, M, N, K, tile_smem);
-    else if (left > 8) tile_block<GM, 2, TO>(A, W, out, M, N, K, tile_smem);
-    else tile_block<GM, 1, TO>(A, W, out, M, N, K, tile_smem);
+    if (kPairs && left > 16) pair_block<TO>(A, W, out, M, N, K, tile_smem);
+    else if (left > 16) tile_block<4, TO>(A, W, out, M, N, K, tile_smem);
+    else if (left > 8) tile_block<2, TO>(A, W, out, M, N, K, tile_smem);
+    else tile_block<1, TO>(A, W, out, M, N, K, tile_smem);
 }
 
-template <int TM, bool kPairs, typename TO>
+template <bool kPairs, typename TO>
 int launch_tile(const float* A, const float* W, TO* out, int M, int N, int K, cudaStream_t stream) {
-    dim3 grid((M + 8 * TM - 1) / (8 * TM), (N + GN - 1) / GN);
+    dim3 grid((M + GM - 1) / GM, (N + GN - 1) / GN);
     if (grid.y > 65535) return PB_ERR_TOO_LARGE;
-    static_assert(TM == 4 || !kPairs, "pairs are computed by blocks of 32 rows");
-    simt_tile_kernel<TM, kPairs, TO><<<grid, 128, 0, stream>>>(A, W, out, M, N, K);
+    simt_tile_kernel<kPairs, TO><<<grid, 128, 0, stream>>>(A, W, out, M, N, K);
     return launch_status();
 }
 
@@ -400,14 +392,11 @@ int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, boo
     if (M <= 8) { if (few) PB_ROWS(2, 1, 4, 4, 256); PB_ROWS(2, 2, 2, 2, 256); }
     if (M <= 16) { if (few) PB_ROWS(2, 1, 8, 4, 256); PB_ROWS(4, 2, 2, 4, 128); }
 #undef PB_ROWS
-    // 64 rows a block where there are blocks for 16 rounds of the SMs (151936 x 4096, 387 rows: 11.3 against 11.9 ms), else 32, whose last
-    // rounds are less empty (4096 x 4096: 33 rows 161 against 269 us, 387 rows 356 against 500, the general kernel 656;
-    // 24576 x 4096, 387 rows: 1.90 against 2.00 ms, 2.96 before)
-    if ((long)((M + 63) / 64) * ((N + GN - 1) / GN) >= 16 * 148) return launch_tile<8, false>(A, W, out, M, N, K, stream);
-    // Pairs where an SM has two blocks and more, whose loads then cover each other's (4096 x 12288, 200 rows: 773 us both ways): with
-    // one, the asynchronous copies are ahead (100 rows 448 against 609; 6144 x 4096, 64 rows 153 against 218).
-    if ((long)((M + 31) / 32) * ((N + GN - 1) / GN) > 148) return launch_tile<4, true>(A, W, out, M, N, K, stream);
-    return launch_tile<4, false>(A, W, out, M, N, K, stream);
+    // Pairs where an SM has two blocks and more, whose loads then cover each other's (4096 x 12288, 200 rows: 773 us both ways;
+    // 151936 x 4096, 387 rows: 10.1 ms, 11.2 with single multiply-adds, 11.3 with single ones and 64 rows a block): with one, the
+    // asynchronous copies are ahead (100 rows 448 against 608; 6144 x 4096, 64 rows 153 against 217).
+    if ((long)((M + GM - 1) / GM) * ((N + GN - 1) / GN) > 148) return launch_tile<true>(A, W, out, M, N, K, stream);
+    return launch_tile<false>(A, W, out, M, N, K, stream);
 }
 
 // ---------------------------------------------------------------- any operands
