@@ -327,15 +327,20 @@ int launch_split(const void* q, const void* k_pool, const void* v_pool, float* p
     const size_t plain = split_smem(D), staged = plain + (size_t)kWarps * 2 * 32 * (D * sizeof(T) + 16);
     const dim3 grid(n_splits, Hkv, n_seqs);
     const bool aligned = (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
-    const long long at_once = 148 * (227 * 1024 / (long long)(staged + 1024));
-    if (aligned && (long long)n_splits * Hkv * n_seqs <= at_once) {
+    const long long blocks = (long long)n_splits * Hkv * n_seqs, at_once = 148 * (227 * 1024 / (long long)(staged + 1024));
+    // Several passes copy the tiles anew for each: not while the blocks are few enough for L1 to hold a pass's rows for the next one
+    // (float32, 20 heads on 4 of 96, 128 blocks: 25.7 us staged, 16.8 plain; 24 on 4 of 128, whose tiles leave an SM one block: 21.4, 25.9).
+    const bool fits = Hq / Hkv <= kGP ? blocks <= at_once : blocks <= at_once && 2 * blocks > at_once;
+    if (aligned && fits) {
         static SmemLimit limit;
         if (const int rc = limit.allow(decode_split_kernel<T, true, kGP, kAcc>, staged)) return rc;
         return launch_pdl(decode_split_kernel<T, true, kGP, kAcc>, grid, kWarps * 32, staged, stream, (const T*)q, (const T*)k_pool, (const T*)v_pool,
                           partial, block_table, table_stride, kv_len, Hq, Hkv, D, page_size, scale, window, n_splits, pool_bounds_now());
     }
-    return launch_pdl(decode_split_kernel<T, false, kGP, kAcc>, grid, kWarps * 32, plain, stream, (const T*)q, (const T*)k_pool, (const T*)v_pool,
-                      partial, block_table, table_stride, kv_len, Hq, Hkv, D, page_size, scale, window, n_splits, pool_bounds_now());
+    // Not early: blocks that come while the kernel ahead still holds SMs are spread unevenly, and one or two to an SM never even out (float32,
+    // 16 heads of 128, 256 blocks of 900 keys 129 us, early 153; 24 on 4 of 128, 256 blocks of 225 51, early 63; 8 of 256, 128 blocks 17, 20).
+    return launch_early(false, decode_split_kernel<T, false, kGP, kAcc>, grid, kWarps * 32, plain, stream, (const T*)q, (const T*)k_pool, (const T*)v_pool,
+                        partial, block_table, table_stride, kv_len, Hq, Hkv, D, page_size, scale, window, n_splits, pool_bounds_now());
 }
 
 // The heads of a pass by the group's size, a lane's elements by the head's.
