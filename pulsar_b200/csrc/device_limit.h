@@ -36,12 +36,11 @@ private:
 // A number above 0 that belongs to a device and is asked for once on each: how many of a launch's clusters it holds, say.
 class DeviceCount {
 public:
-    // The current device's number, or 0 where it cannot be had; that is not remembered, so the next call asks again.  device(int*) gives
-    // the current device, ask(int*) its number; both return 0 or an error.
-    template <typename Device, typename Ask>
-    int get(Device device, Ask ask) {
-        int dev = 0, n = 0;
-        if (device(&dev) != 0) return 0;
+    // The number of `dev`, the current device, or 0 where it cannot be had; that is not remembered, so the next call asks again.
+    // ask(int*) gives the number and returns 0 or an error.
+    template <typename Ask>
+    int get(int dev, Ask ask) {
+        int n = 0;
         const bool kept = dev >= 0 && dev < kDevices;               // more devices than are kept account of are asked every time
         if (kept) n = known_[dev].load(std::memory_order_relaxed);
         if (n > 0) return n;

@@ -410,9 +410,9 @@ cudaLaunchConfig_t stream_config(cudaLaunchAttribute (&attr)[2], int slices, int
 // Clusters of `slices` blocks that the device holds at once (one block an SM; clusters do not cross the chip's GPU processing
 // clusters, so not every SM can be used by every size).
 template <int MODE, typename OutT>
-int resident_clusters(int slices) {
+int resident_clusters(int slices, int dev) {
     static DeviceCount known[kMaxSlices + 1];
-    return known[slices].get([](int* dev) { return (int)cudaGetDevice(dev); }, [&](int* n) {
+    return known[slices].get(dev, [&](int* n) {
         cudaLaunchAttribute attr[2];
         const cudaLaunchConfig_t cfg = stream_config(attr, slices, slices, kSmem, false, nullptr);
         const cudaError_t rc = cudaOccupancyMaxActiveClusters(n, gemm_tcgen05_stream_kernel<MODE, OutT>, &cfg);
@@ -448,10 +448,11 @@ int cut(StreamArgs& a, int k_tiles) {          // the clusters that the device h
     static const int slices_forced = forced("PULSAR_STREAM_SLICES");
     const int width = MODE == kSwiGLU ? a.inter.n : a.N, quads = a.n_pad / 4;
     float best = 0.0f;
-    int clusters = 0;
+    int clusters = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     for (int s = 1; s <= kMaxSlices && s <= k_tiles; ++s) {
         if (slices_forced > 0 && s != std::min(slices_forced, std::min(kMaxSlices, k_tiles))) continue;
-        const int n = resident_clusters<MODE, OutT>(s);
+        const int n = resident_clusters<MODE, OutT>(s, dev);
         if (n == 0) continue;
         const int slice_tiles = (k_tiles + s - 1) / s, share = (quads + s - 1) / s;
         for (int rows = kRows; rows >= 48; rows -= 16) {

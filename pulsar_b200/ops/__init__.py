@@ -235,14 +235,14 @@ class Pinned:
 
     def _copy(self, dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
         assert dst.is_cuda != src.is_cuda and dst.dtype == src.dtype and 0 <= n <= min(dst.numel(), src.numel()) and dst.is_contiguous() and src.is_contiguous()
-        where = dst.device if dst.is_cuda else src.device
+        where = (dst if dst.is_cuda else src).device
         if _device is None or where.index != _device():            # the stream is that of the tensor's device, whichever is current
             with torch.cuda.device(where):
-                self._launch(dst, src, n)
+                self._copy_here(dst, src, n)
         else:
-            self._launch(dst, src, n)
+            self._copy_here(dst, src, n)
 
-    def _launch(self, dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
+    def _copy_here(self, dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
         try:
             check(fn("pb_copy")(dst.data_ptr(), src.data_ptr(), n * src.element_size(), stream()), "copy", kernels=0)
         finally:
@@ -1060,9 +1060,9 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
         while n_dec < len(q_lens) and q_lens[n_dec] == 1:
             n_dec += 1
         table, cu_q, kv_len = cache.block_table, ctx.cu_q, ctx.kv_len
-        behind = (table, cu_q, kv_len, q_lens)                    # of the portions (a slice costs the host more than a microsecond a layer)
-        if n_dec > 0:
-            behind = (table[n_dec:], cu_q[n_dec:], kv_len[n_dec:], q_lens[n_dec:])
+        p_table, p_cu, p_len, p_lens = table, cu_q, kv_len, q_lens           # of the portions
+        if n_dec > 0:                                 # (a slice costs the host more than a microsecond a layer)
+            p_table, p_cu, p_len, p_lens = table[n_dec:], cu_q[n_dec:], kv_len[n_dec:], q_lens[n_dec:]
 
         def decode(beside: bool) -> None:
             n_splits = decode_shares(n_dec, hkv, table.shape[1] * page_size)
@@ -1075,9 +1075,9 @@ def attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, scale: float, wind
         if n_dec > 0 and not beside:
             decode(False)
         if use_tcgen05:
-            paged_attention_prefill_tcgen05(q, cache.k_pool, cache.v_pool, out, *behind[:3], prefill_tcgen05_tiles(behind[3]), scale, window)
+            paged_attention_prefill_tcgen05(q, cache.k_pool, cache.v_pool, out, p_table, p_cu, p_len, prefill_tcgen05_tiles(p_lens), scale, window)
         else:
-            paged_attention_prefill_tc(q, cache.k_pool, cache.v_pool, out, *behind[:3], prefill_tc_tiles(behind[3]), scale, window)
+            paged_attention_prefill_tc(q, cache.k_pool, cache.v_pool, out, p_table, p_cu, p_len, prefill_tc_tiles(p_lens), scale, window)
         if beside:
             decode(True)
         return

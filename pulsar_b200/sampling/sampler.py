@@ -47,7 +47,7 @@ class GenerationParams:
 
     def device_top_k(self) -> int:
         """``top_k`` as the kernels take it (a greedy row has no use for its own)."""
-        k = 0 if self.greedy else int(self.top_k)
+        k = int(self.top_k) if self.temperature > 0.0 else 0
         if not -_MAX_TOP_K - 1 <= k <= _MAX_TOP_K:
             raise ValueError(f"top_k must be at most {_MAX_TOP_K}, found {self.top_k}")
         return k

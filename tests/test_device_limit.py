@@ -84,7 +84,6 @@ COUNTS = r"""
 #include <vector>
 static thread_local int current = 0;
 static std::atomic<int> asked;
-static int device(int* d) { if (current < 0) return 100; *d = current; return 0; }
 static int ask(int* n) { ++asked; *n = 10 * (current + 1); return 0; }
 static int fail(int* n) { ++asked; *n = 5; return 2; }
 static int none(int* n) { ++asked; *n = 0; return 0; }
@@ -93,19 +92,16 @@ static int none(int* n) { ++asked; *n = 0; return 0; }
 int main() {
     static pb::DeviceCount a, b;
     // a failure and an answer of none are not remembered; each device has its own number, asked for once
-    CHECK(a.get(device, fail) == 0 && a.get(device, none) == 0 && asked == 2);
+    CHECK(a.get(0, fail) == 0 && a.get(0, none) == 0 && asked == 2);
     for (int round = 0; round < 3; ++round)
-        for (current = 0; current < 3; ++current) CHECK(a.get(device, ask) == 10 * (current + 1));
+        for (current = 0; current < 3; ++current) CHECK(a.get(current, ask) == 10 * (current + 1));
     CHECK(asked == 5);
-    current = 1;
-    CHECK(a.get(device, fail) == 20 && b.get(device, fail) == 0);
-    current = -1;
-    CHECK(a.get(device, ask) == 0);
-    current = 70;
-    CHECK(a.get(device, ask) == 710 && a.get(device, ask) == 710 && asked == 8);
+    CHECK(a.get(1, fail) == 20 && b.get(1, fail) == 0);
+    current = 70;                                       // beyond the devices that are kept account of
+    CHECK(a.get(70, ask) == 710 && a.get(70, ask) == 710 && asked == 8);
     std::vector<std::thread> threads;
     for (int t = 0; t < 8; ++t)
-        threads.emplace_back([t] { current = 10 + t % 4; for (int i = 0; i < 10000; ++i) CHECK(b.get(device, ask) == 10 * (current + 1)); });
+        threads.emplace_back([t] { current = 10 + t % 4; for (int i = 0; i < 10000; ++i) CHECK(b.get(current, ask) == 10 * (current + 1)); });
     for (auto& t : threads) t.join();
     return 0;
 }
