@@ -13,10 +13,10 @@
 // that is a multiple of 16 up to 256, float32 or bfloat16 storage, optional window.
 //
 // Bound by latency: a share is a tile or a few of 32 keys a warp.  While all blocks fit the SMs with a tile for each of their warps
-// in shared memory (kStaged), a warp asks for a tile's keys and values at once, by 16-byte asynchronous copies; with more blocks the
-// rows are read as they are needed, which lets an SM hold more blocks.  The heads of a pass have their chains side by side: no branch
+// in shared memory (kStaged), a warp asks for a tile's keys and values at once, by 16-byte asynchronous copies, and the launch is early;
+// with more blocks the rows are read as they are needed, which lets an SM hold more blocks.  The heads of a pass have their chains side by side: no branch
 // stands between them.  us with the merge, float32, 8 key heads of 128, groups of 4 (before: rows as needed, heads one after the other):
-// 4 sequences of 460 keys 12.6 (18.0), 2 of 3,000 32.7 (33.9), 8 of 500 19.7 (20.7); 6 of 50, 8 heads of 64, groups of 2, 9.2 (12.3).
+// 4 sequences of 460 keys 12.7 (18.2), 2 of 3,000 27.2 (33.5), 8 of 500 16.9 (20.3); 6 of 50, 8 heads of 64, groups of 2, 9.3 (12.4).
 //
 // Role in the reference: pulsar-core/src/kernels/paged_attention.cu:295-412
 // (paged_decode_split_kernel, paged_decode_combine_kernel; auto_splits :432-438).

@@ -141,7 +141,7 @@ __device__ __forceinline__ float squared_relu(float x) {
 // kernel has called pdl_trigger (or exited).  It must call pdl_wait before it touches anything
 // an earlier kernel writes (or reads and later overwrites); pdl_wait returns once the preceding
 // kernel has completed and its writes are visible.  Every kernel of the chain waits in all of its
-// blocks, so completion is transitive.  Kernels with a main loop trigger late, behind it, so that
+// blocks (the decode attention beside a prefill kernel in its last one, at its end), so completion is transitive.  Kernels with a main loop trigger late, behind it, so that
 // the next kernel's launch overlaps only this kernel's tail; short ones (norms, prepares, merges)
 // trigger first thing, so several kernels ahead may still be running when a kernel begins: what
 // one reads before pdl_wait has to be finished long before, as loaded weights and the keys of

@@ -34,7 +34,7 @@ using namespace pb;
 // other's banks.
 // us on the sizes of an 8B layer (64 x 64 tiles of the general kernel): 6144 x 4096 1 row 19.8 (277), 4 rows 24.4, 8 rows
 // 29.6, 16 rows 58; 4096 x 4096 15.1 / 17.7 / 23.2 / 38.5 (282); 24576 x 4096 64 / 69 / 86 / 174 (480); 4096 x 12288
-// 39.5 / 45.8 / 59.3 / 108 (851); 151936 x 4096 375 (6.6 TB/s) / 387 / 466 to 509 / 969.
+// 39.5 / 45.8 / 59.3 / 108 (851); 151936 x 4096 375 (6.6 TB/s) / 387 / 466 to 540 / 969.
 constexpr int RN = 32, RLOAD = 128;
 
 template <int R, int T, int CW, int RST, int RK, typename TO>
@@ -371,7 +371,7 @@ int launch_f32(const float* A, const float* W, TO* out, int M, int N, int K, boo
     // With one block an SM or fewer a block's ring has to keep HBM busy by itself, and its chain is as long as the barriers between its
     // stages make it: four stages of 256 k, where more blocks an SM take four of 128 (five to eight rows: two of 256).  us, 64 k a stage:
     // 4096 x 4096 4 rows 21.2 -> 17.6, 8 rows 27.1 -> 23.2; 24576 x 4096 4 rows 74.9 -> 69.2, 8 rows 103.3 -> 85.7 (93.6 with 128 k),
-    // 16 rows 188.5 -> 174; 151936 x 4096 8 rows 618 -> 509; 2048 x 2048 one row 11.9 -> 8.1.
+    // 16 rows 188.5 -> 174; 151936 x 4096 8 rows 562 to 618 -> 466 to 540; 2048 x 2048 one row 11.9 -> 8.1.
     // Stages of 64 k under a short K: a long stage is waited for and multiplied whole however few of its k there are.  us with 64 k / with
     // long stages: 1024 x 64 1 row 1.4 / 1.8, 8 rows 1.3 / 2.8, x 128 2 rows 1.8 / 1.9, 4 rows 1.9 / 2.1, 8 rows 1.9 / 2.7, 16 rows 3.0 / 3.5,
     // x 192 4 rows 2.3 / 2.1, x 320 8 rows 3.6 / 4.7, x 512 4.9 / 4.7, x 576 6.2 / 7.2, 16 rows 10.3 / 8.7; 8192 x 192 16 rows 5.4 / 6.4.

@@ -15,9 +15,10 @@
 // share it is (asynchronous stores that count on the receiver's barrier), which adds them in the order of the slices.  No partial
 // sum travels through L2.  Tail behind the last stage: 2.5 us (4.4 with sums fetched from the peers instead of sent by them).
 // us (the library's product, with the gating kernel behind gate/up; both in a graph of launches over weights larger than L2):
-//   48 tokens: 6144 x 4096 11.8 (11.5), 4096 x 4096 9.7 (10.0), gate/up 24576 x 4096 32.1 (40.2), 4096 x 12288 18.5 (21.8),
-//   151936 x 4096 182 (221; 6.9 TB/s); 111 tokens: gate/up 39.7 (47.5), the others behind the library's (the tokens' tile is read
-//   again from L2 with every tile: at 111 tokens as many bytes as W's).
+//   48 tokens: 6144 x 4096 11.3 (11.7), 4096 x 4096 9.0 (9.9), gate/up 24576 x 4096 32.2 (38.0), 4096 x 12288 19.1 (21.2),
+//   151936 x 4096 181 (206; 6.9 TB/s); 111 tokens: gate/up 39.5 (46.0), most others behind the library's (the tokens' tile is read
+//   again from L2 with every tile: at 111 tokens as many bytes as W's).  Between other kernels some 3 us more of this one's time is
+//   hidden than of the library's.
 //
 // Roles in a block (224 threads): warp 0 / one thread issues the TMA loads of W (with an evict-first L2 hint: weights are read once
 // per step and are far larger than L2), before the kernel waits for its predecessor; warp 6 / one thread those of x, behind it; warp

@@ -14,7 +14,7 @@ def _unaligned(t):
     return view
 
 
-# n: one block, a remainder, blocks for more than one an SM (4800); k: less than a stage, whole stages, tails; the last: 64 rows a block
+# n: one block, a remainder, blocks for more than one an SM (4800); k: less than a stage, whole stages, tails; the last: many blocks
 @pytest.mark.parametrize("n,k", [(1, 4), (33, 64), (130, 68), (321, 516), (4800, 132), (153600, 8)])
 @pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8, 9, 16, 17, 31, 33, 65, 100])
 def test_products_of_rows_and_tiles(m, n, k):
@@ -36,8 +36,8 @@ def test_products_of_rows_and_tiles(m, n, k):
         assert torch.equal(half, out.bfloat16())
 
 
-# every ring of stages turns more than twice, with a ragged tail: 16 and 8 stages of 64 k for every number of rows that streams the
-# weights, three stages of 16 k of the tiles of 64 rows
+# every ring of stages turns more than twice, with a ragged tail: four stages of 256 and of 128 k, two of 256, for every number of rows that
+# streams the weights, two of 32 k of the tiles
 @pytest.mark.parametrize("m,n,k", [(m, 130, 2116) for m in range(1, 17)] + [(m, 4800, 1092) for m in range(1, 17)]
                          + [(65, 153600, 132), (100, 153600, 132), (33, 130, 1092), (100, 321, 2116)])
 def test_products_whose_stages_are_used_again(m, n, k):
